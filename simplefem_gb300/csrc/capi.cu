@@ -206,6 +206,17 @@ const char* method_title(int method) {
     }
 }
 
+// Slices and values for the dataflow solvers; false (and the memory given back) when they
+// cannot be made, so that the solve takes the kernels over the CSR layout instead.
+bool flow_prepare(feec_system* s, bool f32) {
+    if (flow_build(s, f32) == FEEC_OK) return true;
+    cudaGetLastError();
+    s->flow.mem.release();
+    s->flow = FlowData{};
+    s->flow.mem.stream = s->home_stream;
+    return false;
+}
+
 // Core solve on a prepared system. xx / bb / res: device arrays in the ORIGINAL numbering.
 // tol_override > 0 replaces the tolerance of REFERENCE mode (the drop-in computes it on the host
 // with the reference's own serial loop).
@@ -287,6 +298,13 @@ int solve_core(feec_system* s, int method, int mode, double* xx, const double* b
     else if (s->nnz < 60000) shape.blocks = 16;
     if (s->user_lanes > 0) shape.lanes = s->user_lanes;
     if (s->user_blocks > 0) shape.blocks = s->user_blocks;
+    // Multicolor layouts run the dataflow solvers (kernels_flow.cu); the barrier-phase kernels
+    // keep index-order layouts, rows with D == 0 (never computed, so never published), caller
+    // launch shapes, and systems whose slices do not fit the device memory.
+    auto use_flow = [&](bool f32) {
+        return layout == FEEC_METHOD_RAINBOW && s->zero_diag_rows == 0 && s->user_blocks <= 0 && s->user_lanes <= 0 &&
+               flow_prepare(s, f32);
+    };
     float ms_total = 0.0f;
     int K_total = 0, outer = 0, status = FEEC_OK;
     double final_norm = 0.0;
@@ -343,9 +361,15 @@ int solve_core(feec_system* s, int method, int mode, double* xx, const double* b
                 a.use_zr_rule = 1;
                 a.max_iter = max_iter - (K_total - k0);
                 a.print_modulo = print_modulo; a.print_tol = tolerance;
+                const bool flow = use_flow(false);
                 FEEC_TRY(reset_status(s));
                 FEEC_TRY(cudaEventRecord(s->ev0, s->stream));
-                FEEC_TRY(launch_eisenstat<double>(a, shape, s->stream));
+                if (flow) {
+                    st = launch_flow_eisenstat(s, a, shape);
+                    if (st != FEEC_OK) return st;
+                } else {
+                    FEEC_TRY(launch_eisenstat<double>(a, shape, s->stream));
+                }
                 FEEC_TRY(cudaEventRecord(s->ev1, s->stream));
                 FEEC_TRY(cudaEventSynchronize(s->ev1));
                 FEEC_TRY(cudaEventElapsedTime(&ms, s->ev0, s->ev1));
@@ -368,9 +392,15 @@ int solve_core(feec_system* s, int method, int mode, double* xx, const double* b
                 a.use_zr_rule = 0;
                 a.rr_stop = tolerance * tolerance / rn2;
                 a.max_iter = max_iter - (K_total - k0);
+                const bool flow = use_flow(false);
                 FEEC_TRY(reset_status(s));
                 FEEC_TRY(cudaEventRecord(s->ev0, s->stream));
-                FEEC_TRY(launch_eisenstat<double>(a, shape, s->stream));
+                if (flow) {
+                    st = launch_flow_eisenstat(s, a, shape);
+                    if (st != FEEC_OK) return st;
+                } else {
+                    FEEC_TRY(launch_eisenstat<double>(a, shape, s->stream));
+                }
                 FEEC_TRY(cudaEventRecord(s->ev1, s->stream));
                 FEEC_TRY(cudaEventSynchronize(s->ev1));
                 FEEC_TRY(cudaEventElapsedTime(&ms, s->ev0, s->ev1));
@@ -381,8 +411,19 @@ int solve_core(feec_system* s, int method, int mode, double* xx, const double* b
                 a.rr_stop = (run_mode == FEEC_MODE_FP64) ? tolerance * tolerance : 0.0;
                 a.max_iter = max_iter - (K_total - k0);
                 a.print_modulo = print_modulo; a.print_tol = tolerance;
-                st = timed_launch_pcg64(s, a, shape, ms);
-                if (st != FEEC_OK) return st;
+                // below pcg_smem_max_rows() the one-block solver (timed_launch_pcg64)
+                if (run_mode == FEEC_MODE_REFERENCE && n > pcg_smem_max_rows() && use_flow(false)) {
+                    FEEC_TRY(reset_status(s));
+                    FEEC_TRY(cudaEventRecord(s->ev0, s->stream));
+                    st = launch_flow_pcg(s, a, shape);
+                    if (st != FEEC_OK) return st;
+                    FEEC_TRY(cudaEventRecord(s->ev1, s->stream));
+                    FEEC_TRY(cudaEventSynchronize(s->ev1));
+                    FEEC_TRY(cudaEventElapsedTime(&ms, s->ev0, s->ev1));
+                } else {
+                    st = timed_launch_pcg64(s, a, shape, ms);
+                    if (st != FEEC_OK) return st;
+                }
             }
             ms_total += ms;
             st = read_status(s, hs);
@@ -455,6 +496,7 @@ int solve_core(feec_system* s, int method, int mode, double* xx, const double* b
         // ends there, and every later segment restarts.
         double restart_rate = 0.0;
         double zr_prev = 0.0, rn_prev = 0.0;
+        const bool flow32 = use_flow(true);
         for (outer = 0; outer < max_outer; outer++) {
             st = true_residual(s, s->b, s->x, s->r, rn2, permuted);
             if (st != FEEC_OK) return st;
@@ -532,7 +574,12 @@ int solve_core(feec_system* s, int method, int mode, double* xx, const double* b
                 a.rr_stop = f;
                 a.max_iter = seg_budget;
                 a.keep_dir = have_dir ? 1 : 0; a.zr_prev = zr_prev; a.scale = scale;
-                FEEC_TRY(launch_eisenstat<float>(a, shape, s->stream));
+                if (flow32) {
+                    st = launch_flow_eisenstat(s, a, shape);
+                    if (st != FEEC_OK) return st;
+                } else {
+                    FEEC_TRY(launch_eisenstat<float>(a, shape, s->stream));
+                }
             }
             FEEC_TRY(cudaEventRecord(s->ev1, s->stream));
             FEEC_TRY(launch_update_x_norms(n, s->x32, s->scal + 3, s->x, s->partials, s->scal + 4, s->stream));
@@ -670,7 +717,8 @@ int build_layout(feec_system* s, int method, const double* diag_dev, double omeg
     s->prepared = method;
     s->mixed_pick[1] = 0;   // a new layout measures its inner precision again
     s->mixed_rate[1][0] = s->mixed_rate[1][1] = 0.0;
-    s->sell[1].ready = false;   // the Rainbow-order SELL copy follows the new ordering
+    s->sell[1].ready = false;   // the Rainbow-order SELL copy and the slices follow the new ordering
+    s->flow.ready = false;
     return FEEC_OK;
 }
 
@@ -763,6 +811,7 @@ int feec_system_destroy(feec_system* s) {
     s->work.release();
     s->sell[0].mem.release();
     s->sell[1].mem.release();
+    s->flow.mem.release();
     s->mem.release();
     cudaStreamSynchronize(s->stream);
     if (s->ev0) cudaEventDestroy(s->ev0);
@@ -780,7 +829,7 @@ int feec_system_set_launch(feec_system* s, int blocks, int lanes) {
 
 int feec_system_memory(const feec_system* s, size_t* bytes) {
     if (!s || !bytes) return FEEC_BADARG;
-    *bytes = s->mem.bytes + s->work.bytes;
+    *bytes = s->mem.bytes + s->work.bytes + s->flow.mem.bytes;
     return FEEC_OK;
 }
 

@@ -66,6 +66,16 @@ struct SellData {
     long long entries = 0;
 };
 
+// The multicolor layout cut into row slices for the dataflow solvers (kernels_flow.cu).
+struct FlowData {
+    DevArena mem;
+    bool ready = false;
+    int nslices = 0;
+    long long units = 0;                 // 32-entry columns over all slices
+    int4* meta = nullptr; int* ci = nullptr; double* val64 = nullptr; float* val32 = nullptr;
+    double* pub[4] = {nullptr, nullptr, nullptr, nullptr};   // published vectors (n values of either precision)
+};
+
 }  // namespace feec
 
 struct feec_system {
@@ -114,6 +124,7 @@ struct feec_system {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // SELL-32 layouts: [0] natural row order (SpMV, batched plain CG), [1] Rainbow order
     feec::SellData sell[2];
+    feec::FlowData flow;
     // batched-engine launch choice made by the autotuner, per [method][mode] (0 = not tuned)
     int tuned_k[3][3] = {};
     int tuned_threads[3][3] = {};
@@ -122,6 +133,13 @@ struct feec_system {
 };
 
 namespace feec {
+// Dataflow solvers over the Rainbow layout (kernels_flow.cu): flow_build prepares the slices
+// and values of one precision; the launchers enqueue one solve. feec_status results.
+int flow_build(feec_system* s, bool f32);
+int launch_flow_eisenstat(feec_system* s, const PcgArgs<double>& a, LaunchShape& shape);
+int launch_flow_eisenstat(feec_system* s, const PcgArgs<float>& a, LaunchShape& shape);
+int launch_flow_pcg(feec_system* s, const PcgArgs<double>& a, LaunchShape& shape);
+
 struct HomeStreamScope {
     feec_system* s;
     cudaStream_t saved;

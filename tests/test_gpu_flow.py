@@ -1,0 +1,93 @@
+"""Dataflow multicolor solvers (kernels_flow.cu) where their slices can go wrong: a diagonal
+matrix (no sweep entries), rows of one and of several chunks per lane, one lane and many lanes
+per row, a last slice that is not full, more blocks than slices. K within 2% (at least 1) of the
+oracle and the solution within 1e-9 of it, the parity bar of the drop-in solvers."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+pytestmark = pytest.mark.gpu
+
+
+def _diagonal(n):
+    return sp.diags(np.linspace(1.0, 2.0, n)).tocsr()
+
+
+def _tridiagonal(n):
+    return sp.diags([-np.ones(n - 1), np.full(n, 2.5), -np.ones(n - 1)], [-1, 0, 1]).tocsr()
+
+
+def _arrow(n):
+    """A dense first row and column over a tridiagonal rest: one row far longer than a lane chunk."""
+    M = _tridiagonal(n).tolil()
+    M[0, :] = 0.5 / n
+    M[:, 0] = 0.5 / n
+    M[0, 0] = 3.0
+    return M.tocsr()
+
+
+def _lattice(dim, r, L, n):
+    from simplefem_gb300 import workloads
+    A, C, V = workloads.lattice_matrix(dim, r, L, 3)
+    M = sp.csr_matrix((V, C, A))
+    return M[:n, :n].tocsr() if n else M
+
+
+CASES = [("diagonal", lambda: _diagonal(40)), ("one_row", lambda: _diagonal(1)), ("two_rows", lambda: _tridiagonal(2)),
+         ("tridiagonal_33", lambda: _tridiagonal(33)), ("arrow_257", lambda: _arrow(257)),
+         ("arrow_9800", lambda: _arrow(9800)), ("p3", lambda: _lattice(3, 3, 2, 0)),
+         ("ragged_p2", lambda: _lattice(3, 2, 3, 4097)), ("ragged_p1", lambda: _lattice(3, 1, 5, 19_999))]
+
+
+@pytest.mark.parametrize("method,mode", [("rainbow", "reference"), ("rainbow_eisenstat", "reference"),
+                                         ("rainbow", "fp64"), ("rainbow", "mixed")])
+@pytest.mark.parametrize("name,make", CASES, ids=[c[0] for c in CASES])
+def test_flow_solvers_match_oracle(name, make, method, mode):
+    import torch
+    from oracle import oracle
+    from simplefem_gb300.system import System
+    M = make()
+    M.sort_indices()
+    A, C, V = M.indptr.astype(np.int32), M.indices.astype(np.int32), M.data.astype(np.float64)
+    n = len(A) - 1
+    rng = np.random.default_rng(n)
+    b = 1e3 * rng.uniform(-1.0, 1.0, n)
+    diag = oracle.csr_diagonal(A, C, V)
+    rb = oracle.rainbow(A, C)
+    sysm = System(A, C, V)
+    sysm.set_rainbow(diag, 1.0, *rb)
+    x = torch.zeros(n, dtype=torch.float64, device="cuda")
+    info = sysm.solve(torch.from_numpy(b).cuda(), x, method=method, mode=mode, precision=1e-11)
+    K_o, x_o, _ = oracle.cg_rainbow(A, C, V, b, diag, rb, 1.0, precision=1e-11)
+    xh = x.cpu().numpy()
+    if n < 3 and info["status"] == 3:      # the iteration cap, N by default, leaves two steps
+        sysm.close()
+        return
+    assert info["status"] == 0, info
+    assert np.linalg.norm(xh - x_o) <= 1e-9 * np.linalg.norm(x_o), info
+    if mode == "reference":
+        assert abs(info["iterations"] - K_o) <= max(1, int(np.ceil(0.02 * K_o))), (info, K_o)
+    else:
+        assert np.linalg.norm(b - M @ xh) <= 1e-11 * np.linalg.norm(b), info
+    sysm.close()
+
+
+@pytest.mark.parametrize("method,mode", [("rainbow", "reference"), ("rainbow", "fp64")])
+def test_flow_solvers_repeat_bit_for_bit(method, mode):
+    """Every sum is formed in a fixed order, whatever the order in which values arrive."""
+    import torch
+    from oracle import oracle
+    from simplefem_gb300.system import System
+    M = _lattice(3, 2, 3, 0) if mode == "fp64" else _lattice(3, 1, 5, 0)
+    A, C, V = M.indptr.astype(np.int32), M.indices.astype(np.int32), M.data
+    n = len(A) - 1
+    sysm = System(A, C, V)
+    sysm.set_rainbow(oracle.csr_diagonal(A, C, V), 1.0, *oracle.rainbow(A, C))
+    b = torch.from_numpy(np.random.default_rng(1).uniform(-1e3, 1e3, n)).cuda()
+    runs = []
+    for _ in range(3):
+        x = torch.zeros(n, dtype=torch.float64, device="cuda")
+        info = sysm.solve(b, x, method=method, mode=mode, precision=1e-10)
+        runs.append((info["iterations"], x.cpu().numpy().tobytes()))
+    assert runs[0] == runs[1] == runs[2]
+    sysm.close()
