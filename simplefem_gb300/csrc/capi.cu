@@ -217,6 +217,15 @@ bool flow_prepare(feec_system* s, bool f32) {
     return false;
 }
 
+bool flow_cg_prepare(feec_system* s, bool f32) {
+    if (flow_cg_build(s, f32) == FEEC_OK) return true;
+    cudaGetLastError();
+    s->flow_cg.mem.release();
+    s->flow_cg = FlowData{};
+    s->flow_cg.mem.stream = s->home_stream;
+    return false;
+}
+
 // Core solve on a prepared system. xx / bb / res: device arrays in the ORIGINAL numbering.
 // tol_override > 0 replaces the tolerance of REFERENCE mode (the drop-in computes it on the host
 // with the reference's own serial loop).
@@ -298,12 +307,17 @@ int solve_core(feec_system* s, int method, int mode, double* xx, const double* b
     else if (s->nnz < 60000) shape.blocks = 16;
     if (s->user_lanes > 0) shape.lanes = s->user_lanes;
     if (s->user_blocks > 0) shape.blocks = s->user_blocks;
-    // Multicolor layouts run the dataflow solvers (kernels_flow.cu); the barrier-phase kernels
-    // keep index-order layouts, rows with D == 0 (never computed, so never published), caller
-    // launch shapes, and systems whose slices do not fit the device memory.
+    // Multicolor layouts and plain CG run the dataflow solvers (kernels_flow.cu,
+    // kernels_flow_cg.cu); the barrier-phase kernels keep index-order layouts, the diagonal
+    // preconditioner, rows with D == 0 (never computed, so never published), caller launch shapes,
+    // and systems whose slices do not fit the device memory.
     auto use_flow = [&](bool f32) {
         return layout == FEEC_METHOD_RAINBOW && s->zero_diag_rows == 0 && s->user_blocks <= 0 && s->user_lanes <= 0 &&
                flow_prepare(s, f32);
+    };
+    auto use_flow_cg = [&](bool f32) {
+        return method == FEEC_METHOD_CG && s->user_blocks <= 0 && s->user_lanes <= 0 &&
+               flow_cg_prepare(s, f32);
     };
     float ms_total = 0.0f;
     int K_total = 0, outer = 0, status = FEEC_OK;
@@ -338,9 +352,15 @@ int solve_core(feec_system* s, int method, int mode, double* xx, const double* b
                 a.max_iter = max_iter - (K_total - k0);
                 a.print_modulo = print_modulo; a.print_tol = tolerance;
                 a.partials = s->partials; a.st = s->st;
+                const bool flow = use_flow_cg(false);
                 FEEC_TRY(reset_status(s));
                 FEEC_TRY(cudaEventRecord(s->ev0, s->stream));
-                FEEC_TRY(launch_cg<double>(a, shape, s->stream));
+                if (flow) {
+                    st = launch_flow_cg(s, a, shape);
+                    if (st != FEEC_OK) return st;
+                } else {
+                    FEEC_TRY(launch_cg<double>(a, shape, s->stream));
+                }
                 FEEC_TRY(cudaEventRecord(s->ev1, s->stream));
                 FEEC_TRY(cudaEventSynchronize(s->ev1));
                 FEEC_TRY(cudaEventElapsedTime(&ms, s->ev0, s->ev1));
@@ -496,7 +516,7 @@ int solve_core(feec_system* s, int method, int mode, double* xx, const double* b
         // ends there, and every later segment restarts.
         double restart_rate = 0.0;
         double zr_prev = 0.0, rn_prev = 0.0;
-        const bool flow32 = use_flow(true);
+        const bool flow32 = method == FEEC_METHOD_CG ? use_flow_cg(true) : use_flow(true);
         for (outer = 0; outer < max_outer; outer++) {
             st = true_residual(s, s->b, s->x, s->r, rn2, permuted);
             if (st != FEEC_OK) return st;
@@ -557,7 +577,12 @@ int solve_core(feec_system* s, int method, int mode, double* xx, const double* b
                 a.max_iter = seg_budget;
                 a.partials = s->partials; a.st = s->st;
                 a.keep_dir = have_dir ? 1 : 0; a.zr_prev = zr_prev; a.scale = scale;
-                FEEC_TRY(launch_cg<float>(a, shape, s->stream));
+                if (flow32) {
+                    st = launch_flow_cg(s, a, shape);
+                    if (st != FEEC_OK) return st;
+                } else {
+                    FEEC_TRY(launch_cg<float>(a, shape, s->stream));
+                }
             } else {
                 // The inner multicolor / index-order SSOR-PCG runs in Eisenstat's formulation:
                 // the same preconditioned iterates, but an iteration is one backward and one
@@ -812,6 +837,7 @@ int feec_system_destroy(feec_system* s) {
     s->sell[0].mem.release();
     s->sell[1].mem.release();
     s->flow.mem.release();
+    s->flow_cg.mem.release();
     s->mem.release();
     cudaStreamSynchronize(s->stream);
     if (s->ev0) cudaEventDestroy(s->ev0);
@@ -829,7 +855,7 @@ int feec_system_set_launch(feec_system* s, int blocks, int lanes) {
 
 int feec_system_memory(const feec_system* s, size_t* bytes) {
     if (!s || !bytes) return FEEC_BADARG;
-    *bytes = s->mem.bytes + s->work.bytes + s->flow.mem.bytes;
+    *bytes = s->mem.bytes + s->work.bytes + s->flow.mem.bytes + s->flow_cg.mem.bytes;
     return FEEC_OK;
 }
 

@@ -74,7 +74,20 @@ struct FlowData {
     long long units = 0;                 // 32-entry columns over all slices
     int4* meta = nullptr; int* ci = nullptr; double* val64 = nullptr; float* val32 = nullptr;
     double* pub[4] = {nullptr, nullptr, nullptr, nullptr};   // published vectors (n values of either precision)
+    // plain CG (kernels_flow_cg.cu): rows in its own order, work vectors in that order
+    int longest = 0;                     // entries per lane of the longest slice
+    int* perm = nullptr; int* iperm = nullptr;
+    double* own[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
 };
+
+struct FlowHostSlice {
+    int row0, nrow, shift, len;          // len: entries per lane
+};
+// Cuts rows [lo, hi) with len[i] entries into slices of at most `longest` entries per lane (up to
+// 32 lanes per row), lanes per row by the modelled time of one pass over them; false (out empty)
+// when every choice needs more than max_slices (kernels_flow.cu).
+bool flow_cut_rows(int lo, int hi, const int* len, int row_ops, int sms, int longest, int max_slices,
+                   std::vector<FlowHostSlice>& out);
 
 }  // namespace feec
 
@@ -124,7 +137,8 @@ struct feec_system {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // SELL-32 layouts: [0] natural row order (SpMV, batched plain CG), [1] Rainbow order
     feec::SellData sell[2];
-    feec::FlowData flow;
+    feec::FlowData flow;               // multicolor layout
+    feec::FlowData flow_cg;            // natural layout, plain CG
     // batched-engine launch choice made by the autotuner, per [method][mode] (0 = not tuned)
     int tuned_k[3][3] = {};
     int tuned_threads[3][3] = {};
@@ -139,6 +153,10 @@ int flow_build(feec_system* s, bool f32);
 int launch_flow_eisenstat(feec_system* s, const PcgArgs<double>& a, LaunchShape& shape);
 int launch_flow_eisenstat(feec_system* s, const PcgArgs<float>& a, LaunchShape& shape);
 int launch_flow_pcg(feec_system* s, const PcgArgs<double>& a, LaunchShape& shape);
+// Plain CG (kernels_flow_cg.cu).
+int flow_cg_build(feec_system* s, bool f32);
+int launch_flow_cg(feec_system* s, const CgArgs<double>& a, LaunchShape& shape);
+int launch_flow_cg(feec_system* s, const CgArgs<float>& a, LaunchShape& shape);
 
 struct HomeStreamScope {
     feec_system* s;

@@ -84,9 +84,19 @@ __device__ __forceinline__ FlowSlice flow_slice(const int4 m) {
     return f;
 }
 
+// The lane's row of a slice: lane 0 of the row's group owns the row.
+struct FlowRow {
+    int i;
+    bool own;
+};
+__device__ __forceinline__ FlowRow flow_row(const FlowSlice& s, int lane) {
+    const int k = lane >> s.shift;
+    return FlowRow{s.row0 + k, k < s.nrow && (lane & ((1 << s.shift) - 1)) == 0};
+}
+
 // A wait's bound: polls are counted, and every 4096 of them the abort flag and the clock are
 // looked at. Returns false once the wait has to be given up (status and abort are set).
-__device__ __noinline__ bool flow_wait_goes_on(DeviceStatus* st, unsigned long long& t0, int site) {
+static __device__ __noinline__ bool flow_wait_goes_on(DeviceStatus* st, unsigned long long& t0, int site) {
     if (ld_volatile_i32(&st->abort)) return false;
     const unsigned long long t = globaltimer_ns();
     if (t0 == 0) t0 = t;
@@ -105,7 +115,7 @@ struct FlowWarp {
     __device__ __forceinline__ void init(const int4* m, int nslices) {
         meta = m;
         lane = threadIdx.x & 31;
-        nw = gridDim.x * kFlowWarps;
+        nw = gridDim.x * (blockDim.x >> 5);
         gw = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
         mine = gw < nslices ? (nslices - 1 - gw) / nw + 1 : 0;
     }
@@ -155,39 +165,44 @@ struct FlowGather {
                                           const FlowCols& cols, long long next_off, int next_len, int lane, const T* X) {
         request(ci, val, off, 0, len, cols, next_off, next_len, lane, X);
     }
+    // Waits for the chunk in flight (m entries of it, at most kFlowChunk) and subtracts it.
+    __device__ __forceinline__ T wait(const FlowCols& cols, int m, const T* X, T acc, DeviceStatus* st, int site,
+                                      bool& live) {
+        unsigned spins = 0;
+        unsigned long long t0 = 0;
+        #pragma unroll
+        for (int b = 0; b < kFlowChunk; b += 4) {
+            if (b < m) {
+                while (live) {
+                    int missing = is_sentinel(g[b]) || is_sentinel(g[b + 1]) || is_sentinel(g[b + 2]) ||
+                                  is_sentinel(g[b + 3]);
+                    asm volatile("" : "+r"(missing));     // one vote for all lanes, whatever their columns
+                    if (!__any_sync(0xffffffffu, missing)) break;
+                    if ((++spins & 4095u) == 0) {
+                        if (!flow_wait_goes_on(st, t0, site)) live = false;
+                        live = __all_sync(0xffffffffu, live);
+                    }
+                    #pragma unroll
+                    for (int u = b; u < kFlowChunk; u++)
+                        if (is_sentinel(g[u])) g[u] = ld_flow(X + cols.c[u]);
+                }
+                switch (m - b) {
+                    default: acc = fma(-v[b], g[b], acc); acc = fma(-v[b + 1], g[b + 1], acc);
+                             acc = fma(-v[b + 2], g[b + 2], acc); acc = fma(-v[b + 3], g[b + 3], acc); break;
+                    case 3: acc = fma(-v[b], g[b], acc); acc = fma(-v[b + 1], g[b + 1], acc);
+                            acc = fma(-v[b + 2], g[b + 2], acc); break;
+                    case 2: acc = fma(-v[b], g[b], acc); acc = fma(-v[b + 1], g[b + 1], acc); break;
+                    case 1: acc = fma(-v[b], g[b], acc); break;
+                }
+            }
+        }
+        return acc;
+    }
     __device__ __forceinline__ T finish(const int* __restrict__ ci, const T* __restrict__ val, long long off, int len,
                                         FlowCols& cols, long long next_off, int next_len, int lane, const T* X, T acc,
                                         DeviceStatus* st, int site, bool& live) {
         for (int k0 = 0;;) {
-            const int m = len - k0;
-            unsigned spins = 0;
-            unsigned long long t0 = 0;
-            #pragma unroll
-            for (int b = 0; b < kFlowChunk; b += 4) {
-                if (b < m) {
-                    while (live) {
-                        int missing = is_sentinel(g[b]) || is_sentinel(g[b + 1]) || is_sentinel(g[b + 2]) ||
-                                      is_sentinel(g[b + 3]);
-                        asm volatile("" : "+r"(missing));     // one vote for all lanes, whatever their columns
-                        if (!__any_sync(0xffffffffu, missing)) break;
-                        if ((++spins & 4095u) == 0) {
-                            if (!flow_wait_goes_on(st, t0, site)) live = false;
-                            live = __all_sync(0xffffffffu, live);
-                        }
-                        #pragma unroll
-                        for (int u = b; u < kFlowChunk; u++)
-                            if (is_sentinel(g[u])) g[u] = ld_flow(X + cols.c[u]);
-                    }
-                    switch (m - b) {
-                        default: acc = fma(-v[b], g[b], acc); acc = fma(-v[b + 1], g[b + 1], acc);
-                                 acc = fma(-v[b + 2], g[b + 2], acc); acc = fma(-v[b + 3], g[b + 3], acc); break;
-                        case 3: acc = fma(-v[b], g[b], acc); acc = fma(-v[b + 1], g[b + 1], acc);
-                                acc = fma(-v[b + 2], g[b + 2], acc); break;
-                        case 2: acc = fma(-v[b], g[b], acc); acc = fma(-v[b + 1], g[b + 1], acc); break;
-                        case 1: acc = fma(-v[b], g[b], acc); break;
-                    }
-                }
-            }
+            acc = wait(cols, len - k0, X, acc, st, site, live);
             cols = ahead;
             k0 += kFlowChunk;
             if (k0 >= len) return acc;
@@ -233,6 +248,18 @@ __device__ __forceinline__ T row_sum(T s, int shift) {
     return s;
 }
 
+// |a| < bound and a < 0 on the bits (bound > 0): the control thread's FP64 comparisons would
+// take 64 cycles each. Both are false for NaN, as the comparisons are.
+__device__ __forceinline__ bool abs_below(double a, double bound) {
+    return (__double_as_longlong(a) & 0x7fffffffffffffffll) < __double_as_longlong(bound);
+}
+__device__ __forceinline__ bool below_zero(double a) {
+    const long long b = __double_as_longlong(a);
+    return b < 0 && (b << 1) != 0 && (unsigned long long)(b << 1) <= 0xffe0000000000000ull;
+}
+// sqrt|a| < the reference's machine epsilon 2^-52 (sparsesolver.cpp:153-157)
+__device__ __forceinline__ bool energy_small(double a) { return abs_below(a, 4.9303806576313238e-32); }
+
 // a * b added to a running sum: FP64 by one fused operation; FP32 with the product's
 // rounding error kept (fma(a, b, -ab) is exact) in the compensated pair.
 __device__ __forceinline__ double acc_product(double acc, double a, double b) { return fma(a, b, acc); }
@@ -244,57 +271,26 @@ __device__ __forceinline__ CompF acc_product(CompF acc, float a, float b) {
 }
 
 struct FlowShared {
-    double warp_sum[kFlowWarps][4];
+    double warp_sum[32][4];   // a block has at most 32 warps
     double total[4][4];
     int ok;
 };
 
-// Grid-wide sums of NV (at most 4) accumulators per thread, which is also the iteration's
-// barrier: everything written before it in any block is visible after it in every block.
-// The totals are returned to thread 0 of every block (identical bits in every block: fixed
-// shuffle trees and a fixed order over blocks). With four sums the warp's tree halves the
-// number of values each step (6 additions instead of 20: an FP64 addition costs a warp 64
-// cycles). `part` must not be one that some block may still be reading (callers alternate
-// two). Returns false in every thread when a wait gave up here or, `live` false, before.
-template <typename T, int NV>
-__device__ __forceinline__ bool flow_reduce(typename AccT<T>::type (&v)[NV], double* part, DeviceStatus* st,
-                                            unsigned long long& epoch, int site, bool live, FlowShared& sh,
-                                            double (&tot)[NV]) {
-    static_assert(NV == 1 || NV == 2 || NV == 4, "sums per reduction");
-    using A = AccT<T>;
-    using Acc = typename A::type;
-    static_assert(kFlowWarps % 8 == 0, "eight warps' sums per shuffle row");
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    Acc k = v[0];
-    int idx = 0, rest = 16;
-    if constexpr (NV == 4) {
-        const bool hi = lane & 16;
-        Acc k0 = A::merge(hi ? v[2] : v[0], A::shfl_xor(hi ? v[0] : v[2], 16));
-        Acc k1 = A::merge(hi ? v[3] : v[1], A::shfl_xor(hi ? v[1] : v[3], 16));
-        const bool mid = lane & 8;
-        k = A::merge(mid ? k1 : k0, A::shfl_xor(mid ? k0 : k1, 8));
-        idx = (hi ? 2 : 0) + (mid ? 1 : 0);
-        rest = 4;
-    } else if constexpr (NV == 2) {
-        const bool hi = lane & 16;
-        k = A::merge(hi ? v[1] : v[0], A::shfl_xor(hi ? v[0] : v[1], 16));
-        idx = hi ? 1 : 0;
-        rest = 8;
-    }
-    for (int off = rest; off > 0; off >>= 1) k = A::merge(k, A::shfl_xor(k, off));
-    if ((lane & (2 * rest - 1)) == 0) sh.warp_sum[warp][idx] = A::value(k);
+// The block's and the grid's part of flow_reduce: every warp has put its NV sums into
+// sh.warp_sum[warp].
+template <int NV>
+__device__ __forceinline__ bool flow_reduce_warps(double* part, DeviceStatus* st, unsigned long long& epoch, int site,
+                                                  bool live, FlowShared& sh, double (&tot)[NV]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const int dead = __syncthreads_or(live ? 0 : 1);   // also orders the block's writes before the release
     if (dead) return false;
     const int nb = gridDim.x;
     if (warp == 0) {
         const int i = lane & 3;
-        double a = 0.0;
-        if (i < NV) {
-            #pragma unroll
-            for (int w = 0; w < kFlowWarps; w += 8) a += sh.warp_sum[w + (lane >> 2)][i];
-        }
-        #pragma unroll
-        for (int off = 4; off < 32; off <<= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
+        double a = i < NV && (lane >> 2) < warps ? sh.warp_sum[lane >> 2][i] : 0.0;
+        for (int w = (lane >> 2) + 8; w < warps; w += 8)
+            if (i < NV) a += sh.warp_sum[w][i];
+        for (int off = 4; off < 4 * warps && off < 32; off <<= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
         if (lane < NV) {
             if (nb == 1) sh.total[0][lane] = a;
             else part[4 * blockIdx.x + lane] = a;
@@ -317,12 +313,21 @@ __device__ __forceinline__ bool flow_reduce(typename AccT<T>::type (&v)[NV], dou
         __syncthreads();
         return true;
     }
-    if (warp < 4) {
+    const int readers = warps < 4 ? warps : 4;
+    if (warp < readers) {
         const int i = lane & 3;
         double a = 0.0;
-        if (i < NV) {
-            #pragma unroll 5
-            for (int b = warp * 8 + (lane >> 2); b < nb; b += 32) a += __ldcg(&part[4 * b + i]);
+        // five blocks' partials requested together (all of them on 152 blocks), then added
+        for (int b0 = warp * 8 + (lane >> 2); b0 < nb; b0 += 40 * readers) {
+            double p[5];
+            #pragma unroll
+            for (int k = 0; k < 5; k++) {
+                const int b = b0 + 8 * readers * k;
+                p[k] = i < NV && b < nb ? __ldcg(&part[4 * b + i]) : 0.0;
+            }
+            #pragma unroll
+            for (int k = 0; k < 5; k++)
+                if (b0 - (lane >> 2) + 8 * readers * k < nb) a += p[k];
         }
         #pragma unroll
         for (int off = 4; off < 32; off <<= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
@@ -331,11 +336,48 @@ __device__ __forceinline__ bool flow_reduce(typename AccT<T>::type (&v)[NV], dou
     __syncthreads();
     if (warp == 0) {
         const int i = lane & 3;
-        const double a = i < NV ? (sh.total[0][i] + sh.total[1][i]) + (sh.total[2][i] + sh.total[3][i]) : 0.0;
+        double a = i < NV ? sh.total[0][i] : 0.0;
+        for (int w = 1; w < readers; w++) a += i < NV ? sh.total[w][i] : 0.0;
         #pragma unroll
         for (int j = 0; j < NV; j++) tot[j] = __shfl_sync(0xffffffffu, a, j);
     }
     return true;
+}
+
+// Grid-wide sums of NV (at most 4) accumulators per thread, which is also the iteration's
+// barrier: everything written before it in any block is visible after it in every block.
+// The totals are returned to warp 0 of every block (identical bits in every block: fixed
+// shuffle trees and a fixed order over blocks). With four sums the warp's tree halves the
+// number of values each step (6 additions instead of 20: an FP64 addition costs a warp 64
+// cycles). `part` must not be one that some block may still be reading (callers alternate
+// two). Returns false in every thread when a wait gave up here or, `live` false, before.
+template <typename T, int NV>
+__device__ __forceinline__ bool flow_reduce(typename AccT<T>::type (&v)[NV], double* part, DeviceStatus* st,
+                                            unsigned long long& epoch, int site, bool live, FlowShared& sh,
+                                            double (&tot)[NV]) {
+    static_assert(NV == 1 || NV == 2 || NV == 4, "sums per reduction");
+    using A = AccT<T>;
+    using Acc = typename A::type;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    Acc k = v[0];
+    int idx = 0, rest = 16;
+    if constexpr (NV == 4) {
+        const bool hi = lane & 16;
+        Acc k0 = A::merge(hi ? v[2] : v[0], A::shfl_xor(hi ? v[0] : v[2], 16));
+        Acc k1 = A::merge(hi ? v[3] : v[1], A::shfl_xor(hi ? v[1] : v[3], 16));
+        const bool mid = lane & 8;
+        k = A::merge(mid ? k1 : k0, A::shfl_xor(mid ? k0 : k1, 8));
+        idx = (hi ? 2 : 0) + (mid ? 1 : 0);
+        rest = 4;
+    } else if constexpr (NV == 2) {
+        const bool hi = lane & 16;
+        k = A::merge(hi ? v[1] : v[0], A::shfl_xor(hi ? v[0] : v[1], 16));
+        idx = hi ? 1 : 0;
+        rest = 8;
+    }
+    for (int off = rest; off > 0; off >>= 1) k = A::merge(k, A::shfl_xor(k, off));
+    if ((lane & (2 * rest - 1)) == 0) sh.warp_sum[warp][idx] = A::value(k);
+    return flow_reduce_warps<NV>(part, st, epoch, site, live, sh, tot);
 }
 
 }  // namespace feec

@@ -48,16 +48,6 @@ struct FlowArgs {
     double zr_prev, scale;
 };
 
-// The lane's row of a slice: lane 0 of the row's group owns the row.
-struct FlowRow {
-    int i;
-    bool own;
-};
-__device__ __forceinline__ FlowRow flow_row(const FlowSlice& s, int lane) {
-    const int k = lane >> s.shift;
-    return FlowRow{s.row0 + k, k < s.nrow && (lane & ((1 << s.shift) - 1)) == 0};
-}
-
 enum { kGoOn = 0, kBreakdown = 1, kSmallEnergy = 2, kConverged = 3, kLastStep = 4 };
 
 // ---------------------------------------------------------------------------
@@ -200,11 +190,11 @@ __global__ void __launch_bounds__(kFlowThreads, 1) flow_eisenstat(FlowArgs<T> a)
             if (K > 0) {
                 if (a.print_modulo > 0 && K % a.print_modulo == 0 && blockIdx.x == 0)
                     printf("(%d/%d)   INTERIM: Residual norm is %.9le < %.9le\n", K, a.n, sqrt(z_r), a.print_tol);
-                if (a.use_zr_rule && fabs(z_r) < a.tol2) ctl = kConverged;
+                if (a.use_zr_rule && abs_below(z_r, a.tol2)) ctl = kConverged;
                 if (a.rr_stop > 0.0 && z_r < a.rr_stop * z_r0) ctl = kConverged;
             }
-            const bool bad = !isfinite(z_r) || z_r < 0.0 || !isfinite(d_Ad) || d_Ad < 0.0;     // :918-933
-            const bool tiny = !bad && sqrt(fabs(d_Ad)) < kMachineEpsilon;
+            const bool bad = !isfinite(z_r) || below_zero(z_r) || !isfinite(d_Ad) || below_zero(d_Ad);   // :918-933
+            const bool tiny = !bad && energy_small(d_Ad);
             if (ctl == kConverged) {
                 // an inner solve (no reference rule) takes the step it has already paid for
                 if (!a.use_zr_rule && !bad && !tiny) ctl = kLastStep;
@@ -330,7 +320,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) flow_pcg(FlowArgs<double> a) 
         if (threadIdx.x == 0) {
             if (a.print_modulo > 0 && K % a.print_modulo == 0 && blockIdx.x == 0)
                 printf("(%d/%d)   INTERIM: Residual norm is %.9le < %.9le\n", K, a.n, sqrt(z_r), a.print_tol);
-            s_ctl = (a.use_zr_rule && fabs(z_r) < a.tol2) ? kConverged : kGoOn;           // :1187-1190
+            s_ctl = (a.use_zr_rule && abs_below(z_r, a.tol2)) ? kConverged : kGoOn;       // :1187-1190
         }
         __syncthreads();
         if (s_ctl == kConverged) { status = FEEC_OK; break; }
@@ -365,8 +355,8 @@ __global__ void __launch_bounds__(kFlowThreads, 1) flow_pcg(FlowArgs<double> a) 
         if (threadIdx.x == 0) {
             const double d_Ad = tot[0];
             int ctl = kGoOn;
-            if (!isfinite(z_r) || z_r < 0.0 || !isfinite(d_Ad) || d_Ad < 0.0) ctl = kBreakdown;
-            else if (sqrt(fabs(d_Ad)) < kMachineEpsilon) ctl = kSmallEnergy;
+            if (!isfinite(z_r) || below_zero(z_r) || !isfinite(d_Ad) || below_zero(d_Ad)) ctl = kBreakdown;
+            else if (energy_small(d_Ad)) ctl = kSmallEnergy;
             s_ctl = ctl;
             s_scal[0] = z_r / d_Ad;
         }
@@ -484,6 +474,45 @@ double slice_rows(int lo, int hi, const int* rp, const int* ls, const int* us, i
 }
 
 }  // namespace
+
+bool flow_cut_rows(int lo, int hi, const int* len, int row_ops, int sms, int longest, int max_slices,
+                   std::vector<FlowHostSlice>& out) {
+    auto lanes = [](int entries, int most) {
+        int shift = 0;
+        while (shift < 5 && part_per_lane(entries, shift) > most) shift++;
+        return shift;
+    };
+    int best = 0;
+    double cost = -1.0;
+    if (hi - lo > 32 * 64 * sms) {
+        best = longest;      // many rows: few lanes each, without weighing the alternatives row by row
+    } else {
+        for (int most : {1, 2, 4, 8, 16, 32}) {
+            if (most > longest) break;
+            double chain = 0.0, ops = 0.0;
+            int slices = 0;
+            for (int i = lo; i < hi; slices++) {
+                const int shift = lanes(len[i], most);
+                const int p = part_per_lane(len[i], shift), chunks = (p + kFlowChunk - 1) / kFlowChunk;
+                chain = std::max(chain, 64.0 * (p + 1) + 92.0 * shift + 500.0 * chunks);
+                ops += p + shift + row_ops;
+                i += 32 >> shift;
+            }
+            const double v = std::max(chain, 19.0 * ops / sms);
+            if (slices <= max_slices && (cost < 0.0 || v < cost)) { cost = v; best = most; }
+        }
+    }
+    out.clear();
+    if (best == 0) return false;
+    for (int i = lo; i < hi;) {
+        FlowHostSlice s{i, 0, lanes(len[i], best), 0};
+        for (; i < hi && s.nrow < (32 >> s.shift) && lanes(len[i], best) <= s.shift; i++, s.nrow++)
+            s.len = std::max(s.len, part_per_lane(len[i], s.shift));
+        out.push_back(s);
+        if ((int)out.size() > max_slices) { out.clear(); return false; }
+    }
+    return true;
+}
 
 // Builds the slices of the multicolor layout (lazily, kept until the layout changes) and the
 // values of the wanted precision.

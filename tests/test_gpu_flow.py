@@ -72,7 +72,50 @@ def test_flow_solvers_match_oracle(name, make, method, mode):
     sysm.close()
 
 
-@pytest.mark.parametrize("method,mode", [("rainbow", "reference"), ("rainbow", "fp64")])
+CG_CASES = CASES + [("tridiagonal_5000", lambda: _tridiagonal(5000)), ("p1_2d", lambda: _lattice(2, 1, 6, 0)),
+                    ("many_rows_published", lambda: _lattice(3, 1, 5, 30_011)),
+                    ("many_rows_barrier", lambda: _lattice(3, 1, 6, 80_033)), ("long_rows_barrier", lambda: _lattice(3, 2, 5, 81_001))]
+
+
+@pytest.mark.parametrize("mode", ["reference", "fp64", "mixed"])
+@pytest.mark.parametrize("name,make", CG_CASES, ids=[c[0] for c in CG_CASES])
+def test_flow_cg_matches_oracle(name, make, mode):
+    import torch
+    from oracle import oracle
+    from simplefem_gb300.system import System
+    M = make()
+    M.sort_indices()
+    A, C, V = M.indptr.astype(np.int32), M.indices.astype(np.int32), M.data.astype(np.float64)
+    n = len(A) - 1
+    rng = np.random.default_rng(n + 1)
+    b, x0 = 1e3 * rng.uniform(-1.0, 1.0, n), 1e3 * rng.uniform(-1.0, 1.0, n)
+    sysm = System(A, C, V)
+    x = torch.from_numpy(x0).cuda()
+    r = torch.zeros(n, dtype=torch.float64, device="cuda")
+    # the reference rule is capped at N steps; the product modes get room beyond that
+    info = sysm.solve(torch.from_numpy(b).cuda(), x, method="cg", mode=mode, precision=1e-12, residual=r,
+                      max_iter=0 if mode == "reference" else 10 * n + 100)
+    xh, rh = x.cpu().numpy(), r.cpu().numpy()
+    K_o, x_o, _ = oracle.cg(A, C, V, b, x0=x0, precision=1e-12)
+    assert info["status"] == (3 if mode == "reference" and K_o == n else 0), (info, K_o)
+    assert np.linalg.norm(xh - x_o) <= 1e-9 * np.linalg.norm(x_o), info
+    assert np.linalg.norm(rh - (b - M @ xh)) <= 1e-6 * np.linalg.norm(b), info     # the drop-in's bar
+    if mode == "reference":
+        assert abs(info["iterations"] - K_o) <= max(1, int(np.ceil(0.02 * K_o))), (info, K_o)
+    else:
+        assert np.linalg.norm(b - M @ xh) <= 1e-12 * np.linalg.norm(b), info
+    # a capped solve stops after exactly that many steps, with x and r of that step
+    if mode == "reference" and K_o > 6:
+        x = torch.from_numpy(x0).cuda()
+        info = sysm.solve(torch.from_numpy(b).cuda(), x, method="cg", mode=mode, precision=1e-12, max_iter=5, residual=r)
+        xh, rh = x.cpu().numpy(), r.cpu().numpy()
+        assert info["status"] == 3 and info["iterations"] == 5, info
+        true = b - M @ xh
+        assert np.linalg.norm(rh - true) <= 1e-12 * max(np.linalg.norm(b), np.linalg.norm(M @ x0)), info
+    sysm.close()
+
+
+@pytest.mark.parametrize("method,mode", [("rainbow", "reference"), ("rainbow", "fp64"), ("cg", "reference")])
 def test_flow_solvers_repeat_bit_for_bit(method, mode):
     """Every sum is formed in a fixed order, whatever the order in which values arrive."""
     import torch
