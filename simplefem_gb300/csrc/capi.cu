@@ -154,30 +154,12 @@ PcgArgs<T> make_pcg_args(feec_system* s, T* x, T* r, T* d, T* z, T* m, T* q, con
 
 int timed_launch_pcg64(feec_system* s, const PcgArgs<double>& a, LaunchShape& shape, float& ms) {
     FEEC_TRY(reset_status(s));
-    // Systems whose three gathered vectors fit one block's shared memory run in one block
-    // (2D P1 refined 6 times: the index-order SSOR sweeps are 258 dependent level phases
-    // per iteration, which one block with shared-memory vectors turns into block barriers
-    // and shared-memory round trips).
-    const bool small = s->user_blocks <= 0 && s->user_lanes <= 0 && a.n <= pcg_smem_max_rows();
-    const bool warp = small && pcg_smem_warp_sweeps(a.n, a.nf, a.nbw);
-    PcgArgs<double> ax = a;
-    if (warp) {
-        // per-row sweep records in sweep order, rebuilt for every solve (they hold omega / D)
-        if (!s->sweep_rec) {
-            HomeStreamScope home(s);
-            FEEC_TRY(s->work.alloc(s->sweep_rec, sweep_record_bytes(a.n)));
-        }
-        FEEC_TRY(launch_build_sweep_records(a, s->sweep_rec, s->stream));
-        ax.sweep_fwd = s->sweep_rec;
-        ax.sweep_bwd = s->sweep_rec + sweep_record_bytes(a.n) / 2;
-    }
+    // Small systems run in one block with the gathered vectors in its shared memory.
+    const bool small = s->user_blocks <= 0 && s->user_lanes <= 0 && small_pcg_fits(s) && small_pcg_prepare(s) == FEEC_OK;
     FEEC_TRY(cudaEventRecord(s->ev0, s->stream));
     if (small) {
-        const double avg = (double)s->nnz / (double)(a.n > 0 ? a.n : 1);
-        shape.lanes = avg <= 10.0 ? 1 : avg <= 20.0 ? 2 : avg <= 40.0 ? 4 : 8;
-        shape.blocks = 1;
-        shape.threads = warp ? 256 : pcg_smem_threads(s->max_phase_rows, shape.lanes);
-        FEEC_TRY(launch_pcg_smem(ax, shape.lanes, shape.threads, s->stream));
+        const int e = launch_small_pcg(s, a, shape);
+        if (e != FEEC_OK) return e;
     } else {
         FEEC_TRY(launch_pcg<double>(a, shape, s->stream));
     }
@@ -431,8 +413,8 @@ int solve_core(feec_system* s, int method, int mode, double* xx, const double* b
                 a.rr_stop = (run_mode == FEEC_MODE_FP64) ? tolerance * tolerance : 0.0;
                 a.max_iter = max_iter - (K_total - k0);
                 a.print_modulo = print_modulo; a.print_tol = tolerance;
-                // below pcg_smem_max_rows() the one-block solver (timed_launch_pcg64)
-                if (run_mode == FEEC_MODE_REFERENCE && n > pcg_smem_max_rows() && use_flow(false)) {
+                // small systems: the one-block solver (timed_launch_pcg64)
+                if (run_mode == FEEC_MODE_REFERENCE && !small_pcg_fits(s) && use_flow(false)) {
                     FEEC_TRY(reset_status(s));
                     FEEC_TRY(cudaEventRecord(s->ev0, s->stream));
                     st = launch_flow_pcg(s, a, shape);
@@ -744,6 +726,7 @@ int build_layout(feec_system* s, int method, const double* diag_dev, double omeg
     s->mixed_rate[1][0] = s->mixed_rate[1][1] = 0.0;
     s->sell[1].ready = false;   // the Rainbow-order SELL copy and the slices follow the new ordering
     s->flow.ready = false;
+    small_release(s);
     return FEEC_OK;
 }
 
@@ -838,6 +821,7 @@ int feec_system_destroy(feec_system* s) {
     s->sell[1].mem.release();
     s->flow.mem.release();
     s->flow_cg.mem.release();
+    small_release(s);
     s->mem.release();
     cudaStreamSynchronize(s->stream);
     if (s->ev0) cudaEventDestroy(s->ev0);

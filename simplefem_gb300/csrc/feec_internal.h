@@ -49,10 +49,6 @@ struct CgArgs {
     // the kernel leaves its last rho_prev in st->extra[0]
     int keep_dir;
     double zr_prev, scale;
-    // one-block solver with one-warp sweeps (kernels_small.cu): per-row sweep records in
-    // forward and backward sweep order, built by launch_build_sweep_records
-    const void* sweep_fwd;
-    const void* sweep_bwd;
 };
 
 template <typename T>
@@ -87,10 +83,6 @@ struct PcgArgs {
     // restart); the kernel leaves its last rho_prev in st->extra[0]
     int keep_dir;
     double zr_prev, scale;
-    // one-block solver with one-warp sweeps (kernels_small.cu): per-row sweep records in
-    // forward and backward sweep order, built by launch_build_sweep_records
-    const void* sweep_fwd;
-    const void* sweep_bwd;
 };
 
 // Rows with more stored entries than this count as long in a multicolor layout: the
@@ -108,14 +100,6 @@ template <typename T> cudaError_t launch_cg(const CgArgs<T>& a, LaunchShape& sha
 template <typename T> cudaError_t launch_pcg(const PcgArgs<T>& a, LaunchShape& shape, cudaStream_t s);
 // SSOR-PCG with Eisenstat's trick over the same phase schedules (kernels_eisenstat.cu).
 template <typename T> cudaError_t launch_eisenstat(const PcgArgs<T>& a, LaunchShape& shape, cudaStream_t s);
-// FP64 SSOR / multicolor SSOR PCG in one block with the gathered vectors in shared memory
-// (kernels_small.cu), for systems of at most pcg_smem_max_rows() rows.
-cudaError_t launch_pcg_smem(const PcgArgs<double>& a, int lanes, int threads, cudaStream_t s);
-int pcg_smem_max_rows();
-int pcg_smem_threads(int max_phase_rows, int lanes);
-bool pcg_smem_warp_sweeps(int n, int nf, int nbw);   // one warp walks the sweeps (256-thread block)
-size_t sweep_record_bytes(int n);                   // both sweeps' records of an n-row system
-cudaError_t launch_build_sweep_records(const PcgArgs<double>& a, void* recs, cudaStream_t s);
 // Largest co-resident grid for the given kernel family and lane count.
 int max_coresident_blocks(int family, int is_float, int lanes, int threads);
 int pick_lanes(double avg_nnz_per_row);

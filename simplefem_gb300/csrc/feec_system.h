@@ -89,6 +89,8 @@ struct FlowHostSlice {
 bool flow_cut_rows(int lo, int hi, const int* len, int row_ops, int sms, int longest, int max_slices,
                    std::vector<FlowHostSlice>& out);
 
+struct SmallData;   // one-block solver's slices and sweep schedules (kernels_small.cu)
+
 }  // namespace feec
 
 struct feec_system {
@@ -119,7 +121,7 @@ struct feec_system {
     double *x = nullptr, *r = nullptr, *d = nullptr, *z = nullptr, *m = nullptr, *q = nullptr, *b = nullptr;
     double* w = nullptr;               // Eisenstat solvers only: auxiliary + technical
     float* w32 = nullptr;              // ... FP32 copy for the mixed-precision inner solves
-    char* sweep_rec = nullptr;         // one-block solver: per-row sweep records (both sweeps)
+    feec::SmallData* small = nullptr;  // one-block solver, built on its first solve
     // MIXED on the whole GPU, per method slot (0: plain CG, 1: preconditioned): 0 = not yet
     // measured, 1 = FP32 inner iterations, 2 = FP64; device ms per decade of residual fall
     int mixed_pick[2] = {0, 0};
@@ -153,6 +155,14 @@ int flow_build(feec_system* s, bool f32);
 int launch_flow_eisenstat(feec_system* s, const PcgArgs<double>& a, LaunchShape& shape);
 int launch_flow_eisenstat(feec_system* s, const PcgArgs<float>& a, LaunchShape& shape);
 int launch_flow_pcg(feec_system* s, const PcgArgs<double>& a, LaunchShape& shape);
+// Fills slices (columns where ci is not null, values of either precision) from a split layout.
+cudaError_t flow_fill(int nslices, const int4* meta, const int* rp, const int* lsplit, const int* usplit, const int* ci_in,
+                      const double* val_in, int* ci, double* val64, float* val32, cudaStream_t st);
+// One-block FP64 SSOR / multicolor SSOR PCG for small systems (kernels_small.cu), reference rule.
+bool small_pcg_fits(const feec_system* s);
+int small_pcg_prepare(feec_system* s);
+int launch_small_pcg(feec_system* s, const PcgArgs<double>& a, LaunchShape& shape);
+void small_release(feec_system* s);
 // Plain CG (kernels_flow_cg.cu).
 int flow_cg_build(feec_system* s, bool f32);
 int launch_flow_cg(feec_system* s, const CgArgs<double>& a, LaunchShape& shape);

@@ -475,6 +475,14 @@ double slice_rows(int lo, int hi, const int* rp, const int* ls, const int* us, i
 
 }  // namespace
 
+cudaError_t flow_fill(int nslices, const int4* meta, const int* rp, const int* lsplit, const int* usplit, const int* ci_in,
+                      const double* val_in, int* ci, double* val64, float* val32, cudaStream_t st) {
+    if (nslices <= 0) return cudaSuccess;
+    note_launch();
+    flow_fill_kernel<<<(nslices + 7) / 8, 256, 0, st>>>(nslices, meta, rp, lsplit, usplit, ci_in, val_in, ci, val64, val32);
+    return cudaGetLastError();
+}
+
 bool flow_cut_rows(int lo, int hi, const int* len, int row_ops, int sms, int longest, int max_slices,
                    std::vector<FlowHostSlice>& out) {
     auto lanes = [](int entries, int most) {
@@ -563,11 +571,8 @@ int flow_build(feec_system* s, bool f32) {
     }
     if (f32) FEEC_TRY(D.mem.alloc(D.val32, (size_t)D.units * 32));
     else FEEC_TRY(D.mem.alloc(D.val64, (size_t)D.units * 32));
-    note_launch();
-    flow_fill_kernel<<<(D.nslices + 7) / 8, 256, 0, st>>>(D.nslices, D.meta, s->rp, s->lsplit, s->usplit, s->ci, s->val,
-                                                         first ? D.ci : nullptr, f32 ? nullptr : D.val64,
-                                                         f32 ? D.val32 : nullptr);
-    FEEC_TRY(cudaGetLastError());
+    FEEC_TRY(flow_fill(D.nslices, D.meta, s->rp, s->lsplit, s->usplit, s->ci, s->val, first ? D.ci : nullptr,
+                       f32 ? nullptr : D.val64, f32 ? D.val32 : nullptr, st));
     D.ready = true;
     return FEEC_OK;
 }

@@ -1,558 +1,624 @@
-// SSOR / multicolor SSOR preconditioned CG for small systems in one thread block, with
-// the vectors the sweeps gather (d, m, z) held in shared memory.
+// SSOR / multicolor SSOR preconditioned CG for small systems in one thread block, with the
+// gathered vectors in shared memory.
 //
-// ConjugateGradientSolverCSR_SSOR (solver/sparsesolver.cpp:446-724) sweeps its rows in
-// index order; over a dependency-level schedule that is 2 x (number of levels) dependent
-// phases per iteration (129 levels on the 2D P1 operator refined 6 times). A phase then
-// holds a few dozen rows, so its cost is its latency: the grid-wide or global-memory
-// version pays an L2 round trip for the gathered values plus a barrier per phase. Here
-// the gathered vectors live in shared memory, the barrier is the block barrier, and the
-// row data of each phase (matrix entries, r, q, x, the sweep factors) is loaded several
-// phases ahead: a phase costs a few shared-memory accesses and one __syncthreads. The
-// arithmetic and its order per row are those of pcg_persistent (same preconditioner,
-// same stopping rule, same skipped rows); only the dot products are summed by one block
-// instead of a grid, and the backward sweep's z.r is summed after the sweep. When the
-// phases average at most 64 rows (index-order levels), one warp walks each sweep with a
-// __syncwarp between phases and the rest of the block joins in between the sweeps.
+// ConjugateGradientSolverCSR_SSOR (solver/sparsesolver.cpp:446-724) sweeps its rows in index
+// order: over a dependency-level schedule that is 2 x (number of levels) dependent phases per
+// iteration (129 levels on the 2D P1 operator refined 6 times) of a few dozen rows each, so a
+// phase costs its latency. What that latency is made of on GB300: a warp's FP64 instruction
+// holds its scheduler 64 cycles whatever its active lanes, a shared-memory access takes 30, a
+// barrier of a few warps 20. So a phase's rows get a lane each (or several for long rows)
+// on as many warps as they fill; a row's factor omega / D is multiplied into its entries and,
+// before the sweep, into its right-hand side; and the phase's entries are staged in shared memory
+// by a warp that does nothing else. Behind a phase's barrier stand one gather and the row's
+// products. Colors (multicolor schedules) hold hundreds of rows and are bound by the one SM's
+// FP64 units instead (19 cycles per warp instruction).
+//
+// The block leaves the other SMs free: small solves on several streams run side by side, which
+// a grid-wide (cooperative) solve does not allow. Index-order systems come here up to about
+// 12,000 rows (their two vectors and the staging ring fill the shared memory; 16 blocks took 750 us
+// per iteration on 4,225 rows); multicolor ones up to kSmallColorRows, beyond which
+// the dataflow solver takes them (alone on the GPU it is the faster one here too: 18 us).
+//
+// Measured per iteration, 2D P1 refined 6 times (4,225 rows): index order 228 us (one warp walking
+// the levels over records, up to three rows a lane) -> 93; multicolor 70 -> 47. 3D P1, 4,913 rows,
+// 49 levels: 221 -> 114; 3D P2, 4,913 rows, 113 levels: 1793 -> 284.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstring>
+#include <vector>
 
-#include "feec_device.cuh"
-#include "feec_internal.h"
+#include "flow_device.cuh"
+#include "feec_system.h"
 #include "persistent_common.cuh"
 
 namespace feec {
 namespace {
 
-constexpr int kSmallPF = 4;   // entries of a row segment prefetched per lane
-constexpr int kRing = 4;      // rows (product) or phases (sweeps) loaded ahead per group
+constexpr int kSmallColorRows = 4608;   // multicolor systems
+// 512: 93 / 47 us per iteration (index order / colors, 4,225 rows); 768: 96 / 48; 1024: 100 / 50
+constexpr int kSmallThreads = 512;
+constexpr int kSmallWarps = kSmallThreads / 32;
+constexpr int kSweepEntries = 4;    // entries of a row part per lane and chunk
+constexpr int kMaxSweepDepth = 8;   // phases staged ahead (at least 3)
 
-struct SmallRow {
-    int i, a, e;               // row (-1: none), segment [a, e) of the part the phase reads
-    int c[kSmallPF];
-    double v[kSmallPF];
-    double r, q, x, w, s;      // row-local values the phase needs
+// What a warp needs for its slice of a phase: per lane 4 columns, 4 values times the row's factor
+// omega / D, and the row (n, the slot past the vector, where the lane has none). Rows are
+// numbered in 16 bits: a system that fits here has fewer.
+struct __align__(16) SweepSlice {
+    double v[32][kSweepEntries];
+    unsigned short c[32][kSweepEntries];
+    unsigned short row[32];
+    // entries per lane in use here, and further chunks of 4 entries: info >> 4 & 0xff of them,
+    // from chunk info >> 12
+    int info, pad[3];
+};
+static_assert(sizeof(SweepSlice) % 16 == 0, "one bulk copy");
+
+// One sweep, phase by phase (dependency levels or colors), 1 << shift lanes per row. Phase p has
+// the `width` slices from width * p (some possibly without rows), staged as one copy; phases
+// wider than that go on in slices [extra[p], extra[p + 1]).
+struct SweepView {
+    int nph, shift, warps, width, depth;
+    int count;                       // most entries per lane; rows of one lane and one chunk: plain
+    bool plain;
+    const SweepSlice* slices; const int* extra;
+    const int* mc; const double* mv;     // further chunks: 32 x 4 columns / values each
 };
 
-enum { kSmFull = 0, kSmForward = 1, kSmBackward = 2 };
-
-// Loads everything a phase needs of row slot k (k >= hi: no row) that does not depend on
-// the phases before it: the matrix entries of its segment, its sweep factors and, for a
-// forward row, its own r, q and x (written only by the row itself, and q by the product
-// before the sweep). A backward row's r is not loaded: the backward sweep's first phase
-// is loaded while the forward sweep still writes r, so z.r is summed after the sweep.
-template <int KIND, int LANES>
-__device__ __forceinline__ SmallRow small_row(const PcgArgs<double>& a, int k, int hi) {
-    SmallRow R;
-    R.i = -1; R.a = 0; R.e = 0; R.r = 0.0; R.q = 0.0; R.x = 0.0; R.w = 0.0; R.s = 0.0;
-    if (k < hi) {
-        if (KIND == kSmBackward) {
-            R.i = __ldg(&a.brows[k]);
-            R.a = __ldg(&a.usplit[R.i]);
-            R.e = __ldg(&a.rp[R.i + 1]);
-        } else {
-            R.i = k;
-            R.a = __ldg(&a.rp[k]);
-            R.e = (KIND == kSmForward) ? __ldg(&a.lsplit[k]) : __ldg(&a.rp[k + 1]);
-        }
-        R.w = __ldg(&a.wd[R.i]);
-        if (KIND == kSmForward) { R.r = a.r[R.i]; R.q = a.q[R.i]; R.x = a.x[R.i]; }
-        if (KIND == kSmBackward) R.s = __ldg(&a.sd[R.i]);
-    }
-    const int lane = threadIdx.x & (LANES - 1);
-    #pragma unroll
-    for (int t = 0; t < kSmallPF; t++) {
-        const int j = R.a + lane + t * LANES;
-        const bool ok = j < R.e;
-        R.c[t] = ok ? __ldg(&a.ci[j]) : 0;
-        R.v[t] = ok ? __ldg(&a.val[j]) : 0.0;
-    }
-    return R;
-}
-
-// Segment dot with the gathered vector in shared memory: the same terms in the same order
-// per lane as seg_dot, then the same shuffle tree.
-template <int LANES>
-__device__ __forceinline__ double small_dot(const SmallRow& R, const PcgArgs<double>& a, const double* sx) {
-    const int lane = threadIdx.x & (LANES - 1);
-    double s = 0.0;
-    #pragma unroll
-    for (int t = 0; t < kSmallPF; t++)
-        if (R.a + lane + t * LANES < R.e) s = fma(R.v[t], sx[R.c[t]], s);
-    for (int j = R.a + lane + kSmallPF * LANES; j < R.e; j += LANES) s = fma(__ldg(&a.val[j]), sx[__ldg(&a.ci[j])], s);
-    #pragma unroll
-    for (int off = LANES / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off, LANES);
-    return s;
-}
-
-// Walks the row slots [lo, hi) of one phase (LANES lanes per row; the trip count is uniform
-// across each warp for the shuffles). `cur` holds the group's first row, loaded ahead;
-// each later row is loaded while the one before it is processed. A warp without a row in
-// the phase branches around the body: a level holds a few dozen rows, and GB300 issues a
-// warp's FP64 instruction for 16 cycles of the SM's FP64 pipe even with every lane masked
-// (the idle warps' masked FP64 work was a third of the kernel's time).
-template <int KIND, int LANES, int THREADS, typename F>
-__device__ __forceinline__ void small_phase(const PcgArgs<double>& a, int lo, int hi, SmallRow cur, F&& body) {
-    constexpr int groups = THREADS / LANES;
-    const int g = threadIdx.x / LANES;
-    for (int base = lo; base < hi; base += groups) {
-        const SmallRow nxt = small_row<KIND, LANES>(a, base + groups + g, hi);
-        if (__any_sync(0xffffffffu, cur.i >= 0)) body(cur);
-        cur = nxt;
-    }
-}
-
-// Rows [lo, hi) without dependences between them (the full-row product): each group keeps
-// kRing of its rows in flight.
-template <int KIND, int LANES, int THREADS, typename F>
-__device__ __forceinline__ void small_rows_ring(const PcgArgs<double>& a, int lo, int hi, F&& body) {
-    constexpr int groups = THREADS / LANES;
-    const int g = threadIdx.x / LANES;
-    SmallRow buf[kRing];
-    #pragma unroll
-    for (int k = 0; k < kRing; k++) buf[k] = small_row<KIND, LANES>(a, lo + k * groups + g, hi);
-    for (int base = lo; base < hi; base += kRing * groups) {
-        #pragma unroll
-        for (int k = 0; k < kRing; k++) {
-            if (base + k * groups < hi) {   // uniform across the warp
-                body(buf[k]);
-                buf[k] = small_row<KIND, LANES>(a, base + (k + kRing) * groups + g, hi);
-            }
-        }
-    }
-}
-
-// The first row slot of the group in phase p of a sweep (forward: rows fptr[p].., backward:
-// slots bptr[p]..); no row past the last phase.
-template <int KIND, int LANES>
-__device__ __forceinline__ SmallRow sweep_first(const PcgArgs<double>& a, int p) {
-    const int g = threadIdx.x / LANES;
-    if (KIND == kSmForward) {
-        if (p >= a.nf) return small_row<KIND, LANES>(a, 0, 0);
-        return small_row<KIND, LANES>(a, __ldg(&a.fptr[p]) + g, __ldg(&a.fptr[p + 1]));
-    }
-    if (p >= a.nbw) return small_row<KIND, LANES>(a, 0, 0);
-    return small_row<KIND, LANES>(a, __ldg(&a.bptr[p]) + g, __ldg(&a.bptr[p + 1]));
-}
-
-// A sweep of dependent phases, one block barrier after each: the group's first row in phase
-// p + kRing is loaded while phase p runs, so a phase waits for its shared-memory gathers and
-// the barrier only. `ring` arrives holding the first kRing phases.
-template <int KIND, int LANES, int THREADS, typename F>
-__device__ __forceinline__ void small_sweep(const PcgArgs<double>& a, SmallRow (&ring)[kRing], F&& body) {
-    const int nph = KIND == kSmForward ? a.nf : a.nbw;
-    for (int p0 = 0; p0 < nph; p0 += kRing) {
-        #pragma unroll
-        for (int k = 0; k < kRing; k++) {
-            const int p = p0 + k;
-            if (p < nph) {   // uniform
-                const int lo = KIND == kSmForward ? __ldg(&a.fptr[p]) : __ldg(&a.bptr[p]);
-                const int hi = KIND == kSmForward ? __ldg(&a.fptr[p + 1]) : __ldg(&a.bptr[p + 1]);
-                small_phase<KIND, LANES, THREADS>(a, lo, hi, ring[k], body);
-                ring[k] = sweep_first<KIND, LANES>(a, p + kRing);
-                __syncthreads();
-            }
-        }
-    }
-}
-
-// ---- sweeps by one warp, for phases of a few dozen rows ----
-// Index-order SSOR levels hold a few dozen rows (2D P1 refined 6 times: 129 levels of 33
-// rows on average), so a level costs the latency of one warp's instruction path. One warp
-// walks a sweep's phases with a __syncwarp between them instead of a block barrier; lane
-// l takes rows l, l + 32, l + 64 of a phase and sums each row's triangular part in CSR
-// order (one lane per row, the order of the reference's loop). Each row of a sweep has a
-// 64-byte record in sweep order (row, first three columns and values of its triangular
-// part, sweep factor), so a phase's records are one contiguous range: the warp copies the
-// ranges of the next phases into a shared-memory ring with 16-byte cp.async copies, which
-// the barriers do not wait for (row data loaded into registers ahead of the barriers did
-// not shorten the phases: the barriers' memory ordering holds the warp until it arrives).
-// The base of a row (r in
-// the forward sweep, the scaled m in the backward sweep) is in shared memory: the x, r
-// update writes r into z's storage, which holds nothing live until the backward sweep.
-struct SweepRecord {    // 64 bytes
-    int i, a, cnt;      // row, start and length of its triangular segment
-    int c[3];           // first three columns (0 past cnt)
-    double v[3];        // first three values (0 past cnt)
-    double w;           // sweep factor
-    double pad;
+struct SmallArgs {
+    int n, nslices;
+    const int4* meta; const int* ci; const double* val;     // full rows, one lane each
+    const double* wd; const double* b;
+    double scale;                                           // 2 - omega
+    double *x, *r, *d, *z, *q;
+    SweepView fwd, bwd;
+    double tol2;
+    int use_zr_rule, max_iter, print_modulo;
+    double print_tol;
+    DeviceStatus* st;
 };
-constexpr int kStageSlots = 3;                    // rows per lane per phase staged (phases of up to 96 rows)
-constexpr int kStages = 4;                        // ring depth: phases in flight
-constexpr int kStageRows = kStageSlots * 32;
-constexpr int kRingDoubles = kStages * kStageRows * (int)sizeof(SweepRecord) / 8;
 
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
+// Doubles of the two vectors and the spare slot (an even count: copies land on 16 bytes).
+__host__ __device__ constexpr int small_doubles(int n) { return 2 * n + 2; }
+
+// v != 0 without the FP64 comparison (its warp instruction takes the SM 19 cycles too)
+__device__ __forceinline__ bool nonzero(double v) { return (__double_as_longlong(v) << 1) != 0; }
+
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void bar_init(unsigned long long* bar) {
+    asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
-// Copies the records of phase p (at most kStageRows of them) into `st` (one commit group,
-// possibly empty).
-__device__ __forceinline__ void stage_phase(const SweepRecord* rec, const int* ptr, int nph, int p, SweepRecord* st,
-                                            int lane) {
-    if (p < nph) {
-        const int lo = ptr[p];
-        const int rows = min(ptr[p + 1] - lo, kStageRows);
-        const char* src = reinterpret_cast<const char*>(rec + lo);
-        char* dst = reinterpret_cast<char*>(st);
-        for (int q = lane; q < 4 * rows; q += 32) cp_async16(dst + 16 * q, src + 16 * q);
-    }
-    cp_async_commit();
+// `bytes` into shared memory (one lane): the barrier completes when they have landed.
+__device__ __forceinline__ void load_slices(void* dst, const void* src, unsigned bytes, unsigned long long* bar) {
+    asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_addr(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_addr(bar))
+                 : "memory");
 }
-
-__device__ __forceinline__ void sweep_record(const SweepRecord& R, const PcgArgs<double>& a, double* x,
-                                             const double* base) {
-    double s = 0.0;
-    #pragma unroll
-    for (int u = 0; u < 3; u++)
-        if (u < R.cnt) s = fma(R.v[u], x[R.c[u]], s);
-    for (int j = R.a + 3; j < R.a + R.cnt; j++) s = fma(__ldg(&a.val[j]), x[__ldg(&a.ci[j])], s);
-    if (R.w != 0.0) x[R.i] = (base[R.i] - s) * R.w;
-}
-
-// A whole sweep by the calling warp over the records `rec` (in sweep order, phases
-// [ptr[p], ptr[p + 1])): x[i] = (base[i] - sum_j A_ij x[j]) * w.
-__device__ __forceinline__ void warp_sweep(const PcgArgs<double>& a, const SweepRecord* rec, const int* ptr, int nph,
-                                           double* x, const double* base, SweepRecord* ring) {
-    const int lane = threadIdx.x & 31;
-    #pragma unroll
-    for (int q = 0; q < kStages - 1; q++) stage_phase(rec, ptr, nph, q, ring + q * kStageRows, lane);
-    for (int p = 0; p < nph; p++) {
-        stage_phase(rec, ptr, nph, p + kStages - 1, ring + ((p + kStages - 1) % kStages) * kStageRows, lane);
-        cp_async_wait<kStages - 1>();   // this lane's copies of phase p have landed ...
-        __syncwarp();                   // ... and every other lane's
-        const SweepRecord* st = ring + (p % kStages) * kStageRows;
-        const int lo = ptr[p], hi = ptr[p + 1];
-        #pragma unroll
-        for (int t = 0; t < kStageSlots; t++) {
-            const int k = lane + 32 * t;
-            if (lo + k < hi) sweep_record(st[k], a, x, base);
+// Waits for a copy; gives up after kWaitNanos (status FEEC_TIMEOUT).
+__device__ __forceinline__ bool wait_slices(unsigned long long* bar, unsigned parity, DeviceStatus* st) {
+    unsigned long long t0 = 0;
+    for (unsigned n = 1;; n++) {
+        unsigned ok;
+        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                     : "=r"(ok)
+                     : "r"(smem_addr(bar)), "r"(parity)
+                     : "memory");
+        if (ok) return true;
+        if ((n & 15u) == 0) {      // a try itself waits for a while
+            const unsigned long long t = globaltimer_ns();
+            if (t0 == 0) t0 = t;
+            if (t - t0 > kWaitNanos) break;
         }
-        for (int k = lo + lane + kStageRows; k < hi; k += 32) sweep_record(rec[k], a, x, base);   // past the ring
-        __syncwarp();   // this phase's results before the next phase gathers them
     }
-    cp_async_wait<0>();
-    __syncwarp();
+    atomicExch(&st->abort, 1);
+    atomicCAS(&st->status, FEEC_OK, FEEC_TIMEOUT);
+    return false;
 }
 
-// One record per row of each sweep: forward slot k is row k (the phases are row ranges),
-// backward slot k is row brows[k].
-__global__ void build_sweep_records(PcgArgs<double> a, SweepRecord* fwd, SweepRecord* bwd) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= a.n) return;
+struct SweepEntries {
+    int row, info;
+    ushort4 c;
+    double v[kSweepEntries];
+};
+__device__ __forceinline__ void read_slice(SweepEntries& e, const SweepSlice& s, int lane) {
+    const double2 a = *reinterpret_cast<const double2*>(&s.v[lane][0]), b = *reinterpret_cast<const double2*>(&s.v[lane][2]);
+    e.v[0] = a.x; e.v[1] = a.y; e.v[2] = b.x; e.v[3] = b.y;
+    e.c = *reinterpret_cast<const ushort4*>(&s.c[lane][0]);
+    e.row = s.row[lane];
+    e.info = s.info;
+}
+
+// x[row] -= sum v x[c] for the slice in `e` (padding entries: column 0, value 0); `between` runs
+// while the gathers travel. The row's factor is in v and, before the sweep, in x, so behind the
+// gathers stand the products alone. COUNT entries per lane; PLAIN: no more, one lane per row.
+template <int COUNT, bool PLAIN, typename F>
+__device__ __forceinline__ void sweep_slice(const SweepEntries& e, const SweepView& s, double* x, int lane, F&& between) {
+    const bool own = PLAIN || (lane & ((1 << s.shift) - 1)) == 0;
+    const unsigned short c[4] = {e.c.x, e.c.y, e.c.z, e.c.w};
+    double g[COUNT];
     #pragma unroll
-    for (int dir = 0; dir < 2; dir++) {
-        const int i = dir == 0 ? k : __ldg(&a.brows[k]);
-        const int lo = dir == 0 ? __ldg(&a.rp[i]) : __ldg(&a.usplit[i]);
-        const int hi = dir == 0 ? __ldg(&a.lsplit[i]) : __ldg(&a.rp[i + 1]);
-        SweepRecord R;
-        R.i = i; R.a = lo; R.cnt = hi - lo;
-        #pragma unroll
-        for (int u = 0; u < 3; u++) {
-            const bool ok = lo + u < hi;
-            R.c[u] = ok ? __ldg(&a.ci[lo + u]) : 0;
-            R.v[u] = ok ? __ldg(&a.val[lo + u]) : 0.0;
+    for (int k = 0; k < COUNT; k++) g[k] = x[c[k]];
+    double acc = own ? x[e.row] : 0.0;
+    between();
+    #pragma unroll
+    for (int k = 0; k < COUNT; k++) acc = fma(-e.v[k], g[k], acc);
+    if constexpr (!PLAIN) {
+        for (int t = 0; t < (e.info >> 4 & 0xff); t++) {
+            #pragma unroll
+            for (int k = 0; k < kSweepEntries; k++) {
+                const int o = (kSweepEntries * ((e.info >> 12) + t) + k) * 32 + lane;
+                acc = fma(-__ldg(&s.mv[o]), x[__ldg(&s.mc[o])], acc);
+            }
         }
-        R.w = __ldg(&a.wd[i]);
-        R.pad = 0.0;
-        (dir == 0 ? fwd : bwd)[k] = R;
+        acc = row_sum<double>(acc, s.shift);
     }
+    if (own) x[e.row] = acc;
 }
 
-__device__ __forceinline__ double small_block_sum(double v) {
-    double vv[1] = {v};
-    block_reduce<double, 1>(vv);
-    __shared__ double s_sum;
-    if (threadIdx.x == 0) s_sum = vv[0];
-    __syncthreads();
-    const double out = s_sum;
-    __syncthreads();
-    return out;
+__device__ __forceinline__ void sweep_barrier(int warps) {
+    asm volatile("bar.sync 1, %0;" ::"r"(warps * 32) : "memory");
 }
 
-template <int LANES, int THREADS, bool WARP>
-__global__ void __launch_bounds__(THREADS) pcg_smem_kernel(PcgArgs<double> a) {
+// A whole sweep by the first s.warps warps of the block and the last warp, which stages the slices,
+// s.depth phases ahead: it issues a phase's copy when the slot's last readers have passed a
+// barrier, and comes to the barrier that ends phase p only when phase p + 2 has landed, so the
+// others never look at a copy's barrier and read the next phase's slice while this phase's gathers
+// travel. (Staging by the sweeping warps themselves put 500 cycles of issue and waiting into
+// each phase; entries requested into registers phases ahead did not shorten the phases: a warp
+// has six scoreboards for its loads and waits for the youngest load on one.) `phase` holds
+// the parity of each slot's barrier. False when a copy never landed.
+template <int COUNT, bool PLAIN>
+__device__ __forceinline__ bool sweep_as(const SweepView& s, double* x, SweepSlice* ring, unsigned long long* bars,
+                                      unsigned& phase, DeviceStatus* st) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool stager = warp == kSmallWarps - 1;      // of every sweep: it keeps the slots' parities
+    if ((warp >= s.warps && !stager) || s.nph == 0) return true;
+    if (stager) {
+        bool ok = true;
+        const unsigned bytes = (unsigned)(s.width * sizeof(SweepSlice));
+        auto issue = [&](int p, int slot) {
+            if (lane == 0 && p < s.nph) load_slices(ring + slot * s.width, s.slices + (long long)p * s.width, bytes, bars + slot);
+        };
+        auto landed = [&](int p, int slot) {
+            if (p >= s.nph) return;
+            ok = ok && wait_slices(bars + slot, phase >> slot & 1u, st);
+            phase ^= 1u << slot;
+        };
+        for (int k = 0; k < s.depth; k++) issue(k, k);
+        landed(0, 0);
+        landed(1, 1);
+        sweep_barrier(s.warps + 1);
+        int slot = 0, two = 2;      // slots of phases p and p + 2
+        for (int p = 0; p < s.nph; p++) {
+            landed(p + 2, two);
+            sweep_barrier(s.warps + 1);
+            issue(p + s.depth, slot);
+            slot = slot + 1 == s.depth ? 0 : slot + 1;
+            two = two + 1 == s.depth ? 0 : two + 1;
+        }
+        return ok;
+    }
+    sweep_barrier(s.warps + 1);
+    SweepEntries even, odd;
+    const SweepSlice* here = ring + warp;
+    read_slice(even, *here, lane);
+    int slot = 0;
+    auto step = [&](int p, const SweepEntries& e, SweepEntries& next) {
+        slot = slot + 1 == s.depth ? 0 : slot + 1;
+        const SweepSlice* ahead = ring + slot * s.width + warp;
+        sweep_slice<COUNT, PLAIN>(e, s, x, lane, [&] { if (p + 1 < s.nph) read_slice(next, *ahead, lane); });
+        if (s.width > s.warps)
+            for (int k = s.warps; warp + k < s.width; k += s.warps) {
+                SweepEntries f;
+                read_slice(f, here[k], lane);
+                sweep_slice<COUNT, PLAIN>(f, s, x, lane, [] {});
+            }
+        if (s.extra)
+            for (int sl = __ldg(&s.extra[p]) + warp; sl < __ldg(&s.extra[p + 1]); sl += s.warps) {
+                SweepEntries f;
+                read_slice(f, s.slices[sl], lane);
+                sweep_slice<COUNT, PLAIN>(f, s, x, lane, [] {});
+            }
+        sweep_barrier(s.warps + 1);      // phase p is complete
+        here = ahead;
+    };
+    for (int p = 0; p < s.nph; p += 2) {
+        step(p, even, odd);
+        if (p + 1 < s.nph) step(p + 1, odd, even);
+    }
+    return true;
+}
+
+__device__ __forceinline__ bool sweep(const SweepView& s, double* x, SweepSlice* ring, unsigned long long* bars,
+                                      unsigned& phase, DeviceStatus* st) {
+    if (!s.plain) return sweep_as<kSweepEntries, false>(s, x, ring, bars, phase, st);
+    if (s.count <= 2) return sweep_as<2, true>(s, x, ring, bars, phase, st);
+    if (s.count == 3) return sweep_as<3, true>(s, x, ring, bars, phase, st);
+    return sweep_as<4, true>(s, x, ring, bars, phase, st);
+}
+
+// Block sum, returned to warp 0. All values meet in shared memory first: summing 512 threads
+// takes 12 + 20 + 3 warp additions instead of the 85 of a tree per warp (19 cycles each).
+__device__ __forceinline__ double small_sum(double v, double* s_val) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    s_val[threadIdx.x] = v;
+    __syncthreads();
+    if (warp < 4) {
+        double a = s_val[threadIdx.x];
+        #pragma unroll
+        for (int k = 1; k < kSmallThreads / 128; k++) a += s_val[threadIdx.x + 128 * k];
+        #pragma unroll
+        for (int off = 16; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
+        if (lane == 0) s_val[kSmallThreads + warp] = a;
+    }
+    __syncthreads();
+    if (warp != 0) return 0.0;
+    return (s_val[kSmallThreads] + s_val[kSmallThreads + 1]) + (s_val[kSmallThreads + 2] + s_val[kSmallThreads + 3]);
+}
+
+// acc - sum over entries [k0, k0 + len) of the lane of val * X[col] with X in shared memory; the
+// next chunk is requested with the products of the current one.
+__device__ __forceinline__ double small_minus(const SmallArgs& a, long long off, int len, int lane, const double* X, double acc) {
+    constexpr int CH = 4;
+    const int* cp = a.ci + off + lane;
+    const double* vp = a.val + off + lane;
+    int c[CH];
+    double v[CH];
+    #pragma unroll
+    for (int u = 0; u < CH; u++) {
+        c[u] = u < len ? __ldg(cp + 32 * u) : -1;
+        v[u] = u < len ? __ldg(vp + 32 * u) : 0.0;
+    }
+    for (int k = 0; k < len; k += CH) {
+        int cn[CH];
+        double vn[CH];
+        #pragma unroll
+        for (int u = 0; u < CH; u++) {
+            const bool ok = k + CH + u < len;
+            cn[u] = ok ? __ldg(cp + 32 * (k + CH + u)) : -1;
+            vn[u] = ok ? __ldg(vp + 32 * (k + CH + u)) : 0.0;
+        }
+        #pragma unroll
+        for (int u = 0; u < CH; u++)
+            if (k + u < len) acc = fma(-v[u], c[u] >= 0 ? X[c[u]] : 0.0, acc);
+        #pragma unroll
+        for (int u = 0; u < CH; u++) { c[u] = cn[u]; v[u] = vn[u]; }
+    }
+    return acc;
+}
+
+__global__ void __launch_bounds__(kSmallThreads, 1) small_pcg(SmallArgs a) {
     extern __shared__ __align__(16) double smem[];
     const int n = a.n;
-    double* vec = WARP ? smem + kRingDoubles : smem;   // one-warp sweeps: the staging ring first
-    double* sdv = vec;           // d
-    double* smv = vec + n;       // m
-    double* szv = vec + 2 * n;   // z
-    const int lane = threadIdx.x & (LANES - 1);
-    const int g = threadIdx.x / LANES;
-    constexpr int groups = THREADS / LANES;
-    __shared__ double s_scal[2];
+    double* sd_ = smem;              // d
+    // the sweeps' vector, in place: (omega / D) r, then m as the forward sweep passes (a row's own
+    // value is read by the row alone, before its m is written), (2 - omega) m, then z as the
+    // backward sweep passes; 0 throughout in rows with D == 0 (factor 0), which the sweeps skip.
+    // Its slot n belongs to the lanes without a row.
+    double* su = smem + n;
+    SweepSlice* ring = reinterpret_cast<SweepSlice*>(smem + small_doubles(n));
+    __shared__ double s_val[kSmallThreads + 4];
+    __shared__ unsigned long long s_bar[kMaxSweepDepth];
+    __shared__ double s_scal;
     __shared__ int s_ctl;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned phase = 0;
+    bool ok = true;
 
-    for (int i = threadIdx.x; i < 3 * n; i += THREADS) vec[i] = 0.0;   // work vectors start at 0
-    SweepRecord* stage_ring = reinterpret_cast<SweepRecord*>(smem);
-    const SweepRecord* frec = reinterpret_cast<const SweepRecord*>(a.sweep_fwd);
-    const SweepRecord* brec = reinterpret_cast<const SweepRecord*>(a.sweep_bwd);
-    const int* sfptr = nullptr;
-    const int* sbptr = nullptr;
-    if constexpr (WARP) {
-        // the phase bounds of both sweeps follow the vectors
-        int* sfp = reinterpret_cast<int*>(vec + 3 * n);
-        int* sbp = sfp + a.nf + 1;
-        for (int i = threadIdx.x; i <= a.nf; i += THREADS) sfp[i] = __ldg(&a.fptr[i]);
-        for (int i = threadIdx.x; i <= a.nbw; i += THREADS) sbp[i] = __ldg(&a.bptr[i]);
-        sfptr = sfp;
-        sbptr = sbp;
-    }
+    for (int i = threadIdx.x; i < small_doubles(n); i += kSmallThreads) smem[i] = 0.0;   // work vectors start at 0
+    if (threadIdx.x < kMaxSweepDepth) bar_init(&s_bar[threadIdx.x]);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
 
-    // ---- restart (sparsesolver.cpp:506-588): r = b - A x for rows with D != 0 ----
-    double arr = 0.0;
-    for (int base = 0; base < n; base += groups) {
-        const int i = base + g;
-        const bool act = i < n;
-        const int lo = act ? __ldg(&a.rp[i]) : 0, hi = act ? __ldg(&a.rp[i + 1]) : 0;
-        double s = 0.0;
-        for (int j = lo + lane; j < hi; j += LANES) s = fma(__ldg(&a.val[j]), a.x[__ldg(&a.ci[j])], s);
-        #pragma unroll
-        for (int off = LANES / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off, LANES);
-        if (act && lane == 0 && __ldg(&a.wd[i]) != 0.0) {
-            const double ri = __ldg(&a.b[i]) - s;
-            a.r[i] = ri;
-            if constexpr (WARP) szv[i] = ri;   // the forward sweep's base
-            arr += ri * ri;
+    // every row, one lane each: body(slice, row, has a row)
+    auto rows = [&](auto&& body) {
+        int4 next = warp < a.nslices ? __ldg(&a.meta[warp]) : make_int4(0, 0, 0, 0);
+        for (int s = warp; s < a.nslices; s += kSmallWarps) {
+            const FlowSlice f = flow_slice(next);
+            if (s + kSmallWarps < a.nslices) next = __ldg(&a.meta[s + kSmallWarps]);
+            body(f, f.row0 + lane, lane < f.nrow);
         }
-    }
-    __syncthreads();   // orders the r writes before the sweeps read them
-    double azr = 0.0;
-    if constexpr (WARP) {
-        if (threadIdx.x < 32) warp_sweep(a, frec, sfptr, a.nf, smv, szv, stage_ring);
+    };
+    // m = (D/w + L)^-1 r, z = (D/w + U)^-1 S m (:528-575, :647-699 / :1118-1170, :1241-1307), in su;
+    // returns z.r (warp 0)
+    auto precondition = [&]() {
+        ok = sweep(a.fwd, su, ring, s_bar, phase, a.st) && ok;
         __syncthreads();
-        for (int i = threadIdx.x; i < n; i += THREADS)
-            if (__ldg(&a.wd[i]) != 0.0) smv[i] *= __ldg(&a.sd[i]);
-        __syncthreads();
-        if (threadIdx.x < 32) warp_sweep(a, brec, sbptr, a.nbw, szv, smv, stage_ring);
-        __syncthreads();
-        for (int i = threadIdx.x; i < n; i += THREADS)
-            if (__ldg(&a.wd[i]) != 0.0) {
-                const double zi = szv[i];
-                sdv[i] = zi;
-                azr += zi * a.r[i];
-            }
-    } else {
-        for (int p = 0; p < a.nf; p++) {                          // forward sweep
-            const int lo_r = __ldg(&a.fptr[p]), hi_r = __ldg(&a.fptr[p + 1]);
-            for (int base = lo_r; base < hi_r; base += groups) {
-                const int i = base + g;
-                const bool act = i < hi_r;
-                const SmallRow R = small_row<kSmForward, LANES>(a, i, hi_r);
-                const double s = small_dot<LANES>(R, a, smv);
-                if (act && lane == 0) {
-                    const double w = __ldg(&a.wd[i]);
-                    if (w != 0.0) smv[i] = (a.r[i] - s) * w;
-                }
-            }
+        if (a.scale != 1.0) {
+            for (int i = threadIdx.x; i < n; i += kSmallThreads) su[i] *= a.scale;
             __syncthreads();
         }
-        for (int p = 0; p < a.nbw; p++) {                         // scale + backward sweep
-            const int lo_r = __ldg(&a.bptr[p]), hi_r = __ldg(&a.bptr[p + 1]);
-            for (int base = lo_r; base < hi_r; base += groups) {
-                const int k = base + g;
-                const bool act = k < hi_r;
-                const SmallRow R = small_row<kSmBackward, LANES>(a, k, hi_r);
-                const double s = small_dot<LANES>(R, a, szv);
-                if (act && lane == 0) {
-                    const double w = __ldg(&a.wd[R.i]);
-                    if (w != 0.0) {
-                        const double mi = smv[R.i] * __ldg(&a.sd[R.i]);
-                        smv[R.i] = mi;
-                        const double zi = (mi - s) * w;
-                        szv[R.i] = zi;
-                        sdv[R.i] = zi;
-                        azr += zi * a.r[R.i];
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    }
-    double z_r = small_block_sum(azr);
-    double r_r = small_block_sum(arr);
+        ok = sweep(a.bwd, su, ring, s_bar, phase, a.st) && ok;
+        __syncthreads();
+        double zr = 0.0;
+        for (int i = threadIdx.x; i < n; i += kSmallThreads)
+            if (nonzero(__ldg(&a.wd[i]))) zr = fma(su[i], a.r[i], zr);
+        return small_sum(zr, s_val);
+    };
 
-    int K = 0;
-    int status = FEEC_MAXITER;
-    double d_Ad = 0.0;
-    SmallRow ring[kRing];
+    // ---- restart (sparsesolver.cpp:506-588 / :1072-1175): r = b - A x for rows with D != 0 ----
+    rows([&](const FlowSlice& f, int i, bool act) {
+        double acc = act ? __ldg(&a.b[i]) : 0.0;
+        acc = small_minus(a, f.off, part_len<kFlowAll>(f), lane, a.x, acc);
+        const double w = act ? __ldg(&a.wd[i]) : 0.0;
+        if (nonzero(w)) { a.r[i] = acc; su[i] = acc * w; }
+    });
+    __syncthreads();
+    double z_r = precondition();
+    for (int i = threadIdx.x; i < n; i += kSmallThreads) sd_[i] = su[i];
+    __syncthreads();
+
+    // scalar control by thread 0 (z_r is its copy); the others read s_scal and s_ctl
+    int K = 0, status = FEEC_MAXITER;
     while (K < a.max_iter) {
         if (threadIdx.x == 0) {
             if (a.print_modulo > 0 && K % a.print_modulo == 0)
                 printf("(%d/%d)   INTERIM: Residual norm is %.9le < %.9le\n", K, n, sqrt(z_r), a.print_tol);
-            int ctl = 0;
-            if (a.use_zr_rule && fabs(z_r) < a.tol2) ctl = 1;                         // :601-604
-            if (a.rr_stop > 0.0 && r_r < a.rr_stop) ctl = 1;
-            s_ctl = ctl;
+            s_ctl = a.use_zr_rule && abs_below(z_r, a.tol2) ? 1 : 0;                          // :601-604 / :1187-1190
         }
-        __syncthreads();
-        if (s_ctl) { status = FEEC_OK; break; }
-
-        double adq = 0.0;                                                            // :614-628
-        small_rows_ring<kSmFull, LANES, THREADS>(a, 0, n, [&](const SmallRow& R) {
-            const double s = small_dot<LANES>(R, a, sdv);
-            if (R.i >= 0 && lane == 0) {
-                const double qi = (R.w != 0.0) ? s : 0.0;
-                a.q[R.i] = qi;
-                adq += sdv[R.i] * qi;
+        double dq = 0.0;                                                                      // :614-628 / :1197-1212
+        rows([&](const FlowSlice& f, int i, bool act) {
+            const double q = -small_minus(a, f.off, part_len<kFlowAll>(f), lane, sd_, 0.0);
+            if (act) {
+                const double qi = nonzero(__ldg(&a.wd[i])) ? q : 0.0;
+                a.q[i] = qi;
+                dq = fma(sd_[i], qi, dq);
             }
         });
-        d_Ad = small_block_sum(adq);    // its barriers also order q before the forward sweep reads it
-        if constexpr (!WARP) {
-            #pragma unroll
-            for (int k = 0; k < kRing; k++) ring[k] = sweep_first<kSmForward, LANES>(a, k);
+        const double d_Ad = small_sum(dq, s_val);    // its barriers also order q before it is read
+        if (threadIdx.x == 0 && s_ctl == 0) {
+            if (!isfinite(z_r) || below_zero(z_r) || !isfinite(d_Ad) || below_zero(d_Ad)) s_ctl = 2;
+            else if (energy_small(d_Ad)) s_ctl = 3;
+            s_scal = z_r / d_Ad;
         }
-        if (threadIdx.x == 0) {
-            int ctl = 0;
-            if (!isfinite(z_r) || z_r < 0.0 || !isfinite(d_Ad) || d_Ad < 0.0) ctl = 1;
-            else if (sqrt(fabs(d_Ad)) < kMachineEpsilon) ctl = 2;
-            s_ctl = ctl;
-            s_scal[0] = z_r / d_Ad;
+        if (__syncthreads_or(!ok)) return;       // a staged copy never landed (FEEC_TIMEOUT)
+        if (s_ctl) { status = s_ctl == 1 ? FEEC_OK : s_ctl == 2 ? FEEC_BREAKDOWN : FEEC_SMALL_ENERGY; break; }
+        const double alpha = s_scal;
+        // :640-667 / :1230-1240, the update of x and r (rows with D != 0)
+        for (int i0 = threadIdx.x; i0 < n; i0 += 4 * kSmallThreads) {
+            double w[4], x[4], r[4], q[4];
+            #pragma unroll
+            for (int k = 0; k < 4; k++) {       // four rows' values requested together
+                const int i = i0 + k * kSmallThreads;
+                const bool in = i < n;
+                w[k] = in ? __ldg(&a.wd[i]) : 0.0;
+                x[k] = in ? a.x[i] : 0.0;
+                r[k] = in ? a.r[i] : 0.0;
+                q[k] = in ? a.q[i] : 0.0;
+            }
+            #pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int i = i0 + k * kSmallThreads;
+                if (nonzero(w[k])) {
+                    a.x[i] = fma(alpha, sd_[i], x[k]);
+                    const double rn = fma(-alpha, q[k], r[k]);
+                    a.r[i] = rn;
+                    su[i] = rn * w[k];
+                }
+            }
         }
         __syncthreads();
-        if (s_ctl == 1) { status = FEEC_BREAKDOWN; break; }
-        if (s_ctl == 2) { status = FEEC_SMALL_ENERGY; break; }
-
-        const double alpha = s_scal[0];
-        arr = 0.0;
-        if constexpr (WARP) {
-            // :640-667, the update of x and r first (rows with D != 0), then the sweep
-            for (int i = threadIdx.x; i < n; i += THREADS)
-                if (__ldg(&a.wd[i]) != 0.0) {
-                    a.x[i] = a.x[i] + alpha * sdv[i];
-                    const double ri = a.r[i] - alpha * a.q[i];
-                    a.r[i] = ri;
-                    szv[i] = ri;   // the forward sweep's base (z's storage is free until the backward sweep)
-                    arr += ri * ri;
-                }
-            __syncthreads();
-            if (threadIdx.x < 32) warp_sweep(a, frec, sfptr, a.nf, smv, szv, stage_ring);
-            __syncthreads();
-            for (int i = threadIdx.x; i < n; i += THREADS)                            // :670-699
-                if (__ldg(&a.wd[i]) != 0.0) smv[i] *= __ldg(&a.sd[i]);
-            __syncthreads();
-            if (threadIdx.x < 32) warp_sweep(a, brec, sbptr, a.nbw, szv, smv, stage_ring);
-            __syncthreads();
-        } else {
-            small_sweep<kSmForward, LANES, THREADS>(a, ring, [&](const SmallRow& R) {             // :640-667
-                const double s = small_dot<LANES>(R, a, smv);
-                if (R.i >= 0 && lane == 0 && R.w != 0.0) {
-                    a.x[R.i] = R.x + alpha * sdv[R.i];
-                    const double ri = R.r - alpha * R.q;
-                    a.r[R.i] = ri;
-                    arr += ri * ri;
-                    smv[R.i] = (ri - s) * R.w;
-                }
-            });
-            #pragma unroll
-            for (int k = 0; k < kRing; k++) ring[k] = sweep_first<kSmBackward, LANES>(a, k);
-            small_sweep<kSmBackward, LANES, THREADS>(a, ring, [&](const SmallRow& R) {            // :670-699
-                const double s = small_dot<LANES>(R, a, szv);
-                if (R.i >= 0 && lane == 0 && R.w != 0.0) {
-                    const double mi = smv[R.i] * R.s;
-                    smv[R.i] = mi;
-                    const double zi = (mi - s) * R.w;
-                    szv[R.i] = zi;
-                }
-            });
+        const double z_r_new = precondition();
+        if (threadIdx.x == 0) {                                                               // :701-706 / :1309-1318
+            s_scal = z_r_new / z_r;
+            z_r = z_r_new;
         }
-        double azr2 = 0.0;
-        for (int i = threadIdx.x; i < n; i += THREADS)                           // z.r, :690-697
-            if (__ldg(&a.wd[i]) != 0.0) azr2 += szv[i] * a.r[i];
-        // the block sums' barriers order x, r and z before the direction update and the next product
-        const double z_r_new = small_block_sum(azr2);
-        r_r = small_block_sum(arr);
-        const double beta = z_r_new / z_r;                                             // :701-706
-        z_r = z_r_new;
-        for (int i = threadIdx.x; i < n; i += THREADS)
-            if (__ldg(&a.wd[i]) != 0.0) sdv[i] = szv[i] + beta * sdv[i];
+        __syncthreads();
+        const double beta = s_scal;
+        for (int i = threadIdx.x; i < n; i += kSmallThreads)
+            sd_[i] = fma(beta, sd_[i], su[i]);   // 0 where D == 0
         __syncthreads();
         K++;
     }
-    // the work vectors go back to global memory (callers may read d, z, m after a solve)
-    for (int i = threadIdx.x; i < n; i += THREADS) { a.d[i] = sdv[i]; a.m[i] = smv[i]; a.z[i] = szv[i]; }
-    finish(a.st, status, K, z_r, r_r);
+    for (int i = threadIdx.x; i < n; i += kSmallThreads) { a.d[i] = sd_[i]; a.z[i] = su[i]; }
+    finish(a.st, status, K, z_r, 0.0);
 }
 
-size_t smem_bytes(int n) { return (size_t)3 * (size_t)n * sizeof(double); }
+// Static shared memory of the kernel, left out of the vectors' share.
+constexpr int kSmallStatic = 8 * (kSmallThreads + 4) + 8 * kMaxSweepDepth + 256;
 
-// The one-warp sweeps also hold the staging ring and the phase bounds of both sweeps.
-size_t smem_bytes_warp(int n, int nf, int nbw) {
-    return smem_bytes(n) + (size_t)kRingDoubles * 8 + sizeof(int) * ((size_t)nf + 1 + (size_t)nbw + 1);
+int optin_bytes() {
+    int dev = 0, optin = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
+    return optin;
 }
 
-template <int LANES, int THREADS, bool WARP>
-cudaError_t launch_small(const PcgArgs<double>& a, cudaStream_t s) {
-    const size_t bytes = WARP ? smem_bytes_warp(a.n, a.nf, a.nbw) : smem_bytes(a.n);
-    cudaError_t e = cudaFuncSetAttribute(pcg_smem_kernel<LANES, THREADS, WARP>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e != cudaSuccess) return e;
-    note_launch();
-    pcg_smem_kernel<LANES, THREADS, WARP><<<1, THREADS, bytes, s>>>(a);
-    return cudaGetLastError();
+// One sweep's slices from the host copy of the layout.
+struct SweepHost {
+    std::vector<int> extra, mc;
+    std::vector<double> mv;
+    std::vector<SweepSlice> slices;
+    int shift = 0, warps = 1, width = 1, depth = 3, count = 0;
+    bool plain = true;
+};
+
+// `room`: slices of the shared memory's ring. False when a row is too long for the form.
+bool build_sweep(SweepHost& h, int nph, const int* pptr, const int* list, const int* from, const int* to,
+                 const int* ci, const double* val, const double* wd, int room, int n) {
+    long long entries = 0;
+    const int rows = pptr[nph];
+    for (int k = 0; k < rows; k++) { const int i = list ? list[k] : k; entries += to[i] - from[i]; }
+    // lanes per row: the average part in one chunk per lane, but one where a phase fills the
+    // block's warps anyway (colors: bound by the SM's FP64 units)
+    const bool wide = rows >= 32 * kSmallWarps / 2 * nph;
+    while (!wide && h.shift < 5 && entries > (long long)rows * (kSweepEntries << h.shift)) h.shift++;
+    const int width = 1 << h.shift, per = 32 >> h.shift;
+    int widest = 1;
+    for (int p = 0; p < nph; p++) widest = std::max(widest, (pptr[p + 1] - pptr[p] + per - 1) / per);
+    // the widest phase in a slot, or as much of it as three slots leave room for
+    h.width = std::max(1, std::min(widest, room / 3));
+    h.warps = std::min(h.width, kSmallWarps - 1);
+    h.depth = std::max(3, std::min(kMaxSweepDepth, room / h.width));
+    std::vector<SweepSlice> more;
+    bool any = false;
+    h.extra.assign(1, nph * h.width);
+    for (int p = 0; p < nph; p++) {
+        int at = 0;
+        for (int k0 = pptr[p]; at < h.width || k0 < pptr[p + 1]; k0 += per, at++) {
+            SweepSlice s;
+            std::memset(&s, 0, sizeof(s));
+            for (int l = 0; l < 32; l++) s.row[l] = (unsigned short)n;
+            const int k1 = std::min(pptr[p + 1], k0 + per);
+            int longest = 0;
+            for (int k = k0; k < k1; k++) { const int i = list ? list[k] : k; longest = std::max(longest, (to[i] - from[i] + width - 1) / width); }
+            const int chunks = std::max(0, (longest + kSweepEntries - 1) / kSweepEntries - 1);
+            const int first = (int)(h.mc.size() / (32 * kSweepEntries));
+            if (chunks > 0xff || first >= 1 << 19) return false;
+            s.info = std::min(longest, kSweepEntries) | chunks << 4 | first << 12;
+            h.count = std::max(h.count, std::min(longest, kSweepEntries));
+            if (chunks > 0) h.plain = false;
+            h.mc.resize(h.mc.size() + (size_t)32 * kSweepEntries * chunks, 0);
+            h.mv.resize(h.mc.size(), 0.0);
+            for (int k = k0; k < k1; k++) {
+                const int i = list ? list[k] : k, base = (k - k0) * width;
+                for (int t = 0; t < width; t++) s.row[base + t] = (unsigned short)i;
+                for (int j = 0; j < to[i] - from[i]; j++) {
+                    const int e = j / width, lane = base + j % width, chunk = e / kSweepEntries;
+                    if (chunk == 0) {
+                        s.c[lane][e] = (unsigned short)ci[from[i] + j];
+                        s.v[lane][e] = val[from[i] + j] * wd[i];
+                    } else {
+                        const size_t o = ((size_t)kSweepEntries * (first + chunk - 1) + e % kSweepEntries) * 32 + lane;
+                        h.mc[o] = ci[from[i] + j];
+                        h.mv[o] = val[from[i] + j] * wd[i];
+                    }
+                }
+            }
+            if (at < h.width) h.slices.push_back(s);
+            else { more.push_back(s); any = true; }
+        }
+        h.extra.push_back(nph * h.width + (int)more.size());
+    }
+    h.slices.insert(h.slices.end(), more.begin(), more.end());
+    if (!any) h.extra.clear();
+    if (h.shift > 0) h.plain = false;
+    return true;
 }
 
-template <int LANES>
-cudaError_t launch_small_threads(const PcgArgs<double>& a, int threads, bool warp_sweeps, cudaStream_t s) {
-    if (warp_sweeps) return launch_small<LANES, 256, true>(a, s);
-    if (threads <= 64) return launch_small<LANES, 64, false>(a, s);
-    if (threads <= 128) return launch_small<LANES, 128, false>(a, s);
-    return launch_small<LANES, 256, false>(a, s);
+int upload_sweep(DevArena& m, cudaStream_t st, const SweepHost& h, int nph, SweepView& v) {
+    int *extra = nullptr, *mc;
+    double* mv;
+    SweepSlice* slices;
+    FEEC_TRY(m.alloc(slices, h.slices.size())); FEEC_TRY(m.alloc(mc, h.mc.size())); FEEC_TRY(m.alloc(mv, h.mv.size()));
+    FEEC_TRY(cudaMemcpyAsync(slices, h.slices.data(), sizeof(SweepSlice) * h.slices.size(), cudaMemcpyHostToDevice, st));
+    FEEC_TRY(cudaMemcpyAsync(mc, h.mc.data(), 4 * h.mc.size(), cudaMemcpyHostToDevice, st));
+    FEEC_TRY(cudaMemcpyAsync(mv, h.mv.data(), 8 * h.mv.size(), cudaMemcpyHostToDevice, st));
+    if (!h.extra.empty()) {
+        FEEC_TRY(m.alloc(extra, h.extra.size()));
+        FEEC_TRY(cudaMemcpyAsync(extra, h.extra.data(), 4 * h.extra.size(), cudaMemcpyHostToDevice, st));
+    }
+    FEEC_TRY(cudaStreamSynchronize(st));   // the host arrays leave scope
+    v.nph = nph; v.shift = h.shift; v.warps = h.warps; v.width = h.width; v.depth = h.depth; v.count = h.count; v.plain = h.plain;
+    v.slices = slices; v.extra = extra; v.mc = mc; v.mv = mv;
+    return FEEC_OK;
+}
+
+// Slices of the ring beside the two vectors.
+int ring_room(int n) {
+    return (int)(((long long)optin_bytes() - kSmallStatic - 8ll * small_doubles(n)) / (long long)sizeof(SweepSlice));
 }
 
 }  // namespace
 
-int pcg_smem_max_rows() {
-    int dev = 0, optin = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
-    const int static_bytes = 2048;   // block reductions and scalars
-    return (optin - static_bytes) / (3 * (int)sizeof(double));
+// Slices and sweep schedules, kept with the layout.
+struct SmallData {
+    DevArena mem;
+    SmallArgs args{};
+};
+
+void small_release(feec_system* s) {
+    if (!s->small) return;
+    s->small->mem.release();
+    delete s->small;
+    s->small = nullptr;
 }
 
-// The block is as wide as the widest sweep phase needs (64, 128 or 256 threads): a phase's
-// cost is its instruction path and barrier, which grow with the warps that take part, and
-// the index-order levels hold a few dozen rows.
-int pcg_smem_threads(int max_phase_rows, int lanes) {
-    const long long need = (long long)max_phase_rows * lanes;
-    return need <= 64 ? 64 : need <= 128 ? 128 : 256;
+bool small_pcg_fits(const feec_system* s) {
+    if (s->n >= 0xffff || ring_room(s->n) < 8) return false;
+    return s->prepared == FEEC_METHOD_SSOR || (s->prepared == FEEC_METHOD_RAINBOW && s->n <= kSmallColorRows);
 }
 
-// Sweeps by one warp when the phases average at most 64 rows (index-order SSOR levels)
-// and the staging ring and row bounds fit beside the vectors; by the whole block otherwise
-// (multicolor phases of hundreds of rows).
-bool pcg_smem_warp_sweeps(int n, int nf, int nbw) {
-    if (nf <= 0 || n > 64 * nf) return false;
-    int dev = 0, optin = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return false;
-    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return false;
-    return smem_bytes_warp(n, nf, nbw) + 2048 <= (size_t)optin;   // 2048: block reductions and scalars
-}
+namespace {
 
-size_t sweep_record_bytes(int n) { return (size_t)2 * (size_t)n * sizeof(SweepRecord); }
-
-cudaError_t launch_build_sweep_records(const PcgArgs<double>& a, void* recs, cudaStream_t s) {
-    SweepRecord* fwd = reinterpret_cast<SweepRecord*>(recs);
-    note_launch();
-    build_sweep_records<<<(a.n + 255) / 256, 256, 0, s>>>(a, fwd, fwd + a.n);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_pcg_smem(const PcgArgs<double>& a, int lanes, int threads, cudaStream_t s) {
-    if (a.n <= 0 || a.n > pcg_smem_max_rows()) return cudaErrorInvalidValue;
-    const bool warp = pcg_smem_warp_sweeps(a.n, a.nf, a.nbw) && a.sweep_fwd && a.sweep_bwd;
-    switch (lanes) {
-        case 1: return launch_small_threads<1>(a, threads, warp, s);
-        case 2: return launch_small_threads<2>(a, threads, warp, s);
-        case 4: return launch_small_threads<4>(a, threads, warp, s);
-        default: return launch_small_threads<8>(a, threads, warp, s);
+int small_build(feec_system* s) {
+    if (s->small) return FEEC_OK;
+    HomeStreamScope home(s);
+    cudaStream_t st = s->stream;
+    const int n = s->n;
+    s->small = new SmallData();
+    s->small->mem.stream = st;
+    DevArena& M = s->small->mem;
+    SmallArgs& a = s->small->args;
+    std::vector<int> rp((size_t)n + 1), ls((size_t)n), us((size_t)n);
+    std::vector<int> fptr((size_t)s->nf + 1), bptr((size_t)s->nbw + 1), brows((size_t)n), ci((size_t)s->nnz);
+    std::vector<double> val((size_t)s->nnz), wd((size_t)n);
+    FEEC_TRY(cudaMemcpyAsync(rp.data(), s->rp, 4 * rp.size(), cudaMemcpyDeviceToHost, st));
+    FEEC_TRY(cudaMemcpyAsync(ls.data(), s->lsplit, 4 * ls.size(), cudaMemcpyDeviceToHost, st));
+    FEEC_TRY(cudaMemcpyAsync(us.data(), s->usplit, 4 * us.size(), cudaMemcpyDeviceToHost, st));
+    FEEC_TRY(cudaMemcpyAsync(fptr.data(), s->fptr, 4 * fptr.size(), cudaMemcpyDeviceToHost, st));
+    FEEC_TRY(cudaMemcpyAsync(bptr.data(), s->bptr, 4 * bptr.size(), cudaMemcpyDeviceToHost, st));
+    FEEC_TRY(cudaMemcpyAsync(brows.data(), s->brows, 4 * brows.size(), cudaMemcpyDeviceToHost, st));
+    FEEC_TRY(cudaMemcpyAsync(ci.data(), s->ci, 4 * ci.size(), cudaMemcpyDeviceToHost, st));
+    FEEC_TRY(cudaMemcpyAsync(val.data(), s->val, 8 * val.size(), cudaMemcpyDeviceToHost, st));
+    FEEC_TRY(cudaMemcpyAsync(wd.data(), s->wd, 8 * wd.size(), cudaMemcpyDeviceToHost, st));
+    FEEC_TRY(cudaStreamSynchronize(st));
+    // full rows, one lane each: one SM's FP64 units are the bound
+    std::vector<int4> meta;
+    long long units = 0;
+    for (int r0 = 0; r0 < n; r0 += 32) {
+        const int nr = std::min(32, n - r0);
+        int l = 0, e = 0, u = 0;
+        for (int i = r0; i < r0 + nr; i++) {
+            l = std::max(l, ls[i] - rp[i]);
+            e = std::max(e, us[i] - ls[i]);
+            u = std::max(u, rp[i + 1] - us[i]);
+        }
+        if (l > 0xffff || u > 0xffff || e > 0x7fff) return FEEC_BADARG;
+        meta.push_back(make_int4(r0, nr | e << 16, l | (int)((unsigned)u << 16), (int)units));
+        units += l + e + u;
     }
+    int4* dmeta; int* dci; double* dval;
+    FEEC_TRY(M.alloc(dmeta, meta.size())); FEEC_TRY(M.alloc(dci, (size_t)units * 32)); FEEC_TRY(M.alloc(dval, (size_t)units * 32));
+    FEEC_TRY(cudaMemcpyAsync(dmeta, meta.data(), sizeof(int4) * meta.size(), cudaMemcpyHostToDevice, st));
+    FEEC_TRY(flow_fill((int)meta.size(), dmeta, s->rp, s->lsplit, s->usplit, s->ci, s->val, dci, dval, nullptr, st));
+    a.n = n; a.nslices = (int)meta.size(); a.meta = dmeta; a.ci = dci; a.val = dval;
+    SweepHost f, b;
+    const int room = ring_room(n);
+    if (!build_sweep(f, s->nf, fptr.data(), nullptr, rp.data(), ls.data(), ci.data(), val.data(), wd.data(), room, n) ||
+        !build_sweep(b, s->nbw, bptr.data(), brows.data(), us.data(), rp.data() + 1, ci.data(), val.data(), wd.data(), room, n))
+        return FEEC_BADARG;
+    const int e = upload_sweep(M, st, f, s->nf, a.fwd);
+    return e != FEEC_OK ? e : upload_sweep(M, st, b, s->nbw, a.bwd);
+}
+
+}  // namespace
+
+int small_pcg_prepare(feec_system* s) {
+    const int e = small_build(s);
+    if (e != FEEC_OK) {
+        cudaGetLastError();
+        small_release(s);
+    }
+    return e;
+}
+
+int launch_small_pcg(feec_system* s, const PcgArgs<double>& p, LaunchShape& shape) {
+    SmallArgs a = s->small->args;
+    a.wd = p.wd; a.scale = 2.0 - p.omega; a.b = p.b; a.x = p.x; a.r = p.r; a.d = p.d; a.z = p.z; a.q = p.q;
+    a.tol2 = p.tol2; a.use_zr_rule = p.use_zr_rule; a.max_iter = p.max_iter; a.print_modulo = p.print_modulo;
+    a.print_tol = p.print_tol; a.st = p.st;
+    const int ring = std::max(a.fwd.width * a.fwd.depth, a.bwd.width * a.bwd.depth);
+    const size_t bytes = 8 * (size_t)small_doubles(s->n) + (size_t)ring * sizeof(SweepSlice);
+    shape.blocks = 1;
+    shape.threads = kSmallThreads;
+    shape.lanes = 1 << a.fwd.shift;
+    note_launch();
+    FEEC_TRY(cudaFuncSetAttribute(small_pcg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    small_pcg<<<1, kSmallThreads, bytes, s->stream>>>(a);
+    return cuda_status(cudaGetLastError());
 }
 
 }  // namespace feec

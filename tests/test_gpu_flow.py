@@ -134,3 +134,67 @@ def test_flow_solvers_repeat_bit_for_bit(method, mode):
         runs.append((info["iterations"], x.cpu().numpy().tobytes()))
     assert runs[0] == runs[1] == runs[2]
     sysm.close()
+
+
+SMALL_CASES = [("one_row", lambda: _diagonal(1)), ("diagonal", lambda: _diagonal(40)), ("tridiagonal_33", lambda: _tridiagonal(33)),
+               ("arrow_257", lambda: _arrow(257)), ("p1_2d", lambda: _lattice(2, 1, 5, 1001)),
+               ("p2_2d", lambda: _lattice(2, 2, 5, 0)), ("p1_3d_wide_levels", lambda: _lattice(3, 1, 5, 9000)),
+               ("p2_3d_long_rows", lambda: _lattice(3, 2, 4, 9000)), ("p3_3d", lambda: _lattice(3, 3, 2, 0)),
+               ("largest_colors", lambda: _lattice(2, 1, 7, 4608))]
+
+
+@pytest.mark.parametrize("method,omega", [("ssor", 1.0), ("ssor", 1.4), ("rainbow", 1.0), ("rainbow", 0.8)])
+@pytest.mark.parametrize("name,make", SMALL_CASES, ids=[c[0] for c in SMALL_CASES])
+def test_one_block_solver_matches_oracle(name, make, method, omega):
+    """One-block SSOR and multicolor PCG (kernels_small.cu): single rows, one and several lanes per
+    row, phases wider than the staging slots, rows of several chunks, and rows with D == 0."""
+    import torch
+    from oracle import oracle
+    from simplefem_gb300.system import System
+    M = make()
+    M.sort_indices()
+    A, C, V = M.indptr.astype(np.int32), M.indices.astype(np.int32), M.data.astype(np.float64)
+    n = len(A) - 1
+    rng = np.random.default_rng(n + 2)
+    b = 1e3 * rng.uniform(-1.0, 1.0, n)
+    diag = oracle.csr_diagonal(A, C, V)
+    sysm = System(A, C, V)
+    if method == "ssor":
+        sysm.set_ssor(diag, omega)
+        K_o, x_o, _ = oracle.cg_ssor(A, C, V, b, diag, omega, precision=1e-11)
+    else:
+        rb = oracle.rainbow(A, C)
+        sysm.set_rainbow(diag, omega, *rb)
+        K_o, x_o, _ = oracle.cg_rainbow(A, C, V, b, diag, rb, omega, precision=1e-11)
+    x = torch.zeros(n, dtype=torch.float64, device="cuda")
+    info = sysm.solve(torch.from_numpy(b).cuda(), x, method=method, mode="reference", precision=1e-11)
+    assert info["status"] == (3 if K_o == n else 0), (info, K_o)
+    assert abs(info["iterations"] - K_o) <= max(1, int(np.ceil(0.02 * K_o))), (info, K_o)
+    assert np.linalg.norm(x.cpu().numpy() - x_o) <= 1e-9 * np.linalg.norm(x_o), info
+    sysm.close()
+
+
+@pytest.mark.parametrize("method", ["ssor", "rainbow"])
+def test_one_block_solver_skips_zero_diagonal_rows(method):
+    import torch
+    from oracle import oracle
+    from simplefem_gb300.system import System
+    M = _lattice(2, 1, 4, 0)
+    A, C, V = M.indptr.astype(np.int32), M.indices.astype(np.int32), M.data
+    n = len(A) - 1
+    b = np.random.default_rng(4).uniform(-1e3, 1e3, n)
+    diag = oracle.csr_diagonal(A, C, V)
+    diag[[3, 77, n - 1]] = 0.0
+    sysm = System(A, C, V)
+    if method == "ssor":
+        sysm.set_ssor(diag, 1.0)
+        K_o, x_o, _ = oracle.cg_ssor(A, C, V, b, diag, 1.0, precision=1e-11)
+    else:
+        rb = oracle.rainbow(A, C)
+        sysm.set_rainbow(diag, 1.0, *rb)
+        K_o, x_o, _ = oracle.cg_rainbow(A, C, V, b, diag, rb, 1.0, precision=1e-11)
+    x = torch.zeros(n, dtype=torch.float64, device="cuda")
+    info = sysm.solve(torch.from_numpy(b).cuda(), x, method=method, mode="reference", precision=1e-11)
+    assert abs(info["iterations"] - K_o) <= max(1, int(np.ceil(0.02 * K_o))), (info, K_o)
+    assert np.linalg.norm(x.cpu().numpy() - x_o) <= 1e-9 * np.linalg.norm(x_o), info
+    sysm.close()
