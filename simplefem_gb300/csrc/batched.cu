@@ -117,18 +117,154 @@ struct Job {
     double* x[kBatchMaxK];
 };
 
+// Teams of a batch whose work items hold one right-hand side each: one block per system, or a
+// cluster of 2 to 16 blocks for a system that would alone take longer than the whole batch spread
+// evenly over the GPU. Items are ordered by group, the widest teams and largest systems first; the
+// groups run side by side, each with a queue of its own.
+struct TeamGroup {
+    int blocks, first, count;      // blocks per team; items [first, first + count) of the order
+};
+
+// A system's work is taken as its iterations (~ sqrt(n)) times the FP64 instructions of one
+// (entries, and kRowOps per row); total / SMs is what the batch takes if nothing is left idle. A
+// team doubles while its blocks hold more than 1 / kTeamShare of that each (two blocks share an
+// SM's FP64 units), and while each block keeps kTeamRows rows: below that a sweep is bound by its
+// barriers. Measured with FP64 Rainbow on mixes of 2D systems of 81 to 66,049 rows: 512 systems
+// (51 of the largest) 803 ms with one block each, 283 / 181 / 181 / 237 ms at kTeamShare 0.5 / 1 /
+// 1.5 / 2 (at 2 the clusters alone outnumber the SMs); 128 systems 617 ms, then 118 / 104 / 66 /
+// 66; 48 systems 405 ms, then 42 / 46 / 45 / 45. Eight systems at kTeamRows 2048 / 4096 / 8192:
+// 13.2 / 15.5 / 21.8 ms.
+std::vector<TeamGroup> plan_teams(const std::vector<feec_system*>& sys, int is_float, int rainbow, std::vector<int>& order) {
+    constexpr double kRowOps = 14.0, kTeamShare = 1.5;
+    constexpr int kTeamRows = 2048;
+    const size_t nsys = sys.size();
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // a mixed-precision batch may also run in FP64, with the same teams
+    int widest = 1;
+    while (widest < 16 && cluster_batched_resident(0, 1, rainbow, 2 * widest) > 0 &&
+           (!is_float || cluster_batched_resident(1, 1, rainbow, 2 * widest) > 0))
+        widest *= 2;
+    std::vector<double> work(nsys);
+    double total = 0.0;
+    for (size_t i = 0; i < nsys; i++) total += work[i] = std::sqrt((double)sys[i]->n) * (sys[i]->nnz + kRowOps * sys[i]->n);
+    std::vector<int> team(nsys, 1);
+    for (size_t i = 0; i < nsys; i++)
+        while (team[i] < widest && work[i] * kTeamShare * sms > total * team[i] && sys[i]->n / kTeamRows >= team[i])
+            team[i] *= 2;
+    order.resize(nsys);
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+        return team[a] != team[b] ? team[a] > team[b] : sys[a]->n > sys[b]->n;
+    });
+    std::vector<TeamGroup> groups;
+    for (size_t k = 0; k < nsys; k++) {
+        if (groups.empty() || groups.back().blocks != team[order[k]]) groups.push_back({team[order[k]], (int)k, 0});
+        groups.back().count++;
+    }
+    return groups;
+}
+
+// Resident teams of each group, and the blocks of all of them. (The queries also set the kernels'
+// attributes, so a capture of the launches holds nothing but stream work.)
+int resident_groups(const std::vector<TeamGroup>& groups, int is_float, int rainbow, int threads, std::vector<int>& teams) {
+    int blocks = 0;
+    teams.clear();
+    for (const TeamGroup& g : groups) {
+        const int fit = g.blocks == 1 ? batched_resident_teams(is_float, 1, rainbow, threads)
+                                      : cluster_batched_resident(is_float, 1, rainbow, g.blocks);
+        teams.push_back(std::min(g.count, fit));
+        blocks += teams.back() * g.blocks;
+    }
+    return blocks;
+}
+
+// Streams and events that let the groups of a batch run side by side: the first on the caller's
+// stream, the others forked from it and joined again.
+struct TeamFork {
+    std::vector<cudaStream_t> streams;
+    std::vector<cudaEvent_t> events;
+    TeamFork() = default;
+    TeamFork(const TeamFork&) = delete;
+    TeamFork& operator=(const TeamFork&) = delete;
+    ~TeamFork() {
+        for (cudaStream_t q : streams) cudaStreamDestroy(q);
+        for (cudaEvent_t q : events) cudaEventDestroy(q);
+    }
+    int make(size_t groups) {
+        for (size_t g = 0; g < groups && groups > 1; g++) {
+            cudaEvent_t ev = nullptr;
+            FEEC_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+            events.push_back(ev);
+            if (g == 0) continue;
+            cudaStream_t q = nullptr;
+            FEEC_TRY(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
+            streams.push_back(q);
+        }
+        return FEEC_OK;
+    }
+};
+
+// args.next_item: one zeroed counter per group. On an error the forks made so far are joined all
+// the same, so `st` still orders whatever was launched.
+cudaError_t launch_groups(const BatchArgs& args, const std::vector<TeamGroup>& groups, const std::vector<int>& teams,
+                          int is_float, int rainbow, int threads, const TeamFork& fork, cudaStream_t st) {
+    cudaError_t e = groups.size() > 1 ? cudaEventRecord(fork.events[0], st) : cudaSuccess;
+    for (size_t g = 0; g < groups.size() && e == cudaSuccess; g++) {
+        cudaStream_t q = g == 0 ? st : fork.streams[g - 1];
+        if (g > 0) e = cudaStreamWaitEvent(q, fork.events[0], 0);
+        BatchArgs part = args;
+        part.items = args.items + groups[g].first;
+        part.nitems = groups[g].count;
+        part.next_item = args.next_item + g;
+        if (e == cudaSuccess)
+            e = groups[g].blocks == 1 ? launch_batched(part, is_float, 1, rainbow, threads, teams[g], q)
+                                      : launch_batched_clusters(part, is_float, 1, rainbow, groups[g].blocks, teams[g], q);
+        if (g > 0) {
+            cudaError_t j = cudaEventRecord(fork.events[g], q);
+            if (j == cudaSuccess) j = cudaStreamWaitEvent(st, fork.events[g], 0);
+            if (e == cudaSuccess) e = j;
+        }
+    }
+    return e;
+}
+
 // One launch of the batched kernel over `jobs`; the per-column results come back in `res`.
 // team_blocks >= 2: clusters of that many blocks are the teams (threads is then the cluster
-// kernel's fixed block size); teams = 0 fills the GPU with resident teams.
+// kernel's fixed block size); team_blocks = 0 (K = 1): teams by system size (plan_teams);
+// teams = 0 fills the GPU with resident teams. `grid` gets the launch's blocks.
 int run_batch_results(cudaStream_t st, const std::vector<feec_system*>& systems, std::vector<Job>& jobs, int method,
                       int mode, int K, double precision, int max_iter, int nresults, int teams, int threads,
                       int team_blocks, int max_outer, bool stall_check, std::vector<BatchResult>& res,
-                      float* elapsed_ms) {
+                      float* elapsed_ms, int* grid) {
     const int is_float = mode == FEEC_MODE_MIXED ? 1 : 0;
+    const int rb = method == FEEC_METHOD_RAINBOW;
     const size_t tsz = is_float ? sizeof(float) : sizeof(double);
     // largest systems first, so the tail of the batch is short
     std::stable_sort(jobs.begin(), jobs.end(),
                      [&](const Job& a, const Job& b) { return systems[a.system]->n > systems[b.system]->n; });
+    std::vector<TeamGroup> groups;
+    std::vector<int> group_teams;
+    TeamFork fork;
+    if (team_blocks == 0) {
+        std::vector<feec_system*> of;
+        for (const Job& jb : jobs) of.push_back(systems[jb.system]);
+        std::vector<int> order;
+        groups = plan_teams(of, is_float, rb, order);
+        std::vector<Job> sorted;
+        for (int k : order) sorted.push_back(jobs[k]);
+        jobs.swap(sorted);
+        *grid = resident_groups(groups, is_float, rb, threads, group_teams);
+        const int e = fork.make(groups.size());
+        if (e != FEEC_OK) return e;
+    } else if (team_blocks >= 2) {
+        const int nc = teams > 0 ? teams : cluster_batched_resident(is_float, K, rb, team_blocks);
+        *grid = std::min<int>(nc, (int)jobs.size()) * team_blocks;
+    } else {
+        *grid = teams > 0 ? teams : std::min<int>(batched_resident_teams(is_float, K, rb, threads), (int)jobs.size());
+    }
+    const size_t queues = std::max<size_t>(groups.size(), 1);
     DevArena tmp;
     tmp.stream = st;
     std::vector<SellView> views;
@@ -140,7 +276,7 @@ int run_batch_results(cudaStream_t st, const std::vector<feec_system*>& systems,
     FEEC_TRY(tmp.alloc(dviews, views.size()));
     FEEC_TRY(tmp.alloc(ditems, jobs.size()));
     FEEC_TRY(tmp.alloc(dres, (size_t)nresults));
-    FEEC_TRY(tmp.alloc(dnext, 1));
+    FEEC_TRY(tmp.alloc(dnext, queues));
     std::vector<BatchItem> items(jobs.size());
     for (size_t i = 0; i < jobs.size(); i++) {
         const Job& jb = jobs[i];
@@ -156,7 +292,7 @@ int run_batch_results(cudaStream_t st, const std::vector<feec_system*>& systems,
     }
     FEEC_TRY(cudaMemcpyAsync(dviews, views.data(), sizeof(SellView) * views.size(), cudaMemcpyHostToDevice, st));
     FEEC_TRY(cudaMemcpyAsync(ditems, items.data(), sizeof(BatchItem) * items.size(), cudaMemcpyHostToDevice, st));
-    FEEC_TRY(cudaMemsetAsync(dnext, 0, sizeof(int), st));
+    FEEC_TRY(cudaMemsetAsync(dnext, 0, sizeof(int) * queues, st));
     FEEC_TRY(cudaMemsetAsync(dres, 0, sizeof(BatchResult) * nresults, st));
     BatchArgs a{};
     a.systems = dviews; a.items = ditems; a.nitems = (int)items.size(); a.next_item = dnext; a.results = dres;
@@ -174,10 +310,12 @@ int run_batch_results(cudaStream_t st, const std::vector<feec_system*>& systems,
     FEEC_TRY(cudaEventCreate(&e0));
     FEEC_TRY(cudaEventCreate(&e1));
     FEEC_TRY(cudaEventRecord(e0, st));
-    if (team_blocks >= 2)
-        FEEC_TRY(launch_batched_clusters(a, is_float, K, method == FEEC_METHOD_RAINBOW, team_blocks, teams, st));
+    if (team_blocks == 0)
+        FEEC_TRY(launch_groups(a, groups, group_teams, is_float, rb, threads, fork, st));
+    else if (team_blocks >= 2)
+        FEEC_TRY(launch_batched_clusters(a, is_float, K, rb, team_blocks, teams, st));
     else
-        FEEC_TRY(launch_batched(a, is_float, K, method == FEEC_METHOD_RAINBOW, threads, teams, st));
+        FEEC_TRY(launch_batched(a, is_float, K, rb, threads, teams, st));
     FEEC_TRY(cudaEventRecord(e1, st));
     res.assign((size_t)nresults, BatchResult{});
     FEEC_TRY(cudaMemcpyAsync(res.data(), dres, sizeof(BatchResult) * nresults, cudaMemcpyDeviceToHost, st));
@@ -213,8 +351,9 @@ int rescue_stagnated(cudaStream_t st, const std::vector<feec_system*>& systems, 
     if (again.empty()) return FEEC_OK;
     std::vector<BatchResult> r2;
     float ms = 0.0f;
+    int grid = 0;
     const int st2 = run_batch_results(st, systems, again, method, FEEC_MODE_FP64, 1, precision, max_iter,
-                                      (int)again.size(), 0, 256, 1, 0, false, r2, &ms);
+                                      (int)again.size(), 0, 256, 0, 0, false, r2, &ms, &grid);
     if (st2 != FEEC_OK) return st2;
     for (size_t k = 0; k < slot.size(); k++) {
         BatchResult& d = res[slot[k]];
@@ -259,9 +398,10 @@ int run_batch(cudaStream_t st, const std::vector<feec_system*>& systems, std::ve
     const int is_float = mode == FEEC_MODE_MIXED ? 1 : 0;
     std::vector<BatchResult> res;
     float ms = 0.0f;
+    int grid = 0;
     const bool rescue = is_float && max_outer == 0;   // the autotuner's trials run a fixed iteration count
     int st2 = run_batch_results(st, systems, jobs, method, mode, K, precision, max_iter, nresults, teams, threads,
-                                team_blocks, max_outer, rescue, res, &ms);
+                                team_blocks, max_outer, rescue, res, &ms, &grid);
     if (st2 != FEEC_OK) return st2;
     if (rescue) {
         st2 = rescue_stagnated(st, systems, jobs, method, precision, max_iter, res, &ms);
@@ -272,14 +412,6 @@ int run_batch(cudaStream_t st, const std::vector<feec_system*>& systems, std::ve
         long long t = 0;
         for (int i = 0; i < nresults; i++) t += res[i].iterations;
         *iter_sum = t;
-    }
-    const int rb = method == FEEC_METHOD_RAINBOW;
-    int grid = 0;
-    if (team_blocks >= 2) {
-        const int nc = teams > 0 ? teams : cluster_batched_resident(is_float, K, rb, team_blocks);
-        grid = std::min<int>(nc, (int)jobs.size()) * team_blocks;
-    } else {
-        grid = teams > 0 ? teams : std::min<int>(batched_resident_teams(is_float, K, rb, threads), (int)jobs.size());
     }
     int worst = FEEC_OK;
     fill_infos(res, precision, ms, grid, infos, worst);
@@ -507,7 +639,7 @@ int feec_solve_many(int nsys, feec_system* const* systems, int method, int mode,
         std::memset(&jb, 0, sizeof(jb));
         jb.system = i; jb.nrhs = 1; jb.first = i; jb.b[0] = b[i]; jb.x[0] = x[i];
     }
-    return run_batch(st, sys, jobs, method, mode, 1, precision, max_iter > 0 ? max_iter : maxn, nsys, infos, 0, 256);
+    return run_batch(st, sys, jobs, method, mode, 1, precision, max_iter > 0 ? max_iter : maxn, nsys, infos, 0, 256, 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -580,10 +712,15 @@ int feec_batch_create(feec_batch** out, int nsys, feec_system* const* systems, i
     // FP64-sized workspace in both modes: a mixed batch also captures and times the FP64
     // iteration (below)
     const size_t tsz = sizeof(double);
-    // largest systems first
-    std::vector<int> order((size_t)nsys);
-    std::iota(order.begin(), order.end(), 0);
-    std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return sys[a]->n > sys[c]->n; });
+    const bool rainbow = method == FEEC_METHOD_RAINBOW;
+    const int threads = team_threads > 0 ? team_threads : 256;
+    // teams by system size; a caller's team size keeps one-block teams, largest systems first
+    std::vector<int> order;
+    std::vector<TeamGroup> groups = plan_teams(sys, is_float, rainbow, order);
+    if (team_threads > 0) {
+        std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return sys[a]->n > sys[c]->n; });
+        groups.assign(1, TeamGroup{1, 0, nsys});
+    }
     std::vector<SellView> views;
     for (auto* sp : sys) views.push_back(sell_view(sp, method));
     SellView* dviews = nullptr;
@@ -593,7 +730,7 @@ int feec_batch_create(feec_batch** out, int nsys, feec_system* const* systems, i
     FEEC_TRY(M.alloc(dviews, views.size()));
     FEEC_TRY(M.alloc(ditems, (size_t)nsys));
     FEEC_TRY(M.alloc(bt->dres, (size_t)nsys));
-    FEEC_TRY(M.alloc(dnext, 1));
+    FEEC_TRY(M.alloc(dnext, groups.size()));
     std::vector<BatchItem> items((size_t)nsys);
     for (int k = 0; k < nsys; k++) {
         const int i = order[k];
@@ -626,24 +763,24 @@ int feec_batch_create(feec_batch** out, int nsys, feec_system* const* systems, i
         jb.system = i; jb.nrhs = 1; jb.first = i; jb.b[0] = b[i]; jb.x[0] = x[i];
         bt->jobs.push_back(jb);
     }
-    const int threads = team_threads > 0 ? team_threads : 256;
-    const bool rainbow = method == FEEC_METHOD_RAINBOW;
-    bt->teams = std::min(nsys, batched_resident_teams(is_float, 1, rainbow, threads));
-    const int teams64 = std::min(nsys, batched_resident_teams(0, 1, rainbow, threads));
-    // capture a launch sequence (batched_resident_teams above already set the kernels'
-    // attributes, so nothing but stream work happens while capturing)
-    auto capture = [&](const BatchArgs& args, int f, int teams, cudaGraph_t& g, cudaGraphExec_t& ex) -> int {
+    std::vector<int> teams, teams64;
+    bt->teams = resident_groups(groups, is_float, rainbow, threads, teams);
+    const int blocks64 = resident_groups(groups, 0, rainbow, threads, teams64);
+    TeamFork fork;
+    int st = fork.make(groups.size());
+    if (st != FEEC_OK) return st;
+    auto capture = [&](const BatchArgs& args, int f, const std::vector<int>& count, cudaGraph_t& g, cudaGraphExec_t& ex) -> int {
         FEEC_TRY(cudaStreamBeginCapture(bt->stream, cudaStreamCaptureModeRelaxed));
-        cudaMemsetAsync(dnext, 0, sizeof(int), bt->stream);
+        cudaMemsetAsync(dnext, 0, sizeof(int) * groups.size(), bt->stream);
         cudaMemsetAsync(bt->dres, 0, sizeof(BatchResult) * nsys, bt->stream);
-        const cudaError_t le = launch_batched(args, f, 1, rainbow, threads, teams, bt->stream);
+        const cudaError_t le = launch_groups(args, groups, count, f, rainbow, threads, fork, bt->stream);
         const cudaError_t ce = cudaStreamEndCapture(bt->stream, &g);
         if (le != cudaSuccess) return cuda_status(le);
         if (ce != cudaSuccess) return cuda_status(ce);
         FEEC_TRY(cudaGraphInstantiate(&ex, g, 0));
         return FEEC_OK;
     };
-    int st = capture(a, is_float, bt->teams, bt->graph, bt->exec);
+    st = capture(a, is_float, teams, bt->graph, bt->exec);
     if (st != FEEC_OK) return st;
     FEEC_TRY(cudaEventCreate(&bt->e0));
     FEEC_TRY(cudaEventCreate(&bt->e1));
@@ -708,7 +845,7 @@ int feec_batch_create(feec_batch** out, int nsys, feec_system* const* systems, i
         if (t64 < t32) {
             std::swap(bt->graph, g64);
             std::swap(bt->exec, ex64);   // the guard destroys the FP32 graph
-            bt->teams = teams64;
+            bt->teams = blocks64;
             bt->inner_fp64 = 1;
         }
     }
