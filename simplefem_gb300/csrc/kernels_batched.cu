@@ -24,10 +24,9 @@ namespace {
 
 using namespace team_solver;
 
-// At least 1024 resident threads per SM (64 registers per thread): the solver is bound by
-// memory latency, so warps in flight matter more than registers.
-template <typename T, int K, bool RAINBOW, int THREADS>
-__global__ void __launch_bounds__(THREADS, (1024 / THREADS) > 0 ? (1024 / THREADS) : 1) batched_solve_kernel(BatchArgs args) {
+// The solver over the queue of work items, for one block.
+template <typename T, int K, bool RAINBOW, typename Team>
+__device__ __forceinline__ void solve_queue(const BatchArgs& args) {
     __shared__ int s_item;
     while (true) {
         if (threadIdx.x == 0) s_item = atomicAdd(args.next_item, 1);
@@ -35,9 +34,24 @@ __global__ void __launch_bounds__(THREADS, (1024 / THREADS) > 0 ? (1024 / THREAD
         const int item = s_item;
         __syncthreads();
         if (item >= args.nitems) return;
-        BlockTeam team;
+        Team team;
         team_solve<T, K, RAINBOW>(team, args, args.items[item]);
     }
+}
+
+// At least 1024 resident threads per SM (64 registers per thread): the solver is bound by
+// memory latency, so warps in flight matter more than registers.
+template <typename T, int K, bool RAINBOW, int THREADS>
+__global__ void __launch_bounds__(THREADS, (1024 / THREADS) > 0 ? (1024 / THREADS) : 1) batched_solve_kernel(BatchArgs args) {
+    solve_queue<T, K, RAINBOW, BlockTeam>(args);
+}
+
+// 512 resident threads per SM (128 registers per thread): launches that would leave half of the
+// other kernel's threads empty.
+constexpr int kWideResident = 512;
+template <typename T, int K, bool RAINBOW, int THREADS>
+__global__ void __launch_bounds__(THREADS, kWideResident / THREADS) batched_wide_kernel(BatchArgs args) {
+    solve_queue<T, K, RAINBOW, WideBlockTeam>(args);
 }
 
 template <typename T, int K, bool RB>
@@ -73,6 +87,20 @@ const void* pick(int is_float, int K, int rainbow, int threads) {
         case 2: return rainbow ? kfn<double, 2, true>(threads) : kfn<double, 2, false>(threads);
         default: return nullptr;
     }
+}
+
+// The wide kernel where the launch has one and its teams all fit at half of the SMs' threads
+// (nullptr otherwise). Both sides at 3D P2, 35,937 rows, teams of 512 threads on 152 SMs: 152
+// teams 77 ms here against 107, 304 teams 151 ms with two blocks per SM (two waves here).
+const void* pick_wide(int is_float, int K, int rainbow, int threads, int teams) {
+    if (!is_float || K != 4 || (threads != 256 && threads != 512)) return nullptr;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (teams > sms * (kWideResident / threads)) return nullptr;
+    if (threads == 256)
+        return rainbow ? (const void*)batched_wide_kernel<float, 4, true, 256> : (const void*)batched_wide_kernel<float, 4, false, 256>;
+    return rainbow ? (const void*)batched_wide_kernel<float, 4, true, 512> : (const void*)batched_wide_kernel<float, 4, false, 512>;
 }
 
 }  // namespace
@@ -113,6 +141,7 @@ cudaError_t launch_batched(const BatchArgs& args, int is_float, int K, int rainb
     if (teams <= 0) teams = batched_resident_teams(is_float, K, rainbow, threads);
     if (teams > args.nitems) teams = args.nitems;
     if (teams <= 0) return cudaSuccess;
+    if (const void* wide = pick_wide(is_float, K, rainbow, threads, teams)) fn = wide;
     BatchArgs copy = args;
     void* kargs[] = {&copy};
     note_launch();

@@ -93,10 +93,9 @@ __device__ __forceinline__ void load_entries(const int* __restrict__ sci, const 
 // Software-pipelined over chunks of CH entries: the column indices and values of the
 // next chunk are requested together with the gathers of the current one, so a chunk
 // costs one memory round trip instead of two.
-template <typename T, typename TV, int K>
+template <typename T, typename TV, int K, int CH>
 __device__ __forceinline__ void block_dot(const int* __restrict__ sci, const TV* __restrict__ sval, long long off,
                                           int len, int lane, const T* X, T (&s)[K]) {
-    constexpr int CH = Chunk<T, K>::value;
     const unsigned long long pol = l2_keep_policy();
     if (len <= 0) return;
     int c[CH]; T v[CH];
@@ -160,6 +159,8 @@ template <> __device__ __forceinline__ const double* sel_sd<double>(const SellVi
 // Neither waits on anything outside its own co-scheduled threads.
 // ---------------------------------------------------------------------------
 struct BlockTeam {
+    template <typename T, int K>
+    static constexpr int chunk() { return Chunk<T, K>::value; }
     __device__ __forceinline__ int rank() const { return 0; }
     __device__ __forceinline__ int size() const { return 1; }
     __device__ __forceinline__ int tid() const { return threadIdx.x; }
@@ -169,7 +170,23 @@ struct BlockTeam {
     __device__ __forceinline__ void sum(typename AccT<T>::type (&v)[NV], double (&out)[NV]) { team_sum<T, NV>(v, out); }
 };
 
+// A block with twice the registers per thread, for launches whose teams leave at least half of the
+// SMs' threads empty: six entries per chunk instead of two keep three times the gathers in flight
+// (same order of products, same bits). FP32, 4 right-hand sides per team of 512 threads:
+// 3D P2, 35,937 rows: 608 columns 107 -> 77 ms (chunks of 4 / 6 / 8: 80 / 76.5 / 76.8), 200 columns
+// 75 -> 66 ms; 2D P1, 4,225 rows, whose blocks hold 2 to 4 entries: 300 columns 9.45 -> 9.15 ms
+// (9.8 without the short chunk). What remains is the L1: a gather of 32 rows touches 11 lines.
+// Entries requested one slice ahead were slower (82 to 92 ms), as were 1024 threads of 64
+// registers (81).
+constexpr int kWideChunk = 6, kShortBlock = 4;
+struct WideBlockTeam : BlockTeam {
+    template <typename T, int K>
+    static constexpr int chunk() { return sizeof(T) == 4 ? kWideChunk : Chunk<T, K>::value; }
+};
+
 struct ClusterTeam {
+    template <typename T, int K>
+    static constexpr int chunk() { return Chunk<T, K>::value; }
     int r, sz, buf;
     __device__ ClusterTeam() : buf(0) {
         cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
@@ -333,7 +350,11 @@ __device__ __forceinline__ void for_slices_dot(const Team& team, const SellView&
         U sum[K];
         #pragma unroll
         for (int j = 0; j < K; j++) sum[j] = U(0);
-        block_dot<U, TV, K>(S.ci, val, off, len, lane, X, sum);
+        constexpr int CH = Team::template chunk<U, K>();
+        if (CH > kShortBlock && len <= kShortBlock)   // no empty slots of a long chunk for a short block
+            block_dot<U, TV, K, kShortBlock>(S.ci, val, off, len, lane, X, sum);
+        else
+            block_dot<U, TV, K, CH>(S.ci, val, off, len, lane, X, sum);
         post(M, state, sum);
     });
 }

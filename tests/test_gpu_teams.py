@@ -1,4 +1,4 @@
-"""Batches whose systems differ so much that the large ones are solved by clusters of blocks: every
+"""The kernels a batch of systems or of right-hand sides is sent to by its size. Batches whose systems differ so much that the large ones are solved by clusters of blocks: every
 system reaches 1e-10 with the exact solution to 1e-9 (the bounds of the batched engine's other
 tests), and agrees with one-block teams, for every cluster size and in both entry points."""
 import numpy as np
@@ -18,11 +18,11 @@ MIXES = {
 }
 
 
-def _system(degree, level, seed, method):
+def _system(degree, level, seed, method, dim=2):
     import simplefem_gb300 as S
     from simplefem_gb300 import workloads
     from simplefem_gb300.system import System
-    A, C, V = workloads.lattice_matrix(2, degree, level, seed)
+    A, C, V = workloads.lattice_matrix(dim, degree, level, seed)
     n = len(A) - 1
     s = System(A, C, V)
     if method == "rainbow":
@@ -76,3 +76,33 @@ def test_teams_by_system_size(cuda, mix, method, mode):
             assert np.linalg.norm(x - exact) <= 1e-9 * np.linalg.norm(exact)
     for s, _ in made.values():
         s.close()
+
+
+@pytest.mark.parametrize("method", ["rainbow", "cg"])
+@pytest.mark.parametrize("threads", [256, 512])
+@pytest.mark.parametrize("dim,degree,level", [(2, 1, 3), (2, 2, 4), (3, 1, 3), (3, 2, 2)])
+def test_half_filled_launch_of_columns(cuda, dim, degree, level, threads, method):
+    """Four columns per team: launches whose teams fill at most half of the SMs' threads take the
+    kernel with long chunks of entries, fuller ones the other; rows of 3 to 60 entries give blocks
+    below, at and above both chunk lengths. Every column meets 1e-10 and the exact solution to 1e-9
+    (the bounds of the batched engine's other tests), a last team with one column included."""
+    torch = cuda
+    from simplefem_gb300 import workloads
+    s, M = _system(degree, level, 7, method, dim)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    most = 4 * sms * (512 // threads)            # the columns of the largest half-filled launch
+    Bh = np.stack([workloads.uniform_vector(40 + j, s.n) for j in range(most + 1)])
+    exact = sla.splu(M.tocsc()).solve(Bh.T).T
+    s.set_batch_config(method, "mixed", 4, threads, 1)
+    for columns in (1, 5, most, most + 1):
+        B = torch.from_numpy(Bh[:columns].copy()).cuda()
+        X = torch.zeros_like(B)
+        # restarted CG may take more than the default budget of n iterations on 81 rows
+        infos = s.solve_batch(B, X, method=method, mode="mixed", precision=1e-10, max_iter=20 * s.n)
+        X = X.cpu().numpy()
+        assert all(q["status"] == 0 for q in infos)
+        res = np.linalg.norm(Bh[:columns] - (M @ X.T).T, axis=1)
+        assert (res <= 1e-10 * np.linalg.norm(Bh[:columns], axis=1)).all()
+        err = np.linalg.norm(X - exact[:columns], axis=1)
+        assert (err <= 1e-9 * np.linalg.norm(exact[:columns], axis=1)).all()
+    s.close()
