@@ -163,6 +163,18 @@ bool small_pcg_fits(const feec_system* s);
 int small_pcg_prepare(feec_system* s);
 int launch_small_pcg(feec_system* s, const PcgArgs<double>& a, LaunchShape& shape);
 void small_release(feec_system* s);
+// Natural-order slices of a matrix (kernels_flow_cg.cu), and the form that a solver over them runs
+// in: every vector in registers, vectors in memory with the gathered one published, or (neither) too
+// large for publishing to pay.
+constexpr int kFlowPublishedRows = 80000;   // measured in kernels_flow_cg.cu
+struct FlowForm {
+    int blocks, threads;
+    bool registers, published;
+};
+int flow_natural_build(FlowData& D, cudaStream_t st, int dev, int n, const int* rowptr, const int* A, const int* C,
+                       const double* V, bool f32);
+FlowForm flow_natural_form(const FlowData& D, int n, int sms);
+cudaError_t flow_permute(int n, const int* perm, const double* src, double* dst, bool back, cudaStream_t st);
 // Plain CG (kernels_flow_cg.cu).
 int flow_cg_build(feec_system* s, bool f32);
 int launch_flow_cg(feec_system* s, const CgArgs<double>& a, LaunchShape& shape);

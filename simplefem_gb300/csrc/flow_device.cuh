@@ -344,17 +344,10 @@ __device__ __forceinline__ bool flow_reduce_warps(double* part, DeviceStatus* st
     return true;
 }
 
-// Grid-wide sums of NV (at most 4) accumulators per thread, which is also the iteration's
-// barrier: everything written before it in any block is visible after it in every block.
-// The totals are returned to warp 0 of every block (identical bits in every block: fixed
-// shuffle trees and a fixed order over blocks). With four sums the warp's tree halves the
-// number of values each step (6 additions instead of 20: an FP64 addition costs a warp 64
-// cycles). `part` must not be one that some block may still be reading (callers alternate
-// two). Returns false in every thread when a wait gave up here or, `live` false, before.
+// A warp's part of flow_reduce: its NV sums into sh.warp_sum. With four sums the tree halves the
+// number of values each step (6 additions instead of 20: an FP64 addition costs a warp 64 cycles).
 template <typename T, int NV>
-__device__ __forceinline__ bool flow_reduce(typename AccT<T>::type (&v)[NV], double* part, DeviceStatus* st,
-                                            unsigned long long& epoch, int site, bool live, FlowShared& sh,
-                                            double (&tot)[NV]) {
+__device__ __forceinline__ void flow_warp_sums(const typename AccT<T>::type (&v)[NV], FlowShared& sh) {
     static_assert(NV == 1 || NV == 2 || NV == 4, "sums per reduction");
     using A = AccT<T>;
     using Acc = typename A::type;
@@ -377,6 +370,19 @@ __device__ __forceinline__ bool flow_reduce(typename AccT<T>::type (&v)[NV], dou
     }
     for (int off = rest; off > 0; off >>= 1) k = A::merge(k, A::shfl_xor(k, off));
     if ((lane & (2 * rest - 1)) == 0) sh.warp_sum[warp][idx] = A::value(k);
+}
+
+// Grid-wide sums of NV (at most 4) accumulators per thread, which is also the iteration's
+// barrier: everything written before it in any block is visible after it in every block.
+// The totals are returned to warp 0 of every block (identical bits in every block: fixed
+// shuffle trees and a fixed order over blocks). `part` must not be one that some block may
+// still be reading (callers alternate two). Returns false in every thread when a wait gave up
+// here or, `live` false, before.
+template <typename T, int NV>
+__device__ __forceinline__ bool flow_reduce(typename AccT<T>::type (&v)[NV], double* part, DeviceStatus* st,
+                                            unsigned long long& epoch, int site, bool live, FlowShared& sh,
+                                            double (&tot)[NV]) {
+    flow_warp_sums<T, NV>(v, sh);
     return flow_reduce_warps<NV>(part, st, epoch, site, live, sh, tot);
 }
 

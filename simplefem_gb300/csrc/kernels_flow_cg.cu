@@ -72,7 +72,7 @@ __device__ __forceinline__ void cg_control(const double (&tot)[4], int K, int n,
     }
 }
 
-// kCgRegisters as above. Otherwise the vectors are in memory: up to kCgPublishedRows rows d is
+// kCgRegisters as above. Otherwise the vectors are in memory: up to kFlowPublishedRows rows d is
 // published (kCgPublished; 9.2 us per iteration against 10.8 on 60,000 rows of 3D P1, equal at
 // 100,000); above, publishing costs a sentinel store per row and gathers that skip L1, and a
 // second grid barrier before the product costs less (kCgBarrier). There the product is bound by
@@ -80,7 +80,6 @@ __device__ __forceinline__ void cg_control(const double (&tot)[4], int K, int n,
 // refined 7 times) and wants 32 warps with 4 entries in flight each: 102 us against 111 for 16
 // warps with 8, 107 for 24 with 4, 125 for 32 with 2, and 130 for cg_persistent.
 enum { kCgPublished = 0, kCgRegisters = 1, kCgBarrier = 2 };
-constexpr int kCgPublishedRows = 80000;
 constexpr int kCgBarrierThreads = 1024;
 constexpr int kCgBarrierChunk = 4;
 
@@ -349,41 +348,48 @@ constexpr int kCgRowOps = 7;   // FP64 operations of a row besides its entries
 
 }  // namespace
 
+// The form a natural-order solver runs in: vectors in registers, published, or neither.
+FlowForm flow_natural_form(const FlowData& D, int n, int sms) {
+    FlowForm f;
+    // one warp per scheduler and block before more blocks are added: fewer partial sums to add
+    f.blocks = std::max(1, std::min(sms, (D.nslices + 3) / 4));
+    const int warps = (D.nslices + f.blocks - 1) / f.blocks;
+    f.threads = 32 * std::min(warps, kFlowWarps);
+    f.registers = warps <= kFlowWarps && D.longest <= kFlowChunk;
+    f.published = n <= kFlowPublishedRows;
+    return f;
+}
+
 // Rows sorted by length (longest first, stable) within windows of kSortWindow, slices, columns
-// and the values of the wanted precision; kept with the system.
-int flow_cg_build(feec_system* s, bool f32) {
-    FlowData& D = s->flow_cg;
-    if (D.ready && (f32 ? (void*)D.val32 : (void*)D.val64)) return FEEC_OK;
-    HomeStreamScope home(s);
-    cudaStream_t st = s->stream;
-    const int n = s->n;
+// and the values of the wanted precision, from the device CSR (A, C, V) whose row pointer is also
+// in host memory.
+int flow_natural_build(FlowData& D, cudaStream_t st, int dev, int n, const int* rowptr, const int* A, const int* C,
+                       const double* V, bool f32) {
     const bool first = !D.ready;
     if (first) {
         D.mem.release();
         D = FlowData{};
         D.mem.stream = st;
         int sms = 0;
-        FEEC_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->dev));
-        std::vector<int> A((size_t)n + 1), perm((size_t)n), iperm((size_t)n), len((size_t)n);
-        FEEC_TRY(cudaMemcpyAsync(A.data(), s->A, sizeof(int) * A.size(), cudaMemcpyDeviceToHost, st));
-        FEEC_TRY(cudaStreamSynchronize(st));
+        FEEC_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        std::vector<int> perm((size_t)n), iperm((size_t)n), len((size_t)n);
         std::vector<int> count;
         for (int w = 0; w < n; w += kSortWindow) {   // counting sort of each window, longest first
             const int hi = std::min(n, w + kSortWindow);
             int longest = 0;
-            for (int i = w; i < hi; i++) longest = std::max(longest, A[i + 1] - A[i]);
+            for (int i = w; i < hi; i++) longest = std::max(longest, rowptr[i + 1] - rowptr[i]);
             if (longest > 1 << 16) {
                 std::iota(perm.begin() + w, perm.begin() + hi, w);
                 std::stable_sort(perm.begin() + w, perm.begin() + hi,
-                                 [&](int p, int q) { return A[p + 1] - A[p] > A[q + 1] - A[q]; });
+                                 [&](int p, int q) { return rowptr[p + 1] - rowptr[p] > rowptr[q + 1] - rowptr[q]; });
             } else {
                 count.assign((size_t)longest + 2, 0);
-                for (int i = w; i < hi; i++) count[longest - (A[i + 1] - A[i]) + 1]++;
+                for (int i = w; i < hi; i++) count[longest - (rowptr[i + 1] - rowptr[i]) + 1]++;
                 for (int l = 0; l <= longest; l++) count[l + 1] += count[l];
-                for (int i = w; i < hi; i++) perm[w + count[longest - (A[i + 1] - A[i])]++] = i;
+                for (int i = w; i < hi; i++) perm[w + count[longest - (rowptr[i + 1] - rowptr[i])]++] = i;
             }
         }
-        for (int i = 0; i < n; i++) { iperm[perm[i]] = i; len[i] = A[perm[i] + 1] - A[perm[i]]; }
+        for (int i = 0; i < n; i++) { iperm[perm[i]] = i; len[i] = rowptr[perm[i] + 1] - rowptr[perm[i]]; }
         std::vector<FlowHostSlice> slices;
         // cut for the register form when its slices fit the grid's warps, else freely
         if (!flow_cut_rows(0, n, len.data(), kCgRowOps, sms, kFlowChunk, sms * kFlowWarps, slices))
@@ -414,12 +420,26 @@ int flow_cg_build(feec_system* s, bool f32) {
     if (f32) FEEC_TRY(D.mem.alloc(D.val32, (size_t)D.units * 32));
     else FEEC_TRY(D.mem.alloc(D.val64, (size_t)D.units * 32));
     note_launch();
-    flow_cg_fill_kernel<<<(D.nslices + 7) / 8, 256, 0, st>>>(D.nslices, D.meta, D.perm, D.iperm, s->A, s->C, s->V,
+    flow_cg_fill_kernel<<<(D.nslices + 7) / 8, 256, 0, st>>>(D.nslices, D.meta, D.perm, D.iperm, A, C, V,
                                                             first ? D.ci : nullptr, f32 ? nullptr : D.val64,
                                                             f32 ? D.val32 : nullptr);
     FEEC_TRY(cudaGetLastError());
     D.ready = true;
     return FEEC_OK;
+}
+
+// A system's slices for plain CG, kept with the system.
+int flow_cg_build(feec_system* s, bool f32) {
+    FlowData& D = s->flow_cg;
+    if (D.ready && (f32 ? (void*)D.val32 : (void*)D.val64)) return FEEC_OK;
+    HomeStreamScope home(s);
+    std::vector<int> rowptr;
+    if (!D.ready) {
+        rowptr.resize((size_t)s->n + 1);
+        FEEC_TRY(cudaMemcpyAsync(rowptr.data(), s->A, sizeof(int) * rowptr.size(), cudaMemcpyDeviceToHost, s->stream));
+        FEEC_TRY(cudaStreamSynchronize(s->stream));
+    }
+    return flow_natural_build(D, s->stream, s->dev, s->n, rowptr.data(), s->A, s->C, s->V, f32);
 }
 
 namespace {
@@ -430,6 +450,13 @@ __global__ void permute_kernel(int n, const int* __restrict__ perm, const T* __r
     if (i >= n) return;
     if (back) dst[perm[i]] = src[i];
     else dst[i] = src[perm[i]];
+}
+
+template <typename T>
+cudaError_t permute(int n, const int* perm, const T* src, T* dst, bool back, cudaStream_t st) {
+    note_launch();
+    permute_kernel<T><<<(n + 255) / 256, 256, 0, st>>>(n, perm, src, dst, back);
+    return cudaGetLastError();
 }
 
 template <typename T>
@@ -451,34 +478,30 @@ int flow_cg_launch(feec_system* s, const CgArgs<T>& p, LaunchShape& shape) {
     a.partials = p.partials; a.st = p.st;
     int sms = 0;
     FEEC_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->dev));
-    // one warp per scheduler and block before more blocks are added: fewer partial sums to add
-    shape.blocks = std::max(1, std::min(sms, (D.nslices + 3) / 4));
-    const int warps = (D.nslices + shape.blocks - 1) / shape.blocks;
-    const int mode = warps <= kFlowWarps && D.longest <= kFlowChunk ? kCgRegisters
-                     : p.n <= kCgPublishedRows ? kCgPublished : kCgBarrier;
-    shape.threads = mode == kCgBarrier ? kCgBarrierThreads : 32 * std::min(warps, kFlowWarps);
+    const FlowForm form = flow_natural_form(D, p.n, sms);
+    const int mode = form.registers ? kCgRegisters : form.published ? kCgPublished : kCgBarrier;
+    shape.blocks = form.blocks;
+    shape.threads = mode == kCgBarrier ? kCgBarrierThreads : form.threads;
     shape.lanes = 1;
-    const int grid = (p.n + 255) / 256;
-    note_launch();
-    permute_kernel<T><<<grid, 256, 0, st>>>(p.n, D.perm, p.b, own[0], false);
-    note_launch();
-    permute_kernel<T><<<grid, 256, 0, st>>>(p.n, D.perm, p.x, own[1], false);
-    FEEC_TRY(cudaGetLastError());
+    FEEC_TRY(permute<T>(p.n, D.perm, p.b, own[0], false, st));
+    FEEC_TRY(permute<T>(p.n, D.perm, p.x, own[1], false, st));
     const void* fn = mode == kCgRegisters ? (const void*)flow_cg<T, kCgRegisters>
                      : mode == kCgPublished ? (const void*)flow_cg<T, kCgPublished> : (const void*)flow_cg<T, kCgBarrier>;
     void* args[] = {&a};
     note_launch();
     FEEC_TRY(cudaLaunchCooperativeKernel(fn, dim3(shape.blocks), dim3(shape.threads), args, 0, st));
-    note_launch();
-    permute_kernel<T><<<grid, 256, 0, st>>>(p.n, D.perm, own[1], p.x, true);
-    note_launch();
-    permute_kernel<T><<<grid, 256, 0, st>>>(p.n, D.perm, own[2], p.r, true);
-    return cuda_status(cudaGetLastError());
+    FEEC_TRY(permute<T>(p.n, D.perm, own[1], p.x, true, st));
+    FEEC_TRY(permute<T>(p.n, D.perm, own[2], p.r, true, st));
+    return FEEC_OK;
 }
 
 }  // namespace
 
 int launch_flow_cg(feec_system* s, const CgArgs<double>& a, LaunchShape& shape) { return flow_cg_launch<double>(s, a, shape); }
 int launch_flow_cg(feec_system* s, const CgArgs<float>& a, LaunchShape& shape) { return flow_cg_launch<float>(s, a, shape); }
+
+cudaError_t flow_permute(int n, const int* perm, const double* src, double* dst, bool back, cudaStream_t st) {
+    return permute<double>(n, perm, src, dst, back, st);
+}
 
 }  // namespace feec

@@ -6,6 +6,10 @@
 //   minres_persistent    — MINRESCSR (:2159-2425)
 //   chebyshev_persistent — ChebyshevIteration_DiagonalPreconditioner (:2428-2590)
 //
+// CR and MINRES with at most kFlowPublishedRows rows run kernels_flow_more.cu instead (one sum per
+// iteration, the gathered vector published); the kernels here serve larger systems and those whose
+// slices do not fit the device memory.
+//
 // As in the CG kernels, every grid-wide sum is reduced deterministically (per-block
 // partials, then every block adds them in the same order), scalar recurrences run in
 // thread 0 of every block on identical inputs and are broadcast through shared memory,
@@ -22,6 +26,7 @@
 
 #include "persistent_common.cuh"
 #include "feec_system.h"
+#include "flow_more.h"
 
 namespace feec {
 namespace {
@@ -416,7 +421,6 @@ int more_dropin(int kind, int N, double* x, const double* b, const int* A, const
     FEEC_TRY(m.alloc(dA, (size_t)N + 1)); FEEC_TRY(m.alloc(dC, (size_t)std::max(nnz, 1)));
     FEEC_TRY(m.alloc(dV, (size_t)std::max(nnz, 1))); FEEC_TRY(m.alloc(bad, 1));
     FEEC_TRY(m.alloc(db, (size_t)N)); FEEC_TRY(m.alloc(dx, (size_t)N)); FEEC_TRY(m.alloc(dres, (size_t)N));
-    for (int k = 0; k < 7; k++) FEEC_TRY(m.alloc(w[k], (size_t)N));
     if (kind == kKindChebyshev) FEEC_TRY(m.alloc(dpre, (size_t)N));
     FEEC_TRY(m.alloc(dst, 1));
     FEEC_TRY(cudaMemcpyAsync(dA, A, sizeof(int) * ((size_t)N + 1), cudaMemcpyHostToDevice, s));
@@ -426,9 +430,7 @@ int more_dropin(int kind, int N, double* x, const double* b, const int* A, const
     }
     FEEC_TRY(cudaMemcpyAsync(db, b, sizeof(double) * (size_t)N, cudaMemcpyHostToDevice, s));
     FEEC_TRY(cudaMemcpyAsync(dx, x, sizeof(double) * (size_t)N, cudaMemcpyHostToDevice, s));
-    FEEC_TRY(cudaMemcpyAsync(dres, residual, sizeof(double) * (size_t)N, cudaMemcpyHostToDevice, s));
     if (dpre) FEEC_TRY(cudaMemcpyAsync(dpre, precon, sizeof(double) * (size_t)N, cudaMemcpyHostToDevice, s));
-    for (int k = 0; k < 7; k++) FEEC_TRY(cudaMemsetAsync(w[k], 0xFF, sizeof(double) * (size_t)N, s));   // NaN
     FEEC_TRY(cudaMemsetAsync(bad, 0, sizeof(int), s));
     FEEC_TRY(cudaMemsetAsync(dst, 0, sizeof(DeviceStatus), s));
     // the kernels index x through C: the CSR is checked on the device first
@@ -438,31 +440,73 @@ int more_dropin(int kind, int N, double* x, const double* b, const int* A, const
     FEEC_TRY(cudaStreamSynchronize(s));
     if (hbad) return FEEC_BADARG;
 
-    // one thread per row for short rows (FP64 issue bound), lanes for long ones
-    const double avg = (double)nnz / N;
-    const int lanes = avg <= 32.0 ? 1 : (avg <= 96.0 ? 4 : 8);
-    const void* fn = more_kernel(kind, lanes);
-    int sms = 0, per_sm = 0;
+    // MINRES and CR with at most kFlowPublishedRows rows run the dataflow kernels
+    // (kernels_flow_more.cu); larger ones, Chebyshev (one sum per iteration as it is) and systems
+    // whose slices do not fit the device memory the barrier-phase kernels of this file.
+    int sms = 0;
     FEEC_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    FEEC_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, 0));
-    const long long want = ((long long)N * lanes + kThreads - 1) / kThreads;
-    int blocks = (int)std::min<long long>(want, (long long)std::min(per_sm, 2) * sms);
-    if (blocks < 1) return FEEC_CUDA_ERROR;
-    FEEC_TRY(m.alloc(part, (size_t)4 * blocks));
-
-    MoreArgs args{};
-    args.n = N; args.rp = dA; args.ci = dC; args.val = dV; args.b = db; args.x = dx; args.res = dres;
-    for (int k = 0; k < 7; k++) args.w[k] = w[k];
-    args.precon = dpre; args.lower = lower; args.upper = upper;
-    args.tol = tolerance; args.print_modulo = print_modulo; args.max_iter = N;
-    args.partials = part; args.st = dst;
+    FlowData flow;
+    struct ReleaseFlow { FlowData& f; ~ReleaseFlow() { f.mem.release(); } } rel_flow{flow};
+    bool use_flow = kind != kKindChebyshev && N <= kFlowPublishedRows;
+    if (use_flow && flow_natural_build(flow, s, dev, N, A, dA, dC, dV, false) != FEEC_OK) {
+        cudaGetLastError();
+        flow.mem.release();
+        use_flow = false;
+    }
+    int blocks = 0, lanes = 1;
     cudaEvent_t e0, e1;
-    FEEC_TRY(cudaEventCreate(&e0)); FEEC_TRY(cudaEventCreate(&e1));
-    void* params[] = {&args};
-    cudaEventRecord(e0, s);
-    note_launch();
-    cudaError_t le = cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(kThreads), params, 0, s);
-    cudaEventRecord(e1, s);
+    cudaError_t le = cudaSuccess;
+    if (use_flow) {
+        const FlowForm form = flow_natural_form(flow, N, sms);
+        blocks = form.blocks;
+        for (int k = 0; k < 5; k++) FEEC_TRY(m.alloc(w[k], (size_t)N));
+        FEEC_TRY(m.alloc(part, (size_t)8 * blocks));
+        FlowMoreArgs args{};
+        args.n = N; args.nslices = flow.nslices; args.meta = flow.meta; args.ci = flow.ci; args.val = flow.val64;
+        args.b = flow.own[0]; args.x = flow.own[1]; args.res = flow.own[2];
+        for (int k = 0; k < 5; k++) args.w[k] = w[k];
+        for (int k = 0; k < 2; k++) {
+            args.pub[k] = flow.pub[k];
+            FEEC_TRY(cudaMemsetAsync(flow.pub[k], 0xFF, sizeof(double) * (size_t)N, s));
+        }
+        args.tol = tolerance; args.print_modulo = print_modulo; args.max_iter = N;
+        args.partials = part; args.st = dst;
+        FEEC_TRY(cudaEventCreate(&e0)); FEEC_TRY(cudaEventCreate(&e1));
+        cudaEventRecord(e0, s);
+        le = flow_permute(N, flow.perm, db, flow.own[0], false, s);
+        if (le == cudaSuccess) le = flow_permute(N, flow.perm, dx, flow.own[1], false, s);
+        if (le == cudaSuccess) le = launch_flow_more(kind == kKindMinres, form, args, s);
+        if (le == cudaSuccess) le = flow_permute(N, flow.perm, flow.own[1], dx, true, s);
+        if (le == cudaSuccess) le = flow_permute(N, flow.perm, flow.own[2], dres, true, s);
+        cudaEventRecord(e1, s);
+    } else {
+        // one thread per row for short rows (FP64 issue bound), lanes for long ones
+        const double avg = (double)nnz / N;
+        lanes = avg <= 32.0 ? 1 : (avg <= 96.0 ? 4 : 8);
+        const void* fn = more_kernel(kind, lanes);
+        int per_sm = 0;
+        FEEC_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, 0));
+        const long long want = ((long long)N * lanes + kThreads - 1) / kThreads;
+        blocks = (int)std::min<long long>(want, (long long)std::min(per_sm, 2) * sms);
+        if (blocks < 1) return FEEC_CUDA_ERROR;
+        for (int k = 0; k < 7; k++) {
+            FEEC_TRY(m.alloc(w[k], (size_t)N));
+            FEEC_TRY(cudaMemsetAsync(w[k], 0xFF, sizeof(double) * (size_t)N, s));   // NaN
+        }
+        FEEC_TRY(m.alloc(part, (size_t)4 * blocks));
+        MoreArgs args{};
+        args.n = N; args.rp = dA; args.ci = dC; args.val = dV; args.b = db; args.x = dx; args.res = dres;
+        for (int k = 0; k < 7; k++) args.w[k] = w[k];
+        args.precon = dpre; args.lower = lower; args.upper = upper;
+        args.tol = tolerance; args.print_modulo = print_modulo; args.max_iter = N;
+        args.partials = part; args.st = dst;
+        FEEC_TRY(cudaEventCreate(&e0)); FEEC_TRY(cudaEventCreate(&e1));
+        void* params[] = {&args};
+        cudaEventRecord(e0, s);
+        note_launch();
+        le = cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(kThreads), params, 0, s);
+        cudaEventRecord(e1, s);
+    }
     DeviceStatus hs{};
     if (le == cudaSuccess) le = cudaMemcpyAsync(&hs, dst, sizeof(DeviceStatus), cudaMemcpyDeviceToHost, s);
     if (le == cudaSuccess) le = cudaStreamSynchronize(s);
