@@ -132,8 +132,13 @@ int true_residual(feec_system* s, const double* bb, const double* xx, double* rr
     const int* rp = permuted ? s->rp : s->A;
     const int* ci = permuted ? s->ci : s->C;
     const double* v = permuted ? s->val : s->V;
-    const int nb = residual_blocks(s->n, s->lanes);
-    FEEC_TRY(launch_residual_f64(s->n, rp, ci, v, bb, xx, rr, s->partials, s->lanes, s->stream));
+    // At most four lanes per row: a warp's FP64 operation takes an SM 19 - 20 cycles whatever its
+    // lanes add, so the tree over more lanes costs more than the shorter loads save (3D P2 refined
+    // 5 times, 28 entries per row: 121 us at 16 lanes, 44 at 4, a solve of six such products 11.9 ms
+    // and 11.5; 3D P3, 50 and more entries per row: 11.86 ms at 32 lanes, 11.77 at 8, 4 and 2).
+    const int lanes = std::min(s->lanes, 4);
+    const int nb = residual_blocks(s->n, lanes);
+    FEEC_TRY(launch_residual_f64(s->n, rp, ci, v, bb, xx, rr, s->partials, lanes, s->stream));
     FEEC_TRY(launch_sum_f64(nb, s->partials, s->scal, s->stream));
     FEEC_TRY(cudaMemcpyAsync(&norm2, s->scal, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
     FEEC_TRY(cudaStreamSynchronize(s->stream));

@@ -238,3 +238,23 @@ def test_minres_and_cr_match_oracle(cuda, name, make, solver):
     assert np.linalg.norm(x - x_o) <= 1e-9 * np.linalg.norm(x_o), info
     # MINRES returns the true residual, CR its recursion's: both are at the solution's accuracy
     assert np.linalg.norm(res - (b - M @ x)) <= 1e-11 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("n", [1, 31, 1025, 8191, 8193, 65_537, 300_001])
+def test_norms_over_blocks(cuda, n):
+    """The right-hand side's norm (one cluster of eight blocks, 8192 values a step) and the true
+    residual's, through the reported quotient of the two, against numpy: a sum of n squares is off by at most a few units per addition in
+    a chain, here n / 8192 + 30 of them, far below 1e-13."""
+    import torch
+    from simplefem_gb300.system import System
+    M = _diagonal(n) if n < 3 else _tridiagonal(n)
+    M.sort_indices()
+    sysm = System(M.indptr.astype(np.int32), M.indices.astype(np.int32), M.data.astype(np.float64))
+    rng = np.random.default_rng(n)
+    b, x0 = rng.uniform(-1.0, 1.0, n), rng.uniform(-1.0, 1.0, n)
+    x = torch.from_numpy(x0).cuda()
+    info = sysm.solve(torch.from_numpy(b).cuda(), x, method="cg", mode="fp64", precision=1e-3, max_iter=1)
+    xh = x.cpu().numpy()
+    rel = np.linalg.norm(b - M @ xh) / np.linalg.norm(b)
+    assert abs(info["true_relres"] - rel) <= 1e-13 * max(rel, 1.0), (info, rel)
+    sysm.close()
