@@ -42,7 +42,7 @@ int grid_of(long long n) { return (int)std::max<long long>(1, (n + kAlgBlock - 1
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kWarpsPerBlock = 4;
 constexpr int kWarpBlock = kWarpsPerBlock * 32;
-constexpr int kRowCap = 1024;   // (column, slot) entries of one row staged in shared memory per warp (8 KB)
+constexpr int kRowCap = 1024;   // words of one row staged in shared memory per warp (4 KB)
 
 int warp_grid(long long rows) { return (int)std::max<long long>(1, (rows + kWarpsPerBlock - 1) / kWarpsPerBlock); }
 
@@ -111,47 +111,121 @@ __device__ void warp_exchange_sort(int2* cs, double* v, int L, int lane) {
     }
 }
 
+// The same sort on packed entries: column - (smallest of the row) above, then the zero flag, then
+// the slot, in one 32-bit word; kNone (no word of a row) marks no entry and pads [L, L + 32).
+// With the column on top, a pass is min and max: an entry of another column is swapped in exactly
+// when its word is smaller, and of two words of one column the smaller holds the nonzero value if
+// only one does. Of two nonzeros the sum goes to the smaller word's slot, whichever it is, and the
+// other is flagged. An empty register holds kNone, so that its position's entry is swapped in.
+// A third of the instructions per step (the sort is issue-bound), one word in shared memory
+// instead of two: compress_rows_kernel on the product of 3D P1 operators refined 4 times
+// (4,913 rows of up to 225 entries) 356 -> 159 us.
+constexpr unsigned kNone = 0xffffffffu;
+
+// Two or four passes per lane and step (fewer shuffles and loads per compare) take the same time.
+__device__ void warp_exchange_sort_packed(unsigned* cs, double* v, int L, unsigned flag, int lane) {
+    const unsigned slot = flag - 1;
+    for (int i = 0; i < L; i += 32) {
+        unsigned r = kNone, p = kNone, nx = cs[i];
+        const int steps = (L - i) + 31;
+        unsigned* out = cs + i - 31;
+        for (int s = 0; s < steps; s++) {
+            unsigned x = __shfl_up_sync(kFull, p, 1);
+            if (lane == 0) x = nx;
+            nx = cs[i + s + 1];                                   // at most L + 31
+            const unsigned lo = min(x, r);
+            p = max(x, r);
+            const bool add = ((x ^ r) | ((x | r) & flag)) < flag;   // one column, two nonzeros
+            r = lo;
+            if (__any_sync(kFull, add)) {
+                slot_add(add, v, (int)(lo & slot), (int)(p & slot));
+                if (add) p |= flag;
+            }
+            if (lane == 31 && p != kNone) out[s] = p;              // position i + s - 31 < L
+        }
+        if (i + lane < L) cs[i + lane] = r;
+        __syncwarp();
+    }
+}
+
 // The nonzero entries of the sorted row, in order, written to (dc, dv); returns their
 // count. This is the reference's zero bubble pass (:624-649), a stable partition.
-__device__ int warp_keep_nonzeros(const int2* cs, const double* v, int L, int* __restrict__ dc,
-                                  double* __restrict__ dv, int lane) {
+// get(q, column, slot): entry q, false for a flagged zero.
+template <typename Get>
+__device__ int warp_keep_nonzeros(Get&& get, const double* v, int L, int* __restrict__ dc, double* __restrict__ dv,
+                                  int lane) {
     int k = 0;
     for (int base = 0; base < L; base += 32) {
         const int q = base + lane;
-        int2 e = make_int2(0, kZeroSlot);
-        if (q < L) e = cs[q];
+        int col = 0, slot = 0;
+        const bool live = q < L && get(q, col, slot);
         double val = 0.0;
-        if (e.y >= 0) val = v[e.y];
-        const bool keep = e.y >= 0 && ((__double_as_longlong(val) << 1) != 0);
+        if (live) val = v[slot];
+        const bool keep = live && ((__double_as_longlong(val) << 1) != 0);
         const unsigned m = __ballot_sync(kFull, keep);
-        if (keep) { const int d = k + __popc(m & ((1u << lane) - 1u)); dc[d] = e.x; dv[d] = val; }
+        if (keep) { const int d = k + __popc(m & ((1u << lane) - 1u)); dc[d] = col; dv[d] = val; }
         k += __popc(m);
     }
     return k;
 }
 
 // One warp per row: the row's entries get slots (zero values flagged), are sorted and
-// merged (the (column, slot) stream in shared memory when the row fits, else in the global
-// scratch `cs`; the values stay in V, where only merges of two nonzeros and the final pass
-// touch them), and the nonzeros are written to (Co, Vo) from the row's start; cnt[r] =
-// their count.
+// merged (the stream in shared memory when the row fits, else in the global scratch `cs`;
+// the values stay in V, where only merges of two nonzeros and the final pass touch them),
+// and the nonzeros are written to (Co, Vo) from the row's start; cnt[r] = their count.
+// A row is packed when its columns' span, its length and the flag fit in one word.
 __global__ void __launch_bounds__(kWarpBlock)
 compress_rows_kernel(int rows, const int* __restrict__ A, const int* __restrict__ C, double* V, int2* cs,
                      int* __restrict__ Co, double* __restrict__ Vo, int* __restrict__ cnt) {
-    __shared__ int2 scs[kWarpsPerBlock][kRowCap];
+    __shared__ __align__(8) unsigned words[kWarpsPerBlock][kRowCap + 32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int r = blockIdx.x * kWarpsPerBlock + w;
     if (r >= rows) return;
     const int lo = A[r], L = A[r + 1] - lo;
-    int2* rcs = L <= kRowCap ? scs[w] : cs + lo;
     double* rv = V + lo;
+    int cmin = INT_MAX, cmax = 0;
     for (int q = lane; q < L; q += 32) {
-        const int zero = ((__double_as_longlong(rv[q]) << 1) == 0) ? kZeroSlot : 0;
-        rcs[q] = make_int2(C[lo + q], q | zero);
+        const int c = C[lo + q];
+        cmin = min(cmin, c);
+        cmax = max(cmax, c);
     }
-    __syncwarp();
-    warp_exchange_sort(rcs, rv, L, lane);
-    const int k = warp_keep_nonzeros(rcs, rv, L, Co + lo, Vo + lo, lane);
+    cmin = __reduce_min_sync(kFull, cmin);
+    cmax = __reduce_max_sync(kFull, cmax);
+    const int bits = 32 - __clz(max(L, 2) - 1);                    // of a slot
+    int k;
+    if (L > 0 && bits < 31 && (unsigned)(cmax - cmin) < (1u << (31 - bits)) - 1u) {
+        const unsigned flag = 1u << bits;
+        unsigned* e = L <= kRowCap ? words[w] : (unsigned*)(cs + lo);   // 2 L >= L + 32 words there
+        for (int q = lane; q < L + 32; q += 32) {
+            unsigned x = kNone;
+            if (q < L) {
+                const bool zero = (__double_as_longlong(rv[q]) << 1) == 0;
+                x = (unsigned)(C[lo + q] - cmin) << (bits + 1) | (zero ? flag : 0u) | (unsigned)q;
+            }
+            e[q] = x;
+        }
+        __syncwarp();
+        warp_exchange_sort_packed(e, rv, L, flag, lane);
+        k = warp_keep_nonzeros([&](int q, int& col, int& slot) {
+            const unsigned x = e[q];
+            col = (int)(x >> (bits + 1)) + cmin;
+            slot = (int)(x & (flag - 1));
+            return (x & flag) == 0;
+        }, rv, L, Co + lo, Vo + lo, lane);
+    } else {
+        int2* e = L <= kRowCap / 2 ? (int2*)words[w] : cs + lo;
+        for (int q = lane; q < L; q += 32) {
+            const int zero = ((__double_as_longlong(rv[q]) << 1) == 0) ? kZeroSlot : 0;
+            e[q] = make_int2(C[lo + q], q | zero);
+        }
+        __syncwarp();
+        warp_exchange_sort(e, rv, L, lane);
+        k = warp_keep_nonzeros([&](int q, int& col, int& slot) {
+            col = e[q].x;
+            slot = e[q].y;
+            return slot >= 0;
+        }, rv, L, Co + lo, Vo + lo, lane);
+    }
     if (lane == 0) cnt[r] = k;
 }
 
