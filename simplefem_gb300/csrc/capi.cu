@@ -18,6 +18,7 @@
 #include "feec_device.cuh"
 #include "feec_internal.h"
 #include "feec_system.h"
+#include "host_checks.h"
 
 namespace feec {
 
@@ -1173,12 +1174,7 @@ int feec_rainbow(int N, const int* A, const int* C, int* num_colors, int* F, int
 }
 
 int feec_csr_check(int rows, int cols, const int* A, const int* C, const double* V) {
-    if (rows < 0 || cols < 0 || !A) return FEEC_BADARG;
-    if (A[0] != 0) return FEEC_BADARG;
-    for (int p = 1; p <= rows; p++) if (A[p - 1] > A[p]) return FEEC_BADARG;
-    const int nnz = A[rows];
-    for (int i = 0; i < nnz; i++)
-        if (C[i] < 0 || C[i] >= cols || !std::isfinite(V[i])) return FEEC_BADARG;
+    if (!csr_ok(rows, cols, A, C) || (A[rows] > 0 && !V) || !all_finite(A[rows], V)) return FEEC_BADARG;
     return FEEC_OK;
 }
 

@@ -31,6 +31,7 @@
 #include "feec_device.cuh"
 #include "feec_internal.h"
 #include "feec_system.h"
+#include "host_checks.h"
 
 namespace feec {
 namespace {
@@ -533,23 +534,20 @@ __global__ void coo_product_big_rows_kernel(int rows, const int* __restrict__ LA
 }
 
 // Host-side checks of a CSR given by host pointers.
-bool csr_ok(int rows, int cols, const int* A, const int* C) {
-    if (rows < 0 || cols < 0 || !A || A[0] != 0) return false;
-    for (int r = 0; r < rows; r++) if (A[r + 1] < A[r]) return false;
-    const int nnz = A[rows];
-    if (nnz > 0 && !C) return false;
-    for (int i = 0; i < nnz; i++) if (C[i] < 0 || C[i] >= cols) return false;
-    return true;
+// Entries of the product of a checked (A1, C1) with a matrix of row pointers A2.
+long long product_entries(int rows, const int* A1, const int* C1, const int* A2) {
+    long long total = 0;
+    for (int i = 0; i < A1[rows]; i++) total += A2[C1[i] + 1] - A2[C1[i]];
+    return total;
 }
 
-// Compress the rows laid out at (dA, dC, dV), compact them into (oA, oC, oV) on the device.
-int compress_and_compact(DevArena& m, cudaStream_t s, int rows, int* dA, int* dC, double* dV, int*& oA, int*& oC,
+// Compress the rows laid out at (dA, dC, dV), `total` entries, compact them into (oA, oC, oV) on the
+// device.
+int compress_and_compact(DevArena& m, cudaStream_t s, int rows, int total, int* dA, int* dC, double* dV, int*& oA, int*& oC,
                          double*& oV, int& nnz_out) {
-    int *cnt = nullptr, *off = nullptr, *scr = nullptr, *Co = nullptr, total = 0;
+    int *cnt = nullptr, *off = nullptr, *scr = nullptr, *Co = nullptr;
     int2* cs = nullptr;
     double* Vo = nullptr;
-    FEEC_TRY(cudaMemcpyAsync(&total, dA + rows, sizeof(int), cudaMemcpyDeviceToHost, s));
-    FEEC_TRY(cudaStreamSynchronize(s));
     FEEC_TRY(m.alloc(cnt, (size_t)rows + 1)); FEEC_TRY(m.alloc(off, (size_t)rows + 1));
     FEEC_TRY(m.alloc(scr, scan_scratch_ints(rows + 1)));
     FEEC_TRY(m.alloc(cs, (size_t)std::max(total, 1))); FEEC_TRY(m.alloc(Co, (size_t)std::max(total, 1)));
@@ -670,7 +668,7 @@ int feec_csr_add(int rows, int cols, const int* A1, const int* C1, const double*
     add_layout_kernel<<<warp_grid(rows), kWarpBlock, 0, s>>>(rows, dA1, dC1, dV1, dA2, dC2, dV2, s1, s2, dA, dC, dV);
     FEEC_TRY(cudaGetLastError());
     int *oA, *oC; double* oV; int n = 0;
-    if ((st = compress_and_compact(sc.m, s, rows, dA, dC, dV, oA, oC, oV, n)) != FEEC_OK) return st;
+    if ((st = compress_and_compact(sc.m, s, rows, (int)cap, dA, dC, dV, oA, oC, oV, n)) != FEEC_OK) return st;
     if ((st = download(s, rows, n, oA, oC, oV, A, C, V)) != FEEC_OK) return st;
     *nnz = n;
     return FEEC_OK;
@@ -679,10 +677,7 @@ int feec_csr_add(int rows, int cols, const int* A1, const int* C1, const double*
 int feec_csr_multiply_size(int rows, int inner, const int* A1, const int* C1, const int* A2, long long* size) {
     if (!csr_ok(rows, inner, A1, C1) || !A2 || !size) return FEEC_BADARG;
     for (int r = 0; r < inner; r++) if (A2[r + 1] < A2[r] || A2[0] != 0) return FEEC_BADARG;
-    long long total = 0;
-    for (int r = 0; r < rows; r++)
-        for (int c1 = A1[r]; c1 < A1[r + 1]; c1++) total += A2[C1[c1] + 1] - A2[C1[c1]];
-    *size = total;
+    *size = product_entries(rows, A1, C1, A2);
     return FEEC_OK;
 }
 
@@ -690,10 +685,10 @@ int feec_csr_multiply(int rows, int inner, int cols, const int* A1, const int* C
                       const int* C2, const double* V2, int* A, int* C, double* V, int* nnz) {
     if (!csr_ok(rows, inner, A1, C1) || !csr_ok(inner, cols, A2, C2) || !A || !nnz) return FEEC_BADARG;
     if ((A1[rows] > 0 && !V1) || (A2[inner] > 0 && !V2)) return FEEC_BADARG;
-    long long cap = 0;
-    int st = feec_csr_multiply_size(rows, inner, A1, C1, A2, &cap);
-    if (st != FEEC_OK) return st;
-    if (cap > INT_MAX || (cap > 0 && (!C || !V))) return FEEC_BADARG;
+    // a bound first: the entries are counted here only where they might not fit an int
+    int st = FEEC_OK, longest = 0;
+    for (int k = 0; k < inner; k++) longest = std::max(longest, A2[k + 1] - A2[k]);
+    if ((long long)A1[rows] * longest > INT_MAX && product_entries(rows, A1, C1, A2) > INT_MAX) return FEEC_BADARG;
     int dev = 0; cudaStream_t s = nullptr;
     if ((st = init_device(dev, s)) != FEEC_OK) return st;
     Scope sc{DevArena{}, s}; sc.m.stream = s;
@@ -705,19 +700,23 @@ int feec_csr_multiply(int rows, int inner, int cols, const int* A1, const int* C
     long long* len64; int *len, *dA, *dC, *scr; double* dV;
     FEEC_TRY(sc.m.alloc(len64, (size_t)rows + 1)); FEEC_TRY(sc.m.alloc(len, (size_t)rows + 1));
     FEEC_TRY(sc.m.alloc(dA, (size_t)rows + 1)); FEEC_TRY(sc.m.alloc(scr, scan_scratch_ints(rows + 1)));
-    FEEC_TRY(sc.m.alloc(dC, (size_t)std::max<long long>(cap, 1))); FEEC_TRY(sc.m.alloc(dV, (size_t)std::max<long long>(cap, 1)));
     FEEC_TRY(cudaMemsetAsync(len + rows, 0, sizeof(int), s));
     note_launch();
     mul_lengths_kernel<<<grid_of(rows), kAlgBlock, 0, s>>>(rows, dA1, dC1, dA2, len64);
     note_launch();
-    ll_to_int_kernel<<<grid_of(rows), kAlgBlock, 0, s>>>(rows, len64, len);   // cap <= INT_MAX: every row fits
+    ll_to_int_kernel<<<grid_of(rows), kAlgBlock, 0, s>>>(rows, len64, len);   // the sum fits an int: every row does
     FEEC_TRY(cudaGetLastError());
     FEEC_TRY(launch_exclusive_scan(rows + 1, len, dA, scr, s));
+    int cap = 0;
+    FEEC_TRY(cudaMemcpyAsync(&cap, dA + rows, sizeof(int), cudaMemcpyDeviceToHost, s));
+    FEEC_TRY(cudaStreamSynchronize(s));
+    if (cap > 0 && (!C || !V)) return FEEC_BADARG;
+    FEEC_TRY(sc.m.alloc(dC, (size_t)std::max(cap, 1))); FEEC_TRY(sc.m.alloc(dV, (size_t)std::max(cap, 1)));
     note_launch();
     mul_layout_kernel<<<warp_grid(rows), kWarpBlock, 0, s>>>(rows, dA1, dC1, dV1, dA2, dC2, dV2, dA, dC, dV);
     FEEC_TRY(cudaGetLastError());
     int *oA, *oC; double* oV; int n = 0;
-    if ((st = compress_and_compact(sc.m, s, rows, dA, dC, dV, oA, oC, oV, n)) != FEEC_OK) return st;
+    if ((st = compress_and_compact(sc.m, s, rows, cap, dA, dC, dV, oA, oC, oV, n)) != FEEC_OK) return st;
     if ((st = download(s, rows, n, oA, oC, oV, A, C, V)) != FEEC_OK) return st;
     *nnz = n;
     return FEEC_OK;
@@ -757,7 +756,7 @@ int feec_csr_transpose(int rows, int cols, const int* A, const int* C, const dou
     transpose_fill_kernel<<<warp_grid(cols), kWarpBlock, 0, s>>>(cols, dB, idx, row_of, dV, dD, dW);
     FEEC_TRY(cudaGetLastError());
     int *oA, *oC; double* oV; int n = 0;
-    if ((st = compress_and_compact(sc.m, s, cols, dB, dD, dW, oA, oC, oV, n)) != FEEC_OK) return st;
+    if ((st = compress_and_compact(sc.m, s, cols, m, dB, dD, dW, oA, oC, oV, n)) != FEEC_OK) return st;
     if ((st = download(s, cols, n, oA, oC, oV, B, D, W)) != FEEC_OK) return st;
     *nnz = n;
     return FEEC_OK;
