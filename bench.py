@@ -213,7 +213,7 @@ def run_spmv(dev, reps=20):
         t = float(np.median(ms))
         b = S_ * nnz + 4 * (n + 1) + 2 * w * n
         gbs = b / (t / 1000.0) / 1e9
-        out[tag] = {"us": 1000 * t, "bytes": b, "achieved_gbs": gbs, "frac": gbs / peak, "kernel": f"sell_spmv_kernel<{'double' if tag == 'fp64' else 'float'}>"}
+        out[tag] = {"us": 1000 * t, "bytes": b, "achieved_gbs": gbs, "frac": gbs / peak, "kernel": f"sell_spmv_{'f64' if tag == 'fp64' else 'f32'}_kernel"}
     out["peak_gbs"] = peak
     out["peak_kind"] = kind
     sysm.close()

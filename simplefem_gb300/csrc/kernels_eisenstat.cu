@@ -18,6 +18,10 @@
 // 2 * phases + 2 grid barriers. T = double is the drop-in (the reference's stopping rule);
 // T = float is the inner solve of the mixed-precision mode (stops when z.r has fallen by
 // a given factor, compensated FP32 sums).
+//
+// Multicolor layouts run flow_eisenstat (kernels_flow.cu), 229 -> 66 us per FP64 iteration on 3D P2
+// refined 5 times. This kernel serves index-order layouts, layouts with rows whose diagonal is 0,
+// caller launch shapes, and systems whose slices do not fit the device memory.
 #include <cmath>
 #include <cstdio>
 

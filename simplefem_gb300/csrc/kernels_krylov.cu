@@ -12,6 +12,12 @@
 //
 // T = double is the drop-in FP64 path; T = float is the inner solver of the
 // mixed-precision mode (FP32 storage, FP32 arithmetic, compensated FP32 dots).
+//
+// Plain CG and multicolor layouts run kernels_flow_cg.cu and kernels_flow.cu (no barrier
+// between phases, one sum per iteration: 2.5 and 2.8 times as fast on 2D P1 refined 6 times and
+// 3D P2 refined 5 times). These kernels serve what those leave: index-order layouts above the
+// one-block solver's size, the diagonal preconditioner, layouts with rows whose diagonal is 0,
+// caller launch shapes, and systems whose slices do not fit the device memory.
 #include <cmath>
 #include <cstdio>
 #include <type_traits>

@@ -2,6 +2,7 @@
 // norms for the defect-correction loop, diagonal extraction, and the integer
 // layout work that turns a CSR matrix plus an ordering into the row-permuted
 // [L | E | U] split layout that the SSOR / multicolor SSOR sweeps stream.
+#include <algorithm>
 #include <cstdint>
 
 #include <cooperative_groups.h>
@@ -298,12 +299,13 @@ __global__ void sell_fill_kernel(int nslices, const int* __restrict__ row0, cons
     }
 }
 
-// SELL-32 SpMV, one thread per row. The matrix is streamed once (evict-first loads,
+// FP32 SELL-32 SpMV, one thread per row. The matrix is streamed once (evict-first loads,
 // so it does not push x out of L2); a chunk of column indices and values is loaded
 // before its gathers so every warp keeps several requests in flight.
-template <typename T>
-__global__ void __launch_bounds__(256) sell_spmv_kernel(SellView v, const T* __restrict__ x, T* __restrict__ y, T scaling) {
-    const T* __restrict__ val = sizeof(T) == 4 ? (const T*)v.val32 : (const T*)v.val64;
+__global__ void __launch_bounds__(256) sell_spmv_f32_kernel(SellView v, const float* __restrict__ x, float* __restrict__ y,
+                                                            float scaling) {
+    using T = float;
+    const float* __restrict__ val = v.val32;
     const int lane = threadIdx.x & 31;
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
@@ -342,8 +344,72 @@ __global__ void __launch_bounds__(256) sell_spmv_kernel(SellView v, const T* __r
             #pragma unroll
             for (int u = 0; u < CH; u++) { c[u] = cn[u]; a[u] = an[u]; }
         }
-        // FP64 issues at 2 lanes/clk/SM on this part: skip the multiply when scaling == 1
         if (lane < nrow) y[row0 + lane] = scaling == T(1) ? s : scaling * s;
+    }
+}
+
+// One slice of the FP64 SELL-32 SpMV in chunks of CH entries, software-pipelined: the next chunk's
+// indices and values are requested together with the current chunk's gathers, so a chunk costs one
+// memory round trip.
+template <int CH>
+__device__ __forceinline__ double sell_row(const int* __restrict__ ci, const double* __restrict__ val, int L,
+                                           const double* __restrict__ x) {
+    double s = 0.0;
+    int c[CH]; double a[CH];
+    #pragma unroll
+    for (int u = 0; u < CH; u++) {
+        const bool ok = u < L;
+        c[u] = ok ? __ldcs(ci + 32 * u) : 0;
+        a[u] = ok ? __ldcs(val + 32 * u) : 0.0;
+    }
+    for (int k0 = 0; k0 < L; k0 += CH) {
+        double xv[CH];
+        #pragma unroll
+        for (int u = 0; u < CH; u++) xv[u] = __ldg(&x[c[u]]);
+        int cn[CH]; double an[CH];
+        ci += 32 * CH; val += 32 * CH;
+        #pragma unroll
+        for (int u = 0; u < CH; u++) {
+            const bool ok = k0 + CH + u < L;
+            cn[u] = ok ? __ldcs(ci + 32 * u) : 0;
+            an[u] = ok ? __ldcs(val + 32 * u) : 0.0;
+        }
+        #pragma unroll
+        for (int u = 0; u < CH; u++) s = fma(a[u], xv[u], s);
+        #pragma unroll
+        for (int u = 0; u < CH; u++) { c[u] = cn[u]; a[u] = an[u]; }
+    }
+    return s;
+}
+
+// FP64 SELL-32 SpMV, one thread per row, co-limited by HBM and by the FP64 rate (19 - 20 cycles of
+// an SM per warp instruction: 15 of them per 32 rows of 3D P1 take 63 us of the 71 on 2,146,689
+// rows). A chunk's unused slots take FP64 time as well, so the chunk is 7 for slices of 7 entries
+// (2D P1) and else 5, which 15 (3D P1) fills and 27 and 65 (3D P2) nearly do; slices longer than
+// kSellLong waste little either way and take 8 for the loads in flight. Against chunks of 8 for
+// all (same sums in the same order), us per product, back to back: 3D P1 refined 7 times 74.1 ->
+// 71.9, 6 times 14.3 -> 12.8; 3D P2 refined 5 times 34.6 -> 32.0; 2D P1 refined 10 times 26.6 -> 22.7;
+// 3D P3 refined 4 times 30.7 both (31.4 with chunks of 5).
+constexpr int kSellLong = 65;
+__global__ void __launch_bounds__(256) sell_spmv_f64_kernel(SellView v, const double* __restrict__ x, double* __restrict__ y,
+                                                            double scaling) {
+    const int lane = threadIdx.x & 31;
+    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nw = (gridDim.x * blockDim.x) >> 5;
+    for (int sl = gw; sl < v.nslices; sl += nw) {
+        const int row0 = __ldg(&v.slice_row0[sl]);
+        const int nrow = __ldg(&v.slice_nrow[sl]);
+        const int4 len = __ldg(&v.slice_len[sl]);
+        const long long off = __ldg(&v.slice_off[sl]) + lane;
+        const int L = len.x + len.y + len.z;
+        const int* ci = v.ci + off;
+        const double* val = v.val64 + off;
+        double s;
+        if (L == 7) s = sell_row<7>(ci, val, L, x);
+        else if (L <= kSellLong) s = sell_row<5>(ci, val, L, x);
+        else s = sell_row<8>(ci, val, L, x);
+        // FP64 issues at 2 lanes/clk/SM on this part: skip the multiply when scaling == 1
+        if (lane < nrow) y[row0 + lane] = scaling == 1.0 ? s : scaling * s;
     }
 }
 
@@ -536,11 +602,12 @@ cudaError_t launch_sell_spmv(const SellView& v, int is_float, const void* x, voi
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int grid = grid_for((long long)v.nslices * 32, 256);
-    if (grid > sms * 8) grid = sms * 8;
+    const int grid = grid_for((long long)v.nslices * 32, 256);
     if (is_float)
-        return launch(sell_spmv_kernel<float>, grid, 256, s, v, (const float*)x, (float*)y, (float)scaling);
-    return launch(sell_spmv_kernel<double>, grid, 256, s, v, (const double*)x, (double*)y, scaling);
+        return launch(sell_spmv_f32_kernel, std::min(grid, sms * 8), 256, s, v, (const float*)x, (float*)y, (float)scaling);
+    // 48 registers: five blocks per SM at a time; 8 and 10 blocks of them in a fixed grid: 24.6 and
+    // 23.6 us on 2D P1 refined 10 times, 16: 22.7
+    return launch(sell_spmv_f64_kernel, std::min(grid, sms * 16), 256, s, v, (const double*)x, (double*)y, scaling);
 }
 
 cudaError_t launch_sell_lengths(int nslices, const int* slice_row0, const int* slice_nrow, const int* rp,

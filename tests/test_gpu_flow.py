@@ -258,3 +258,29 @@ def test_norms_over_blocks(cuda, n):
     rel = np.linalg.norm(b - M @ xh) / np.linalg.norm(b)
     assert abs(info["true_relres"] - rel) <= 1e-13 * max(rel, 1.0), (info, rel)
     sysm.close()
+
+
+@pytest.mark.parametrize("scaling", [1.0, -0.75])
+@pytest.mark.parametrize("length", [1, 4, 5, 6, 7, 8, 14, 15, 16, 64, 65, 66, 72, 73, 130])
+def test_product_over_slice_lengths(cuda, length, scaling):
+    """y = scaling A x for slices of one length each around the chunk lengths (5, 7, 8), a last slice
+    that is not full and rows without entries among them. A row of k entries is off by at most k
+    units of rounding of its sum of magnitudes, plus one for the scaling."""
+    import torch
+    from simplefem_gb300.system import System
+    n = 32 * 5 + 9
+    rng = np.random.default_rng(length)
+    counts = np.full(n, length)
+    counts[[3, 40]] = 0
+    A = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    C = np.concatenate([np.sort(rng.choice(n, k, replace=False)) for k in counts]).astype(np.int32)
+    V = rng.standard_normal(len(C))
+    x = rng.standard_normal(n)
+    M = sp.csr_matrix((V, C, A), shape=(n, n))
+    s = System(A, C, V)
+    y = torch.full((n,), np.nan, dtype=torch.float64, device="cuda")
+    s.apply(torch.from_numpy(x).cuda(), y, scaling)
+    y = y.cpu().numpy()
+    bound = (length + 1) * np.finfo(np.float64).eps * abs(scaling) * (abs(M) @ np.abs(x))
+    assert (np.abs(y - scaling * (M @ x)) <= bound).all()
+    s.close()
