@@ -789,7 +789,7 @@ int feec_batch_create(feec_batch** out, int nsys, feec_system* const* systems, i
     if (is_float) {
         // FP32 storage pays where the batch is bound by memory traffic; for batches of small
         // systems the FP32 segments' extra iterations can cost more than it saves (512 2D
-        // systems of 81 to 66,049 unknowns: 580 solves/s mixed against 706 in FP64). The
+        // systems of 81 to 66,049 unknowns, one block each: 580 solves/s mixed against 706 in FP64). The
         // batch is replayed once each way from the same initial guess (the FP32 run
         // including the FP64 finish of stagnated systems), x is put back, and the faster
         // graph is kept; results report it in inner_fp64.

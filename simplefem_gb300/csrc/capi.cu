@@ -253,7 +253,7 @@ int solve_core(feec_system* s, int method, int mode, double* xx, const double* b
     // and its second with FP64 ones (device time per decade of residual fall) and keeps the
     // faster for later solves of the same method. The phases of a single solve are latency-
     // bound, so FP32 storage may not pay for its extra iterations (3D P1 refined 7 times:
-    // 223 ms against 168 in FP64); the result reports the choice in inner_fp64.
+    // 118 ms against 98 in FP64); the result reports the choice in inner_fp64.
     const int pick_slot = method == FEEC_METHOD_CG ? 0 : 1;
     bool inner64 = false;
     if (mode == FEEC_MODE_MIXED) {
