@@ -204,7 +204,9 @@ MORE_CASES = CASES + [("scaled_identity", lambda: 2.0 * sp.identity(70, format="
                       ("tridiagonal_5000", lambda: _tridiagonal(5000)), ("p1_2d", lambda: _lattice(2, 1, 6, 0)),
                       ("many_rows_published", lambda: _lattice(3, 1, 5, 30_011)),
                       ("p2_published", lambda: _lattice(3, 2, 4, 0)),
-                      ("empty_rows", lambda: _lattice(2, 1, 4, 0))]
+                      ("empty_rows", lambda: _lattice(2, 1, 4, 0)),
+                      ("rows_90011", lambda: _lattice(3, 1, 6, 90_011)),
+                      ("rows_200017", lambda: _lattice(3, 1, 6, 200_017))]
 
 
 @pytest.mark.parametrize("solver", ["minres", "cr"])
