@@ -453,19 +453,25 @@ int more_dropin(int kind, int N, double* x, const double* b, const int* A, const
     FlowData flow;
     struct ReleaseFlow { FlowData& f; ~ReleaseFlow() { f.mem.release(); } } rel_flow{flow};
     bool use_flow = kind == kKindMinres || (kind != kKindChebyshev && N <= kFlowCrRows);
-    if (use_flow && flow_natural_build(flow, s, dev, N, A, dA, dC, dV, false) != FEEC_OK) {
-        cudaGetLastError();
-        flow.mem.release();
-        use_flow = false;
+    FlowForm form{};
+    if (use_flow) {
+        bool ok = flow_natural_build(flow, s, dev, N, A, dA, dC, dV, false) == FEEC_OK;
+        if (ok) {
+            form = flow_natural_form(flow, N, sms);
+            for (int k = 0; k < 5 && ok; k++) ok = flow.mem.alloc(w[k], (size_t)N) == cudaSuccess;
+            ok = ok && flow.mem.alloc(part, (size_t)8 * form.blocks) == cudaSuccess;
+        }
+        if (!ok) {
+            cudaGetLastError();
+            flow.mem.release();
+            use_flow = false;
+        }
     }
     int blocks = 0, lanes = 1;
     cudaEvent_t e0, e1;
     cudaError_t le = cudaSuccess;
     if (use_flow) {
-        const FlowForm form = flow_natural_form(flow, N, sms);
         blocks = form.blocks;
-        for (int k = 0; k < 5; k++) FEEC_TRY(m.alloc(w[k], (size_t)N));
-        FEEC_TRY(m.alloc(part, (size_t)8 * blocks));
         FlowMoreArgs args{};
         args.n = N; args.nslices = flow.nslices; args.meta = flow.meta; args.ci = flow.ci; args.val = flow.val64;
         args.b = flow.own[0]; args.x = flow.own[1]; args.res = flow.own[2];
