@@ -157,7 +157,6 @@ __global__ void __launch_bounds__(MODE == kCgBarrier ? kCgBarrierThreads : kFlow
             // lanes: 4 FP64 operations instead of 10 (6 for two lanes per row)
             const int t = lane & ((1 << s0.shift) - 1);
             const bool row = (lane >> s0.shift) < s0.nrow;
-            int rest = 0;
             if (s0.shift >= 2) {
                 Acc k = AT::zero();
                 if (row && t < 4) k = acc_product(k, t == 1 ? d0 : t == 3 ? q0 : r0, t == 0 ? r0 : q0);
@@ -180,11 +179,10 @@ __global__ void __launch_bounds__(MODE == kCgBarrier ? kCgBarrierThreads : kFlow
                     sums[2] = acc_product(sums[2], r0, q0);
                     sums[3] = acc_product(sums[3], q0, q0);
                 }
-                rest = 1;
+                flow_warp_sums<T, 4>(sums, sh);
             }
-            const bool ok = rest ? flow_reduce<T, 4>(sums, a.partials + (K & 1) * 4 * gridDim.x, st, epoch, 92, live, sh, tot)
-                                 : flow_reduce_warps<4>(a.partials + (K & 1) * 4 * gridDim.x, st, epoch, 92, live, sh, tot);
-            if (!ok) return;
+            // one call for all warps: those of a block may have taken different branches above
+            if (!flow_reduce_warps<4>(a.partials + (K & 1) * 4 * gridDim.x, st, epoch, 92, live, sh, tot)) return;
         } else {
             // x += alpha d, r -= alpha q, d = r + beta d of the last iteration (:158-183)
             if constexpr (MODE == kCgPublished) {
