@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) flow_eisenstat(FlowArgs<T> a)
     });
     double tot[4];
     if (!flow_reduce<T, 4>(sums, a.partials + 4 * gridDim.x, st, epoch, 71, live, sh, tot)) return;
-    double z_r = tot[0], z_r_prev = tot[0], z_r_next = 0.0;   // thread 0 only
+    double z_r = tot[0], z_r_prev = tot[0];   // thread 0 only
     const double z_r0 = tot[0];
     int K = 0;
     if (threadIdx.x == 0) {
@@ -204,9 +204,8 @@ __global__ void __launch_bounds__(kFlowThreads, 1) flow_eisenstat(FlowArgs<T> a)
                 ctl = kSmallEnergy;
             }
             const double al = z_r / d_Ad;
-            z_r_next = fma(al, fma(al, tot[3], -2.0 * tot[2]), z_r);
             s_scal[0] = al;
-            s_scal[1] = z_r_next / z_r;
+            s_scal[1] = fma(al, fma(al, tot[3], -2.0 * tot[2]), z_r) / z_r;
             s_ctl = ctl;
         }
         __syncthreads();
@@ -221,19 +220,25 @@ __global__ void __launch_bounds__(kFlowThreads, 1) flow_eisenstat(FlowArgs<T> a)
             break;
         }
     }
+    double zr_last[1] = {0.0};
     if (step) {
+        Acc last[1] = {AT::zero()};
         const T alpha = (T)s_scal[0];
         T* const m_pub = a.pub[(K - 1) & 1];
         for (int j = 0; j < mine; j++) {
             const FlowSlice s = flow_slice(w.raw(j));
             const FlowRow row = flow_row(s, lane);
             if (row.own) {
+                const T ri = fma(-alpha, a.w[row.i], a.r[row.i]);
                 a.x[row.i] = fma(alpha, ld_flow(m_pub + row.i), a.x[row.i]);
-                a.r[row.i] = fma(-alpha, a.w[row.i], a.r[row.i]);
+                a.r[row.i] = ri;
+                last[0] = acc_product(last[0], T(ri * __ldg(&a.sd[row.i])), ri);
             }
         }
+        // the reported z.r is that of the final r, summed, not the expansion that beta is made of
+        if (!flow_reduce<T, 1>(last, a.partials + (K & 1) * 4 * gridDim.x, st, epoch, 75, live, sh, zr_last)) return;
     }
-    finish(st, status, K, step ? z_r_next : z_r, 0.0);
+    finish(st, status, K, step ? zr_last[0] : z_r, 0.0);
     if (blockIdx.x == 0 && threadIdx.x == 0) st->extra[0] = step ? z_r : z_r_prev;
 }
 

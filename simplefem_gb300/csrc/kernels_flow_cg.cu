@@ -7,7 +7,8 @@
 // (flow_device.cuh), and the sum that gives alpha also gives beta: with r.r, d.q, r.q and q.q
 // of the same r, alpha = r.r / d.q and r'.r' = r.r - 2 alpha r.q + alpha^2 q.q, the square of
 // r' = r - alpha q expanded. The next iteration sums r'.r' itself, for its alpha and for the
-// stopping rule, so the expansion's rounding (a few units of r.r in r'.r') only enters beta.
+// stopping rule, so the expansion's rounding (a few units of r.r in r'.r') only enters beta; a solve that ends
+// at the iteration cap sums its last residual once more for the reported norm.
 //
 // Rows are cut into slices as for the multicolor solvers, rows of equal length next to each
 // other (sorted within windows of kSortWindow, so that gathers stay local). When every warp
@@ -300,21 +301,32 @@ __global__ void __launch_bounds__(MODE == kCgBarrier ? kCgBarrierThreads : kFlow
         }
         if (K >= a.max_iter) { status = FEEC_MAXITER; break; }
     }
+    Acc last[1] = {AT::zero()};
     if constexpr (REG) {
-        if (row0.own) { a.x[row0.i] = x0; a.r[row0.i] = r0; }
+        if (row0.own) {
+            a.x[row0.i] = x0;
+            a.r[row0.i] = r0;
+            last[0] = acc_product(last[0], r0, r0);
+        }
     } else if (status == FEEC_MAXITER) {
         for (int j = 0; j < w.mine; j++) {
             const FlowSlice s = flow_slice(w.raw(j));
             const FlowRow row = flow_row(s, lane);
             if (row.own) {
                 const int i = row.i;
+                const T r = fma(-alpha, a.q[i], a.r[i]);
                 a.x[i] = fma(alpha, a.d[i], a.x[i]);
-                a.r[i] = fma(-alpha, a.q[i], a.r[i]);
+                a.r[i] = r;
+                last[0] = acc_product(last[0], r, r);
             }
         }
     }
-    const double rr_next = status == FEEC_MAXITER ? ctl.beta * tot[0] : tot[0];
-    finish(st, status, K, rr_next, tot[1]);
+    // at the cap no iteration follows that would sum the last residual: it is summed here
+    double rr[1] = {tot[0]};
+    if (status == FEEC_MAXITER &&
+        !flow_reduce<T, 1>(last, a.partials + (K & 1) * 4 * gridDim.x, st, epoch, 89, live, sh, rr))
+        return;
+    finish(st, status, K, rr[0], tot[1]);
     if (blockIdx.x == 0 && threadIdx.x == 0) st->extra[0] = tot[0];
 }
 

@@ -59,3 +59,58 @@ def test_cg_blocks_with_slices_of_different_shapes(long, short, per_row, mode):
     if mode == "reference":
         assert abs(info["iterations"] - K_o) <= max(1, int(np.ceil(0.02 * K_o))), (info, K_o)
     s.close()
+
+
+def _lattice(dim, r, L, n):
+    from simplefem_gb300 import workloads
+    A, C, V = workloads.lattice_matrix(dim, r, L, 3)
+    M = sp.csr_matrix((V, C, A))
+    return M[:n, :n].tocsr() if n else M
+
+
+# (operator, cap): the cap that the drop-ins default to (N) on systems that are exact there, and
+# one in the middle of a solve in each form of the kernels
+CAPPED = [("one_row", lambda: sp.csr_matrix([[3.7]]), 1), ("two_rows", lambda: _tridiagonal(2), 2),
+          ("identity_row", lambda: 0.3 * sp.identity(50, format="csr"), 1), ("three_rows", lambda: _tridiagonal(3), 3),
+          ("registers", lambda: _lattice(2, 1, 5, 0), 9), ("published", lambda: _lattice(3, 2, 4, 20_011), 5),
+          ("barrier", lambda: _lattice(3, 1, 6, 81_001), 5)]
+
+
+@pytest.mark.parametrize("method", ["cg", "rainbow_eisenstat", "rainbow"])
+@pytest.mark.parametrize("name,make,cap", CAPPED, ids=[c[0] for c in CAPPED])
+def test_capped_solve_reports_the_norm_of_its_residual(name, make, cap, method):
+    """final_norm of a solve that ends at the cap is the norm of the residual it returns: ||r|| for
+    plain CG, sqrt(z.r) with z = S r for Eisenstat's form, whose r is the one S scales (omega = 1:
+    S = D). A sum of n squares is off by at most a few units per addition in a chain, of which there
+    are far fewer than 1000 here: 1e-12. For the two-sweep form, whose z is not returned: that the
+    reported z.r is no more than that of an exact solve's rounding on the exact systems."""
+    import torch
+    from oracle import oracle
+    from simplefem_gb300.system import System
+    M = make()
+    A, C, V = _csr(M)
+    n = len(A) - 1
+    diag = oracle.csr_diagonal(A, C, V)
+    s = System(A, C, V)
+    if method != "cg":
+        s.set_rainbow(diag, 1.0, *oracle.rainbow(A, C))
+    for seed in range(12 if n < 100 else 1):
+        b = 1e3 * np.random.default_rng(seed).uniform(-1.0, 1.0, n)
+        x = torch.zeros(n, dtype=torch.float64, device="cuda")
+        r = torch.zeros(n, dtype=torch.float64, device="cuda")
+        info = s.solve(torch.from_numpy(b).cuda(), x, method=method, mode="reference", precision=1e-300, max_iter=cap,
+                       residual=r)
+        if info["status"] == 0:      # below the drop-ins' absolute floor already
+            continue
+        assert info["status"] == 3 and info["iterations"] == cap, info
+        rh = r.cpu().numpy()
+        if method == "cg":
+            norm = np.linalg.norm(rh)
+        elif method == "rainbow_eisenstat":
+            norm = np.sqrt(np.sum(diag * rh * rh))
+        else:
+            if cap >= n:
+                assert info["final_norm"] <= 1e-12 * np.sqrt(np.sum(b * b / diag)), info
+            continue
+        assert abs(info["final_norm"] - norm) <= 1e-12 * norm, (info, norm)
+    s.close()
