@@ -114,3 +114,36 @@ def test_capped_solve_reports_the_norm_of_its_residual(name, make, cap, method):
             continue
         assert abs(info["final_norm"] - norm) <= 1e-12 * norm, (info, norm)
     s.close()
+
+
+@pytest.mark.parametrize("n", [700, 200_003])
+def test_a_dense_row_is_set_up_in_linear_time(n):
+    """A dense first row and column: parts of more entries than are ordered at once. The first solve
+    of 200,003 rows, slices included, stays below a second and a half (its entries compared pair by
+    pair take several); the solution within 1e-9 of the oracle's and K within 2% (at least 1)."""
+    import time
+    import torch
+    from oracle import oracle
+    from simplefem_gb300.system import System
+    rest = np.arange(1, n)
+    rows = np.concatenate([np.zeros(n, int), rest, rest])
+    cols = np.concatenate([np.arange(n), np.zeros(n - 1, int), rest])
+    vals = np.concatenate([[3.0], np.full(n - 1, 0.5 / n), np.full(n - 1, 0.5 / n), np.linspace(1.0, 2.0, n - 1)])
+    M = sp.csr_matrix((vals, (rows, cols)), shape=(n, n))
+    A, C, V = _csr(M)
+    b = 1e3 * np.random.default_rng(n).uniform(-1.0, 1.0, n)
+    diag = oracle.csr_diagonal(A, C, V)
+    rb = oracle.rainbow(A, C)
+    K_o, x_o, _ = oracle.cg_rainbow(A, C, V, b, diag, rb, 1.0, precision=1e-11)
+    s = System(A, C, V)
+    s.set_rainbow(diag, 1.0, *rb)
+    bd, x = torch.from_numpy(b).cuda(), torch.zeros(n, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    t = time.perf_counter()
+    info = s.solve(bd, x, method="rainbow_eisenstat", mode="reference", precision=1e-11)
+    torch.cuda.synchronize()
+    t = time.perf_counter() - t
+    assert info["status"] == 0 and abs(info["iterations"] - K_o) <= max(1, int(np.ceil(0.02 * K_o))), (info, K_o)
+    assert np.linalg.norm(x.cpu().numpy() - x_o) <= 1e-9 * np.linalg.norm(x_o), info
+    assert t < 1.5, t
+    s.close()
