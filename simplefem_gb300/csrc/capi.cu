@@ -97,11 +97,12 @@ int ensure_work(feec_system* s) {
     FEEC_TRY(s->work.alloc(s->x32, n)); FEEC_TRY(s->work.alloc(s->r32, n)); FEEC_TRY(s->work.alloc(s->d32, n));
     FEEC_TRY(s->work.alloc(s->z32, n)); FEEC_TRY(s->work.alloc(s->m32, n)); FEEC_TRY(s->work.alloc(s->q32, n));
     FEEC_TRY(s->work.alloc(s->b32, n));
-    // partial sums: up to 3 doubles per block of the largest co-resident grid, plus residual blocks
+    // partial sums: 3 doubles per block of the barrier-phase kernels' largest grid (8 blocks per SM)
+    // or of the residual's, 8 per block of the dataflow solvers' (one block per SM)
     int dev_sms = 0;
     cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, s->dev);
     const size_t nblk = std::max<size_t>((size_t)dev_sms * 8, (size_t)residual_blocks(s->n, 32));
-    FEEC_TRY(s->work.alloc(s->partials, 3 * nblk + 64));
+    FEEC_TRY(s->work.alloc(s->partials, std::max<size_t>(3 * nblk + 64, kFlowPartials * (size_t)dev_sms)));
     FEEC_TRY(s->work.alloc(s->scal, 16));
     FEEC_TRY(s->work.alloc(s->st, 1));
     if (!s->ev0) FEEC_TRY(cudaEventCreate(&s->ev0));
@@ -845,7 +846,7 @@ int feec_system_set_launch(feec_system* s, int blocks, int lanes) {
 
 int feec_system_memory(const feec_system* s, size_t* bytes) {
     if (!s || !bytes) return FEEC_BADARG;
-    *bytes = s->mem.bytes + s->work.bytes + s->flow.mem.bytes + s->flow_cg.mem.bytes;
+    *bytes = s->mem.bytes + s->work.bytes + s->flow.mem.bytes + s->flow_cg.mem.bytes + small_bytes(s);
     return FEEC_OK;
 }
 

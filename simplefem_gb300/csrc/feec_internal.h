@@ -37,7 +37,7 @@ struct CgArgs {
     int max_iter;       // ... or after max_iter iterations
     int print_modulo;
     double print_tol;   // tolerance printed in interim lines
-    double* partials;   // >= 3 * gridDim.x doubles
+    double* partials;   // >= 3 * gridDim.x doubles (dataflow kernels: 8)
     DeviceStatus* st;
     // diagonal preconditioner (ConjugateGradientSolverCSR_DiagonalPreconditioner) when not
     // null: z = precon * r, rows with precon == 0 are skipped, the stop test is on z.r
@@ -71,7 +71,7 @@ struct PcgArgs {
     int max_iter;
     int print_modulo;
     double print_tol;
-    double* partials;    // >= 3 * gridDim.x doubles
+    double* partials;    // >= 3 * gridDim.x doubles (dataflow kernels: 8)
     DeviceStatus* st;
     // Eisenstat variants only
     const T* dg;         // the diagonal D, permuted like the rows

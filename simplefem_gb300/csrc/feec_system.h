@@ -149,6 +149,8 @@ struct feec_system {
 };
 
 namespace feec {
+// Doubles of partial sums per block of a dataflow solver (two sets of four).
+constexpr size_t kFlowPartials = 8;
 // Dataflow solvers over the Rainbow layout (kernels_flow.cu): flow_build prepares the slices
 // and values of one precision; the launchers enqueue one solve. feec_status results.
 int flow_build(feec_system* s, bool f32);
@@ -163,6 +165,7 @@ bool small_pcg_fits(const feec_system* s);
 int small_pcg_prepare(feec_system* s);
 int launch_small_pcg(feec_system* s, const PcgArgs<double>& a, LaunchShape& shape);
 void small_release(feec_system* s);
+size_t small_bytes(const feec_system* s);
 // Natural-order slices of a matrix (kernels_flow_cg.cu), and the form that a solver over them runs
 // in: every vector in registers, vectors in memory with the gathered one published, or (neither) too
 // large for publishing to pay.

@@ -459,7 +459,7 @@ int more_dropin(int kind, int N, double* x, const double* b, const int* A, const
         if (ok) {
             form = flow_natural_form(flow, N, sms);
             for (int k = 0; k < 5 && ok; k++) ok = flow.mem.alloc(w[k], (size_t)N) == cudaSuccess;
-            ok = ok && flow.mem.alloc(part, (size_t)8 * form.blocks) == cudaSuccess;
+            ok = ok && flow.mem.alloc(part, kFlowPartials * form.blocks) == cudaSuccess;
         }
         if (!ok) {
             cudaGetLastError();

@@ -536,6 +536,8 @@ void small_release(feec_system* s) {
     s->small = nullptr;
 }
 
+size_t small_bytes(const feec_system* s) { return s->small ? s->small->mem.bytes : 0; }
+
 bool small_pcg_fits(const feec_system* s) {
     if (s->n >= 0xffff || ring_room(s->n) < 8) return false;
     return s->prepared == FEEC_METHOD_SSOR || (s->prepared == FEEC_METHOD_RAINBOW && s->n <= kSmallColorRows);

@@ -147,3 +147,27 @@ def test_a_dense_row_is_set_up_in_linear_time(n):
     assert np.linalg.norm(x.cpu().numpy() - x_o) <= 1e-9 * np.linalg.norm(x_o), info
     assert t < 1.5, t
     s.close()
+
+
+@pytest.mark.parametrize("method", ["ssor", "rainbow"])
+def test_memory_counts_the_one_block_solvers_tables(method):
+    """The first solve of a small system lays out full rows (12 bytes an entry) and staged sweep
+    slices: memory_bytes grows by at least the former."""
+    import torch
+    from oracle import oracle
+    from simplefem_gb300.system import System
+    A, C, V = _csr(_lattice(2, 1, 6, 0))
+    n = len(A) - 1
+    diag = oracle.csr_diagonal(A, C, V)
+    s = System(A, C, V)
+    if method == "ssor":
+        s.set_ssor(diag, 1.0)
+    else:
+        s.set_rainbow(diag, 1.0, *oracle.rainbow(A, C))
+    x = torch.zeros(n, dtype=torch.float64, device="cuda")
+    b = torch.ones_like(x)
+    s.solve(b, x, method="cg", mode="reference", precision=1e-6)      # the work vectors
+    before = s.memory_bytes()
+    s.solve(b, x, method=method, mode="reference", precision=1e-6)
+    assert s.memory_bytes() >= before + 12 * len(C)
+    s.close()
