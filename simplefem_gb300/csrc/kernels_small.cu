@@ -14,9 +14,10 @@
 // FP64 units instead (19 cycles per warp instruction).
 //
 // The block leaves the other SMs free: small solves on several streams run side by side, which
-// a grid-wide (cooperative) solve does not allow. Index-order systems come here up to about
-// 12,000 rows (their two vectors and the staging ring fill the shared memory; 16 blocks took 750 us
-// per iteration on 4,225 rows); multicolor ones up to kSmallColorRows, beyond which
+// a grid-wide (cooperative) solve does not allow. Index-order systems come here up to
+// 13,569 rows, where their two vectors leave a ring of eight slices (us per iteration here and in
+// pcg_persistent: 2D P1, 9,000 rows 156 / 495, 12,000 rows 182 / 900, 13,569 rows 285 / 972; 3D P2, 9,000
+// rows 515 / 808, 13,500 rows 657 / 1224); multicolor ones up to kSmallColorRows, beyond which
 // the dataflow solver takes them (alone on the GPU it is the faster one here too: 18 us).
 //
 // Measured per iteration, 2D P1 refined 6 times (4,225 rows): index order 228 us (one warp walking
@@ -41,6 +42,7 @@ constexpr int kSmallThreads = 512;
 constexpr int kSmallWarps = kSmallThreads / 32;
 constexpr int kSweepEntries = 4;    // entries of a row part per lane and chunk
 constexpr int kMaxSweepDepth = 8;   // phases staged ahead (at least 3)
+constexpr int kMaxPadding = 4;      // staged slices to slices with rows, at most
 
 // What a warp needs for its slice of a phase: per lane 4 columns, 4 values times the row's factor
 // omega / D, and the row (n, the slot past the vector, where the lane has none). Rows are
@@ -57,9 +59,10 @@ static_assert(sizeof(SweepSlice) % 16 == 0, "one bulk copy");
 
 // One sweep, phase by phase (dependency levels or colors), 1 << shift lanes per row. Phase p has
 // the `width` slices from width * p (some possibly without rows), staged as one copy; phases
-// wider than that go on in slices [extra[p], extra[p + 1]).
+// wider than that go on in slices [extra[p], extra[p + 1]), which their warps read from memory.
+// `empty` is a slice without rows.
 struct SweepView {
-    int nph, shift, warps, width, depth;
+    int nph, shift, warps, width, depth, empty;
     int count;                       // most entries per lane; rows of one lane and one chunk: plain
     bool plain;
     const SweepSlice* slices; const int* extra;
@@ -169,7 +172,10 @@ __device__ __forceinline__ void sweep_barrier(int warps) {
 // each phase; entries requested into registers phases ahead did not shorten the phases: a warp
 // has six scoreboards for its loads and waits for the youngest load on one.) `phase` holds
 // the parity of each slot's barrier. False when a copy never landed.
-template <int COUNT, bool PLAIN>
+// FAR: more warps than slices in a slot; warp `width` and those after it read their first slice of a
+// phase from memory, a phase ahead. A kernel of its own: in one kernel with the others it slows
+// their phases by 3 - 13 %.
+template <int COUNT, bool PLAIN, bool FAR = false>
 __device__ __forceinline__ bool sweep_as(const SweepView& s, double* x, SweepSlice* ring, unsigned long long* bars,
                                       unsigned& phase, DeviceStatus* st) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -201,22 +207,34 @@ __device__ __forceinline__ bool sweep_as(const SweepView& s, double* x, SweepSli
         return ok;
     }
     sweep_barrier(s.warps + 1);
+    const bool staged = !FAR || warp < s.width;
+    auto beyond = [&](int p) {
+        if (p >= s.nph) return s.empty;
+        const int at = __ldg(&s.extra[p]) + warp - s.width;
+        return at < __ldg(&s.extra[p + 1]) ? at : s.empty;
+    };
     SweepEntries even, odd;
     const SweepSlice* here = ring + warp;
-    read_slice(even, *here, lane);
+    int far = 0;                             // not staged: the warp's slice of the next phase
+    if (staged) read_slice(even, *here, lane);
+    else { read_slice(even, s.slices[beyond(0)], lane); far = beyond(1); }
     int slot = 0;
     auto step = [&](int p, const SweepEntries& e, SweepEntries& next) {
         slot = slot + 1 == s.depth ? 0 : slot + 1;
         const SweepSlice* ahead = ring + slot * s.width + warp;
-        sweep_slice<COUNT, PLAIN>(e, s, x, lane, [&] { if (p + 1 < s.nph) read_slice(next, *ahead, lane); });
-        if (s.width > s.warps)
+        sweep_slice<COUNT, PLAIN>(e, s, x, lane, [&] {
+            if (p + 1 >= s.nph) return;
+            if (staged) read_slice(next, *ahead, lane);
+            else { read_slice(next, s.slices[far], lane); far = beyond(p + 2); }
+        });
+        if (!FAR && s.width > s.warps)
             for (int k = s.warps; warp + k < s.width; k += s.warps) {
                 SweepEntries f;
                 read_slice(f, here[k], lane);
                 sweep_slice<COUNT, PLAIN>(f, s, x, lane, [] {});
             }
         if (s.extra)
-            for (int sl = __ldg(&s.extra[p]) + warp; sl < __ldg(&s.extra[p + 1]); sl += s.warps) {
+            for (int sl = __ldg(&s.extra[p]) + warp + (FAR ? s.warps - s.width : 0); sl < __ldg(&s.extra[p + 1]); sl += s.warps) {
                 SweepEntries f;
                 read_slice(f, s.slices[sl], lane);
                 sweep_slice<COUNT, PLAIN>(f, s, x, lane, [] {});
@@ -231,8 +249,13 @@ __device__ __forceinline__ bool sweep_as(const SweepView& s, double* x, SweepSli
     return true;
 }
 
+template <bool FAR>
 __device__ __forceinline__ bool sweep(const SweepView& s, double* x, SweepSlice* ring, unsigned long long* bars,
                                       unsigned& phase, DeviceStatus* st) {
+    if constexpr (FAR) {
+        if (s.warps > s.width) return sweep_as<kSweepEntries, false, true>(s, x, ring, bars, phase, st);
+        return sweep_as<kSweepEntries, false>(s, x, ring, bars, phase, st);
+    }
     if (!s.plain) return sweep_as<kSweepEntries, false>(s, x, ring, bars, phase, st);
     if (s.count <= 2) return sweep_as<2, true>(s, x, ring, bars, phase, st);
     if (s.count == 3) return sweep_as<3, true>(s, x, ring, bars, phase, st);
@@ -289,6 +312,7 @@ __device__ __forceinline__ double small_minus(const SmallArgs& a, long long off,
     return acc;
 }
 
+template <bool FAR>
 __global__ void __launch_bounds__(kSmallThreads, 1) small_pcg(SmallArgs a) {
     extern __shared__ __align__(16) double smem[];
     const int n = a.n;
@@ -324,13 +348,13 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_pcg(SmallArgs a) {
     // m = (D/w + L)^-1 r, z = (D/w + U)^-1 S m (:528-575, :647-699 / :1118-1170, :1241-1307), in su;
     // returns z.r (warp 0)
     auto precondition = [&]() {
-        ok = sweep(a.fwd, su, ring, s_bar, phase, a.st) && ok;
+        ok = sweep<FAR>(a.fwd, su, ring, s_bar, phase, a.st) && ok;
         __syncthreads();
         if (a.scale != 1.0) {
             for (int i = threadIdx.x; i < n; i += kSmallThreads) su[i] *= a.scale;
             __syncthreads();
         }
-        ok = sweep(a.bwd, su, ring, s_bar, phase, a.st) && ok;
+        ok = sweep<FAR>(a.bwd, su, ring, s_bar, phase, a.st) && ok;
         __syncthreads();
         double zr = 0.0;
         for (int i = threadIdx.x; i < n; i += kSmallThreads)
@@ -431,7 +455,7 @@ struct SweepHost {
     std::vector<int> extra, mc;
     std::vector<double> mv;
     std::vector<SweepSlice> slices;
-    int shift = 0, warps = 1, width = 1, depth = 3, count = 0;
+    int shift = 0, warps = 1, width = 1, depth = 3, empty = 0, count = 0;
     bool plain = true;
 };
 
@@ -447,10 +471,31 @@ bool build_sweep(SweepHost& h, int nph, const int* pptr, const int* list, const 
     while (!wide && h.shift < 5 && entries > (long long)rows * (kSweepEntries << h.shift)) h.shift++;
     const int width = 1 << h.shift, per = 32 >> h.shift;
     int widest = 1;
-    for (int p = 0; p < nph; p++) widest = std::max(widest, (pptr[p + 1] - pptr[p] + per - 1) / per);
-    // the widest phase in a slot, or as much of it as three slots leave room for
+    long long real = 0;
+    for (int p = 0; p < nph; p++) {
+        const int c = (pptr[p + 1] - pptr[p] + per - 1) / per;
+        widest = std::max(widest, c);
+        real += std::max(c, 1);
+    }
+    // A warp for each slice of the widest phase, and that phase in a slot, or as much of it as three
+    // slots leave room for; warps without a slice in the slot only where they are more than half
+    // (us per iteration with and without them: 3D P1, 13,000 rows 261 / 340, 13,500 rows 277 / 550; 3D P2,
+    // 13,500 rows 658 / 1418; but 3D P1, 11,000 rows 239 / 221; 2D P1, 13,300 rows 276 / 247, 13,569 rows
+    // 294 / 286). Where few phases are that wide (a slot each would be mostly
+    // empty: the slices of 3,000 levels of one row beside one of 1,500 rows took 196 MB, and their
+    // copies 0.99 us a phase), as many warps as keep the rounds of the wide ones to an eighth of
+    // the phases.
+    h.warps = std::min(widest, kSmallWarps - 1);
     h.width = std::max(1, std::min(widest, room / 3));
-    h.warps = std::min(h.width, kSmallWarps - 1);
+    if (2 * h.width >= h.warps) h.warps = std::min(h.width, h.warps);
+    if ((long long)nph * h.width > kMaxPadding * real) {
+        for (h.warps = 1; h.warps < std::min(widest, kSmallWarps - 1); h.warps++) {
+            long long more = 0;
+            for (int p = 0; p < nph; p++) more += std::max(0, (pptr[p + 1] - pptr[p] + per * h.warps - 1) / (per * h.warps) - 1);
+            if (8 * more <= nph) break;
+        }
+        h.width = std::max(1, std::min(h.width, std::min(h.warps, (int)(kMaxPadding * real / nph))));
+    }
     h.depth = std::max(3, std::min(kMaxSweepDepth, room / h.width));
     std::vector<SweepSlice> more;
     bool any = false;
@@ -494,6 +539,11 @@ bool build_sweep(SweepHost& h, int nph, const int* pptr, const int* list, const 
     }
     h.slices.insert(h.slices.end(), more.begin(), more.end());
     if (!any) h.extra.clear();
+    SweepSlice none;
+    std::memset(&none, 0, sizeof(none));
+    for (int l = 0; l < 32; l++) none.row[l] = (unsigned short)n;
+    h.empty = (int)h.slices.size();
+    h.slices.push_back(none);
     if (h.shift > 0) h.plain = false;
     return true;
 }
@@ -511,7 +561,7 @@ int upload_sweep(DevArena& m, cudaStream_t st, const SweepHost& h, int nph, Swee
         FEEC_TRY(cudaMemcpyAsync(extra, h.extra.data(), 4 * h.extra.size(), cudaMemcpyHostToDevice, st));
     }
     FEEC_TRY(cudaStreamSynchronize(st));   // the host arrays leave scope
-    v.nph = nph; v.shift = h.shift; v.warps = h.warps; v.width = h.width; v.depth = h.depth; v.count = h.count; v.plain = h.plain;
+    v.nph = nph; v.shift = h.shift; v.warps = h.warps; v.width = h.width; v.depth = h.depth; v.empty = h.empty; v.count = h.count; v.plain = h.plain;
     v.slices = slices; v.extra = extra; v.mc = mc; v.mv = mv;
     return FEEC_OK;
 }
@@ -618,8 +668,9 @@ int launch_small_pcg(feec_system* s, const PcgArgs<double>& p, LaunchShape& shap
     shape.threads = kSmallThreads;
     shape.lanes = 1 << a.fwd.shift;
     note_launch();
-    FEEC_TRY(cudaFuncSetAttribute(small_pcg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    small_pcg<<<1, kSmallThreads, bytes, s->stream>>>(a);
+    const auto kernel = a.fwd.warps > a.fwd.width || a.bwd.warps > a.bwd.width ? small_pcg<true> : small_pcg<false>;
+    FEEC_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    kernel<<<1, kSmallThreads, bytes, s->stream>>>(a);
     return cuda_status(cudaGetLastError());
 }
 

@@ -171,3 +171,47 @@ def test_memory_counts_the_one_block_solvers_tables(method):
     s.solve(b, x, method=method, mode="reference", precision=1e-6)
     assert s.memory_bytes() >= before + 12 * len(C)
     s.close()
+
+
+def _chain_and_rows(chain, rows):
+    """Levels of one row each (a chain) beside one level of many rows."""
+    return sp.block_diag([_tridiagonal(chain), sp.diags(np.linspace(1.0, 2.0, rows))]).tocsr()
+
+
+LEVELS = [("chain_3000_and_1500", lambda: _chain_and_rows(3000, 1500)), ("chain_8000_and_600", lambda: _chain_and_rows(8000, 600)),
+          ("chain_9001", lambda: _chain_and_rows(9000, 1)), ("p1_2d_12700", lambda: _lattice(2, 1, 7, 12_700)),
+          ("p1_2d_last_in_one_block", lambda: _lattice(2, 1, 7, 13_569)), ("p1_2d_first_beyond", lambda: _lattice(2, 1, 7, 13_570)),
+          ("p2_3d_13500", lambda: _lattice(3, 2, 4, 13_500)), ("p1_3d_13000", lambda: _lattice(3, 1, 5, 13_000))]
+
+
+@pytest.mark.parametrize("name,make", LEVELS, ids=[c[0] for c in LEVELS])
+def test_index_order_schedules_of_uneven_levels(name, make):
+    """Index-order SSOR where the staged slots cannot hold the widest level: a wide level among
+    levels of one row, and systems up to the last that fits a block (vectors that leave room for two
+    slices a slot). K within 2% (at least 1) of the oracle, the solution within 1e-9 of it; the
+    tables stay a small multiple of the matrix: a slot's slices hold 32 rows in 1,360 bytes, at most
+    four are staged for one that holds rows, over two sweeps, beside 12 bytes per entry, columns of
+    32 of them padded to the longest of 32 rows (six times the entries here at most)."""
+    import torch
+    from oracle import oracle
+    from simplefem_gb300.system import System
+    M = make()
+    A, C, V = _csr(M)
+    n = len(A) - 1
+    b = 1e3 * np.random.default_rng(n).uniform(-1.0, 1.0, n)
+    diag = oracle.csr_diagonal(A, C, V)
+    K_o, x_o, _ = oracle.cg_ssor(A, C, V, b, diag, 1.0, precision=1e-10)
+    s = System(A, C, V)
+    s.set_ssor(diag, 1.0)
+    x = torch.zeros(n, dtype=torch.float64, device="cuda")
+    bd = torch.from_numpy(b).cuda()
+    s.solve(bd, x, method="cg", mode="reference", precision=1e-2)
+    before = s.memory_bytes()
+    x.zero_()
+    info = s.solve(bd, x, method="ssor", mode="reference", precision=1e-10)
+    assert info["status"] == 0, info
+    assert abs(info["iterations"] - K_o) <= max(1, int(np.ceil(0.02 * K_o))), (info, K_o)
+    assert np.linalg.norm(x.cpu().numpy() - x_o) <= 1e-9 * np.linalg.norm(x_o), info
+    if name.startswith("chain"):
+        assert s.memory_bytes() - before <= 2 * 4 * 1360 * (n // 32 + n) + 6 * 12 * len(C)
+    s.close()
