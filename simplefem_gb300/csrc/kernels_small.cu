@@ -13,8 +13,8 @@
 // products. Colors (multicolor schedules) hold hundreds of rows and are bound by the one SM's
 // FP64 units instead (19 cycles per warp instruction).
 //
-// The block leaves the other SMs free: small solves on several streams run side by side, which
-// a grid-wide (cooperative) solve does not allow. Index-order systems come here up to
+// The block leaves the other SMs free: small solves on several streams run side by side.
+// Index-order systems come here up to
 // 13,569 rows, where their two vectors leave a ring of eight slices (us per iteration here and in
 // pcg_persistent: 2D P1, 9,000 rows 156 / 495, 12,000 rows 182 / 900, 13,569 rows 285 / 972; 3D P2, 9,000
 // rows 515 / 808, 13,500 rows 657 / 1224); multicolor ones up to kSmallColorRows, beyond which

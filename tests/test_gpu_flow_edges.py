@@ -215,3 +215,67 @@ def test_index_order_schedules_of_uneven_levels(name, make):
     if name.startswith("chain"):
         assert s.memory_bytes() - before <= 2 * 4 * 1360 * (n // 32 + n) + 6 * 12 * len(C)
     s.close()
+
+
+@pytest.mark.parametrize("method,mode", [("rainbow", "fp64"), ("rainbow", "mixed"), ("rainbow_eisenstat", "reference"),
+                                         ("cg", "fp64")])
+def test_small_solves_on_several_streams_share_the_gpu(method, mode):
+    """Eight threads with a stream and a system of 4,225 rows each: the results are those of a solve
+    alone, bit for bit, and together they take less than half of the time of one after the other
+    (they fit the SMs side by side)."""
+    import threading
+    import time
+    import torch
+    from oracle import oracle
+    from simplefem_gb300.system import System
+    A, C, V = _csr(_lattice(2, 1, 6, 0))
+    n = len(A) - 1
+    diag, rb = oracle.csr_diagonal(A, C, V), oracle.rainbow(A, C)
+    T, reps = 8, 6
+    b = torch.from_numpy(1e3 * np.random.default_rng(3).uniform(-1.0, 1.0, n)).cuda()
+    systems, xs = [], []
+    for _ in range(T):
+        s = System(A, C, V)
+        s.set_rainbow(diag, 1.0, *rb)
+        systems.append(s)
+        xs.append(torch.zeros_like(b))
+    streams = [torch.cuda.Stream() for _ in range(T)]
+
+    def solve(i):
+        with torch.cuda.stream(streams[i]):
+            xs[i].zero_()
+            systems[i].solve(b, xs[i], method=method, mode=mode, precision=1e-10)
+
+    torch.cuda.synchronize()
+    for _ in range(3):          # layouts and, for mixed, the choice of the inner precision
+        for i in range(T):
+            solve(i)
+    alone = [x.cpu().numpy().tobytes() for x in xs]
+    t = time.perf_counter()
+    for _ in range(reps):
+        for i in range(T):
+            solve(i)
+    torch.cuda.synchronize()
+    serial = time.perf_counter() - t
+    gate = threading.Barrier(T + 1)
+
+    def worker(i):
+        gate.wait()
+        for _ in range(reps):
+            solve(i)
+        gate.wait()
+
+    threads = [threading.Thread(target=worker, args=(i,)) for i in range(T)]
+    for th in threads:
+        th.start()
+    gate.wait()
+    t = time.perf_counter()
+    gate.wait()
+    together = time.perf_counter() - t
+    for th in threads:
+        th.join()
+    torch.cuda.synchronize()
+    assert [x.cpu().numpy().tobytes() for x in xs] == alone
+    assert together < 0.5 * serial, (together, serial)
+    for s in systems:
+        s.close()
