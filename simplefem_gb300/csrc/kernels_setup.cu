@@ -384,12 +384,16 @@ __device__ __forceinline__ double sell_row(const int* __restrict__ ci, const dou
 
 // FP64 SELL-32 SpMV, one thread per row, co-limited by HBM and by the FP64 rate (19 - 20 cycles of
 // an SM per warp instruction: 15 of them per 32 rows of 3D P1 take 63 us of the 71 on 2,146,689
-// rows). A chunk's unused slots take FP64 time as well, so the chunk is 7 for slices of 7 entries
-// (2D P1) and else 5, which 15 (3D P1) fills and 27 and 65 (3D P2) nearly do; slices longer than
-// kSellLong waste little either way and take 8 for the loads in flight. Against chunks of 8 for
+// rows). A chunk's unused slots take FP64 time as well, so the chunk is 7 for slices of 6 and 7
+// entries (2D P1), 8 for those that it fills, and else 5, which 15 (3D P1) fills and 27 and 65 (3D P2)
+// nearly do; slices longer than kSellLong waste little either way and take 8 for the loads in
+// flight. (An unused slot also reads x[0], times 0: rows of whole chunks never do.) Against chunks of 8 for
 // all (same sums in the same order), us per product, back to back: 3D P1 refined 7 times 74.1 ->
 // 71.9, 6 times 14.3 -> 12.8; 3D P2 refined 5 times 34.6 -> 32.0; 2D P1 refined 10 times 26.6 -> 22.7;
-// 3D P3 refined 4 times 30.7 both (31.4 with chunks of 5).
+// 3D P3 refined 4 times 30.7 both (31.4 with chunks of 5). Rows of one length, 20 M entries or 400,000
+// rows, 8 / 5 / this: 6 entries 13.2 / 14.3 / 12.1, 8 entries 13.3 / 14.4 / 13.2, 16 entries 20.8 /
+// 22.8 / 20.7, 25 entries 32.8 / 27.1 / 27.1, 32 entries 32.0 / 33.3 / 32.8, 50 entries 51.4 / 46.0 / 46.1,
+// 56 entries 45.2 / 47.2 / 45.5; 31 entries 32.4 / 33.6 / 33.4, the worst for it.
 constexpr int kSellLong = 65;
 __global__ void __launch_bounds__(256) sell_spmv_f64_kernel(SellView v, const double* __restrict__ x, double* __restrict__ y,
                                                             double scaling) {
@@ -405,8 +409,8 @@ __global__ void __launch_bounds__(256) sell_spmv_f64_kernel(SellView v, const do
         const int* ci = v.ci + off;
         const double* val = v.val64 + off;
         double s;
-        if (L == 7) s = sell_row<7>(ci, val, L, x);
-        else if (L <= kSellLong) s = sell_row<5>(ci, val, L, x);
+        if (L == 7 || L == 6) s = sell_row<7>(ci, val, L, x);
+        else if (L <= kSellLong && (L & 7) != 0) s = sell_row<5>(ci, val, L, x);
         else s = sell_row<8>(ci, val, L, x);
         // FP64 issues at 2 lanes/clk/SM on this part: skip the multiply when scaling == 1
         if (lane < nrow) y[row0 + lane] = scaling == 1.0 ? s : scaling * s;

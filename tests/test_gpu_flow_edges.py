@@ -279,3 +279,25 @@ def test_small_solves_on_several_streams_share_the_gpu(method, mode):
     assert together < 0.5 * serial, (together, serial)
     for s in systems:
         s.close()
+
+
+@pytest.mark.parametrize("length", [8, 16, 40, 64, 72])
+def test_product_reads_no_entry_that_a_row_does_not_have(cuda, length):
+    """Rows of whole chunks of eight entries that do not touch unknown 0 are finite when x is infinite
+    there. A row of k entries is off by at most k units of rounding of its sum of magnitudes."""
+    import torch
+    from simplefem_gb300.system import System
+    n = 32 * 6 + 5
+    rng = np.random.default_rng(length)
+    A = (np.arange(n + 1) * length).astype(np.int32)
+    C = np.concatenate([np.sort(1 + rng.choice(n - 1, length, replace=False)) for _ in range(n)]).astype(np.int32)
+    V = rng.standard_normal(len(C))
+    x = rng.standard_normal(n)
+    M = sp.csr_matrix((V, C, A), shape=(n, n))
+    exact, bound = M @ x, length * np.finfo(np.float64).eps * (abs(M) @ np.abs(x))
+    x[0] = np.inf
+    s = System(A, C, V)
+    y = torch.full((n,), np.nan, dtype=torch.float64, device="cuda")
+    s.apply(torch.from_numpy(x).cuda(), y)
+    assert (np.abs(y.cpu().numpy() - exact) <= bound).all()
+    s.close()
