@@ -722,6 +722,7 @@ int build_layout(feec_system* s, int method, const double* diag_dev, double omeg
     }
     FEEC_TRY(cudaStreamSynchronize(st));
     s->nf = (int)fptr.size() - 1;
+    s->color_ranges = method == FEEC_METHOD_RAINBOW ? fptr : std::vector<int>();
     s->nbw = (int)bptr.size() - 1;
     s->max_phase_rows = 0;
     for (size_t p = 0; p + 1 < fptr.size(); p++) s->max_phase_rows = std::max(s->max_phase_rows, fptr[p + 1] - fptr[p]);

@@ -80,14 +80,13 @@ struct FlowData {
     double* own[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
 };
 
-struct FlowHostSlice {
-    int row0, nrow, shift, len;          // len: entries per lane
-};
-// Cuts rows [lo, hi) with len[i] entries into slices of at most `longest` entries per lane (up to
-// 32 lanes per row), lanes per row by the modelled time of one pass over them; false (out empty)
-// when every choice needs more than max_slices (kernels_flow.cu).
-bool flow_cut_rows(int lo, int hi, const int* len, int row_ops, int sms, int longest, int max_slices,
-                   std::vector<FlowHostSlice>& out);
+// Slices (kernels_slices.cu): the rows of colors ranges[c] .. ranges[c + 1] of a split layout, or a
+// matrix's rows sorted by length within windows of kSortWindow (perm, iperm). They set D's slices,
+// units and longest part; scratch and tables are allocated on st.
+constexpr int kSortWindow = 2048;
+int cut_colors(FlowData& D, cudaStream_t st, int sms, const std::vector<int>& ranges, const int* rp, const int* lsplit,
+               const int* usplit);
+int cut_natural(FlowData& D, cudaStream_t st, int sms, int n, const int* rp);
 
 struct SmallData;   // one-block solver's slices and sweep schedules (kernels_small.cu)
 
@@ -140,6 +139,7 @@ struct feec_system {
     // SELL-32 layouts: [0] natural row order (SpMV, batched plain CG), [1] Rainbow order
     feec::SellData sell[2];
     feec::FlowData flow;               // multicolor layout
+    std::vector<int> color_ranges;     // rows of each color, host copy of fptr (multicolor layouts)
     feec::FlowData flow_cg;            // natural layout, plain CG
     // batched-engine launch choice made by the autotuner, per [method][mode] (0 = not tuned)
     int tuned_k[3][3] = {};
@@ -174,8 +174,7 @@ struct FlowForm {
     int blocks, threads;
     bool registers, published;
 };
-int flow_natural_build(FlowData& D, cudaStream_t st, int dev, int n, const int* rowptr, const int* A, const int* C,
-                       const double* V, bool f32);
+int flow_natural_build(FlowData& D, cudaStream_t st, int dev, int n, const int* A, const int* C, const double* V, bool f32);
 FlowForm flow_natural_form(const FlowData& D, int n, int sms);
 cudaError_t flow_permute(int n, const int* perm, const double* src, double* dst, bool back, cudaStream_t st);
 // Plain CG (kernels_flow_cg.cu).

@@ -13,7 +13,7 @@
 // it is known and its readers wait for that value alone (flow_device.cuh), so phases
 // overlap wherever the matrix lets them; the entries of a slice and the row's own values
 // are requested before the wait; and rows take one lane each unless that leaves
-// schedulers idle (flow_build chooses lanes per slice). The only grid-wide barriers left
+// schedulers idle (kernels_slices.cu chooses lanes per slice). The only grid-wide barriers left
 // are the sums: one per iteration (Eisenstat) and two (PCG).
 //
 // Row slices: every slice belongs to one warp, the same in both sweeps, so a row's own
@@ -431,58 +431,6 @@ __global__ void flow_fill_kernel(int nslices, const int4* __restrict__ meta, con
     }
 }
 
-// Lanes per row of each slice. A warp's FP64 instruction holds its scheduler 64 cycles and
-// the SM's FP64 units 19 (measured), and a chunk of kFlowChunk entries takes a trip to L2 of
-// about 500. With p entries per lane a phase therefore lasts at least as long as its
-// slowest slice, 64 (p + log2 lanes + 1) + 500 per chunk, and at least 19 cycles per
-// instruction of its slices over the SMs: few entries per lane shorten the chain, many lanes
-// per row issue the row's other ~12 operations for fewer rows at once. Each phase takes the
-// bound on p with the smallest sum over the two sweeps of the larger of the two. (3D P2: one
-// lane for the first seven colors, four to eight for the 65-entry rows after them. FP32 was
-// fastest on the same slices: with at most 8 entries per lane everywhere 67 us per iteration
-// on 3D P2 refined 5 times against 55.)
-constexpr int kRowOps = 12;
-
-struct HostSlice {
-    int row0, nrow, shift, l, e, u;
-};
-
-int part_per_lane(int entries, int shift) { return (entries + (1 << shift) - 1) >> shift; }
-
-// Slices of rows [lo, hi) with at most `most` entries per lane and part (32 lanes at most);
-// returns the modelled cycles.
-double slice_rows(int lo, int hi, const int* rp, const int* ls, const int* us, int most, int sms,
-                  std::vector<HostSlice>* out) {
-    double chain[2] = {0.0, 0.0}, ops[2] = {0.0, 0.0};
-    for (int i = lo; i < hi;) {
-        auto need = [&](int k) {
-            const int longest = std::max(ls[k] - rp[k], rp[k + 1] - us[k]);
-            int sh = 0;
-            while (sh < 5 && part_per_lane(longest, sh) > most) sh++;
-            return sh;
-        };
-        const int shift = need(i);
-        HostSlice s{i, 0, shift, 0, 0, 0};
-        while (i < hi && s.nrow < (32 >> shift) && need(i) <= shift) {
-            s.l = std::max(s.l, part_per_lane(ls[i] - rp[i], shift));
-            s.e = std::max(s.e, part_per_lane(us[i] - ls[i], shift));
-            s.u = std::max(s.u, part_per_lane(rp[i + 1] - us[i], shift));
-            s.nrow++;
-            i++;
-        }
-        const int part[2] = {s.l, s.u};
-        for (int w = 0; w < 2; w++) {
-            const int chunks = (part[w] + kFlowChunk - 1) / kFlowChunk;
-            chain[w] = std::max(chain[w], 64.0 * (part[w] + shift + 1) + 500.0 * chunks);
-            ops[w] += part[w] + shift + kRowOps;
-        }
-        if (out) out->push_back(s);
-    }
-    double cost = 0.0;
-    for (int w = 0; w < 2; w++) cost += std::max(chain[w], 19.0 * ops[w] / sms);
-    return cost;
-}
-
 }  // namespace
 
 cudaError_t flow_fill(int nslices, const int4* meta, const int* rp, const int* lsplit, const int* usplit, const int* ci_in,
@@ -491,45 +439,6 @@ cudaError_t flow_fill(int nslices, const int4* meta, const int* rp, const int* l
     note_launch();
     flow_fill_kernel<<<(nslices + 7) / 8, 256, 0, st>>>(nslices, meta, rp, lsplit, usplit, ci_in, val_in, ci, val64, val32);
     return cudaGetLastError();
-}
-
-bool flow_cut_rows(int lo, int hi, const int* len, int row_ops, int sms, int longest, int max_slices,
-                   std::vector<FlowHostSlice>& out) {
-    auto lanes = [](int entries, int most) {
-        int shift = 0;
-        while (shift < 5 && part_per_lane(entries, shift) > most) shift++;
-        return shift;
-    };
-    int best = 0;
-    double cost = -1.0;
-    if (hi - lo > 32 * 64 * sms) {
-        best = longest;      // many rows: few lanes each, without weighing the alternatives row by row
-    } else {
-        for (int most : {1, 2, 4, 8, 16, 32}) {
-            if (most > longest) break;
-            double chain = 0.0, ops = 0.0;
-            int slices = 0;
-            for (int i = lo; i < hi; slices++) {
-                const int shift = lanes(len[i], most);
-                const int p = part_per_lane(len[i], shift), chunks = (p + kFlowChunk - 1) / kFlowChunk;
-                chain = std::max(chain, 64.0 * (p + 1) + 92.0 * shift + 500.0 * chunks);
-                ops += p + shift + row_ops;
-                i += 32 >> shift;
-            }
-            const double v = std::max(chain, 19.0 * ops / sms);
-            if (slices <= max_slices && (cost < 0.0 || v < cost)) { cost = v; best = most; }
-        }
-    }
-    out.clear();
-    if (best == 0) return false;
-    for (int i = lo; i < hi;) {
-        FlowHostSlice s{i, 0, lanes(len[i], best), 0};
-        for (; i < hi && s.nrow < (32 >> s.shift) && lanes(len[i], best) <= s.shift; i++, s.nrow++)
-            s.len = std::max(s.len, part_per_lane(len[i], s.shift));
-        out.push_back(s);
-        if ((int)out.size() > max_slices) { out.clear(); return false; }
-    }
-    return true;
 }
 
 // Builds the slices of the multicolor layout (lazily, kept until the layout changes) and the
@@ -547,37 +456,10 @@ int flow_build(feec_system* s, bool f32) {
         D.mem.stream = st;
         int sms = 0;
         FEEC_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->dev));
-        std::vector<int> rp((size_t)n + 1), ls((size_t)n), us((size_t)n), fptr((size_t)s->nf + 1);
-        FEEC_TRY(cudaMemcpyAsync(rp.data(), s->rp, sizeof(int) * rp.size(), cudaMemcpyDeviceToHost, st));
-        FEEC_TRY(cudaMemcpyAsync(ls.data(), s->lsplit, sizeof(int) * ls.size(), cudaMemcpyDeviceToHost, st));
-        FEEC_TRY(cudaMemcpyAsync(us.data(), s->usplit, sizeof(int) * us.size(), cudaMemcpyDeviceToHost, st));
-        FEEC_TRY(cudaMemcpyAsync(fptr.data(), s->fptr, sizeof(int) * fptr.size(), cudaMemcpyDeviceToHost, st));
-        FEEC_TRY(cudaStreamSynchronize(st));
-        std::vector<HostSlice> slices;
-        for (int c = 0; c < s->nf; c++) {
-            int best = 16;
-            double cost = -1.0;
-            for (int most : {1, 2, 4, 8, 12, 16, 24, 32}) {
-                const double v = slice_rows(fptr[c], fptr[c + 1], rp.data(), ls.data(), us.data(), most, sms, nullptr);
-                if (cost < 0.0 || v < cost) { cost = v; best = most; }
-            }
-            slice_rows(fptr[c], fptr[c + 1], rp.data(), ls.data(), us.data(), best, sms, &slices);
-        }
-        std::vector<int4> meta(slices.size());
-        long long units = 0;
-        for (size_t k = 0; k < slices.size(); k++) {
-            const HostSlice& h = slices[k];
-            if (h.l > 0xffff || h.u > 0xffff || h.e > 0xff || units > 0x7fffffffll) return FEEC_BADARG;
-            meta[k] = make_int4(h.row0, h.nrow | h.shift << 8 | h.e << 16, h.l | (int)((unsigned)h.u << 16), (int)units);
-            units += h.l + h.e + h.u;
-        }
-        D.units = units;
-        D.nslices = (int)meta.size();
-        FEEC_TRY(D.mem.alloc(D.meta, meta.size()));
-        FEEC_TRY(D.mem.alloc(D.ci, (size_t)units * 32));
+        const int e = cut_colors(D, st, sms, s->color_ranges, s->rp, s->lsplit, s->usplit);
+        if (e != FEEC_OK) return e;
+        FEEC_TRY(D.mem.alloc(D.ci, (size_t)D.units * 32));
         for (int k = 0; k < 4; k++) FEEC_TRY(D.mem.alloc(D.pub[k], (size_t)n));
-        FEEC_TRY(cudaMemcpyAsync(D.meta, meta.data(), sizeof(int4) * meta.size(), cudaMemcpyHostToDevice, st));
-        FEEC_TRY(cudaStreamSynchronize(st));   // meta leaves scope
     }
     if (f32) FEEC_TRY(D.mem.alloc(D.val32, (size_t)D.units * 32));
     else FEEC_TRY(D.mem.alloc(D.val64, (size_t)D.units * 32));

@@ -20,8 +20,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
-#include <numeric>
-#include <vector>
 
 #include "flow_device.cuh"
 #include "feec_system.h"
@@ -29,8 +27,6 @@
 
 namespace feec {
 namespace {
-
-constexpr int kSortWindow = 2048;
 
 template <typename T>
 struct FlowCgArgs {
@@ -354,8 +350,6 @@ __global__ void flow_cg_fill_kernel(int nslices, const int4* __restrict__ meta, 
     }
 }
 
-constexpr int kCgRowOps = 7;   // FP64 operations of a row besides its entries
-
 }  // namespace
 
 // The form a natural-order solver runs in: vectors in registers, published, or neither.
@@ -371,10 +365,8 @@ FlowForm flow_natural_form(const FlowData& D, int n, int sms) {
 }
 
 // Rows sorted by length (longest first, stable) within windows of kSortWindow, slices, columns
-// and the values of the wanted precision, from the device CSR (A, C, V) whose row pointer is also
-// in host memory.
-int flow_natural_build(FlowData& D, cudaStream_t st, int dev, int n, const int* rowptr, const int* A, const int* C,
-                       const double* V, bool f32) {
+// and the values of the wanted precision, from the device CSR (A, C, V).
+int flow_natural_build(FlowData& D, cudaStream_t st, int dev, int n, const int* A, const int* C, const double* V, bool f32) {
     const bool first = !D.ready;
     if (first) {
         D.mem.release();
@@ -382,50 +374,11 @@ int flow_natural_build(FlowData& D, cudaStream_t st, int dev, int n, const int* 
         D.mem.stream = st;
         int sms = 0;
         FEEC_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        std::vector<int> perm((size_t)n), iperm((size_t)n), len((size_t)n);
-        std::vector<int> count;
-        for (int w = 0; w < n; w += kSortWindow) {   // counting sort of each window, longest first
-            const int hi = std::min(n, w + kSortWindow);
-            int longest = 0;
-            for (int i = w; i < hi; i++) longest = std::max(longest, rowptr[i + 1] - rowptr[i]);
-            if (longest > 1 << 16) {
-                std::iota(perm.begin() + w, perm.begin() + hi, w);
-                std::stable_sort(perm.begin() + w, perm.begin() + hi,
-                                 [&](int p, int q) { return rowptr[p + 1] - rowptr[p] > rowptr[q + 1] - rowptr[q]; });
-            } else {
-                count.assign((size_t)longest + 2, 0);
-                for (int i = w; i < hi; i++) count[longest - (rowptr[i + 1] - rowptr[i]) + 1]++;
-                for (int l = 0; l <= longest; l++) count[l + 1] += count[l];
-                for (int i = w; i < hi; i++) perm[w + count[longest - (rowptr[i + 1] - rowptr[i])]++] = i;
-            }
-        }
-        for (int i = 0; i < n; i++) { iperm[perm[i]] = i; len[i] = rowptr[perm[i] + 1] - rowptr[perm[i]]; }
-        std::vector<FlowHostSlice> slices;
-        // cut for the register form when its slices fit the grid's warps, else freely
-        if (!flow_cut_rows(0, n, len.data(), kCgRowOps, sms, kFlowChunk, sms * kFlowWarps, slices))
-            flow_cut_rows(0, n, len.data(), kCgRowOps, sms, 32, n, slices);
-        std::vector<int4> meta(slices.size());
-        long long units = 0;
-        int longest = 0;
-        for (size_t k = 0; k < slices.size(); k++) {
-            const FlowHostSlice& h = slices[k];
-            if (h.len > 0xffff || units > 0x7fffffffll) return FEEC_BADARG;
-            meta[k] = make_int4(h.row0, h.nrow | h.shift << 8, (int)((unsigned)h.len << 16), (int)units);
-            units += h.len;
-            longest = std::max(longest, h.len);
-        }
-        D.units = units;
-        D.nslices = (int)meta.size();
-        D.longest = longest;
-        FEEC_TRY(D.mem.alloc(D.meta, meta.size()));
-        FEEC_TRY(D.mem.alloc(D.ci, (size_t)units * 32));
-        FEEC_TRY(D.mem.alloc(D.perm, (size_t)n)); FEEC_TRY(D.mem.alloc(D.iperm, (size_t)n));
+        const int e = cut_natural(D, st, sms, n, A);
+        if (e != FEEC_OK) return e;
+        FEEC_TRY(D.mem.alloc(D.ci, (size_t)D.units * 32));
         for (int k = 0; k < 2; k++) FEEC_TRY(D.mem.alloc(D.pub[k], (size_t)n));
         for (int k = 0; k < 5; k++) FEEC_TRY(D.mem.alloc(D.own[k], (size_t)n));
-        FEEC_TRY(cudaMemcpyAsync(D.meta, meta.data(), sizeof(int4) * meta.size(), cudaMemcpyHostToDevice, st));
-        FEEC_TRY(cudaMemcpyAsync(D.perm, perm.data(), sizeof(int) * perm.size(), cudaMemcpyHostToDevice, st));
-        FEEC_TRY(cudaMemcpyAsync(D.iperm, iperm.data(), sizeof(int) * iperm.size(), cudaMemcpyHostToDevice, st));
-        FEEC_TRY(cudaStreamSynchronize(st));   // the host arrays leave scope
     }
     if (f32) FEEC_TRY(D.mem.alloc(D.val32, (size_t)D.units * 32));
     else FEEC_TRY(D.mem.alloc(D.val64, (size_t)D.units * 32));
@@ -443,13 +396,7 @@ int flow_cg_build(feec_system* s, bool f32) {
     FlowData& D = s->flow_cg;
     if (D.ready && (f32 ? (void*)D.val32 : (void*)D.val64)) return FEEC_OK;
     HomeStreamScope home(s);
-    std::vector<int> rowptr;
-    if (!D.ready) {
-        rowptr.resize((size_t)s->n + 1);
-        FEEC_TRY(cudaMemcpyAsync(rowptr.data(), s->A, sizeof(int) * rowptr.size(), cudaMemcpyDeviceToHost, s->stream));
-        FEEC_TRY(cudaStreamSynchronize(s->stream));
-    }
-    return flow_natural_build(D, s->stream, s->dev, s->n, rowptr.data(), s->A, s->C, s->V, f32);
+    return flow_natural_build(D, s->stream, s->dev, s->n, s->A, s->C, s->V, f32);
 }
 
 namespace {

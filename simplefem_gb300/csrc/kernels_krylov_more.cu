@@ -455,7 +455,7 @@ int more_dropin(int kind, int N, double* x, const double* b, const int* A, const
     bool use_flow = kind == kKindMinres || (kind != kKindChebyshev && N <= kFlowCrRows);
     FlowForm form{};
     if (use_flow) {
-        bool ok = flow_natural_build(flow, s, dev, N, A, dA, dC, dV, false) == FEEC_OK;
+        bool ok = flow_natural_build(flow, s, dev, N, dA, dC, dV, false) == FEEC_OK;
         if (ok) {
             form = flow_natural_form(flow, N, sms);
             for (int k = 0; k < 5 && ok; k++) ok = flow.mem.alloc(w[k], (size_t)N) == cudaSuccess;
