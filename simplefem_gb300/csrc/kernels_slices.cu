@@ -1,15 +1,16 @@
 // Cuts the rows of a layout into the slices of the dataflow solvers (FlowSlice, flow_device.cuh), on
 // the device: a solve of a few iterations takes a millisecond or two, so the cut must not cost
-// more than that. Set-up beside the first solve, walking the rows on the host once for each choice of
-// lanes per row -> here: multicolor 3D P1 refined 7 times (2,146,689 rows) 50 -> 0.9 ms, 6 times 6.7 ->
-// 0.3, 3D P2 refined 5 times (274,625 rows) 7.4 -> 0.5; natural order 13.3 -> 0.4, 2.6 -> 0.3, 3.3 -> 0.4;
-// 2D P1 refined 6 times (4,225 rows) 0.15 -> 0.20. Bound by the walk's chain of loads and votes, and for
-// the large ones by the fill of the slices.
+// more than that. First solves less later ones, with the rows walked on the host once for each choice of
+// lanes per row -> here: colors of 3D P1 refined 7 times (2,146,689 rows) 50 -> 1.0 ms, 6 times 6.7 -> 0.3,
+// 3D P2 refined 5 times (274,625 rows) 7.4 -> 0.5; natural order 13.3 -> 0.7, 2.6 -> 0.3, 3.3 -> 0.3; 2D P1
+// refined 6 times (4,225 rows) 0.15 -> 0.20. Bound by the chains of a window's walk (90 to 113 us on 3D P2
+// refined 5 times) and, for colors, by the fill of the slices (190 us).
 //
-// Rows are cut window by window, a warp per window and choice, greedily from the window's first row:
-// a slice takes the following rows as long as they need no more lanes than its first and fit 32
-// lanes. Windows are multiples of 32 rows from the start of a color (or of the matrix), so that rows
-// of one length fill their slices.
+// The rows of a color (or of a matrix) are cut greedily from the first: a slice takes the following
+// rows as long as they need no more lanes than its first and fit 32 lanes. So that windows of kWindow
+// rows can be cut at the same time, each is cut from all the rows where the slice before it may end,
+// one per lane: its first to its 32nd. The windows' ends are then chained (cut_choose_kernel), which
+// gives the one cut that starts at the color's first row.
 //
 // Lanes per row of each slice. A warp's FP64 instruction holds its scheduler 64 cycles and the SM's
 // FP64 units 19 (measured), and a chunk of kFlowChunk entries takes a trip to L2 of about 500. With p
@@ -31,8 +32,7 @@
 namespace feec {
 namespace {
 
-// Windows of 1,024 and 2,048 rows: 0.6 ms for the natural order of 3D P2 refined 5 times (0.4 here).
-constexpr int kWindow = 256;
+constexpr int kWindow = 512;
 constexpr int kRowOps = 12, kNaturalRowOps = 7;   // FP64 operations of a row besides its entries
 constexpr int kMaxChoices = 8;
 constexpr unsigned kAll = 0xffffffffu;
@@ -46,9 +46,9 @@ struct CutRows {
     const int* len;                    // natural order: entries per row
 };
 
+// Of the slices that start in a window.
 struct CutStats {
-    int chain[2], slices, longest, bad, pad;
-    long long ops[2], units;
+    int chain[2], ops[2], slices, longest, units, bad;
 };
 
 struct CutTotal {
@@ -58,110 +58,128 @@ struct CutTotal {
 
 __device__ __forceinline__ int per_lane(int entries, int shift) { return (entries + (1 << shift) - 1) >> shift; }
 
-// body(first row, rows, shift, entries per lane of L, E and U) for the slices of rows [lo, hi), by a warp.
-template <bool NATURAL, typename F>
-__device__ __forceinline__ void cut_window(const CutRows& rows, int lo, int hi, int most, F&& body) {
-    const int lane = threadIdx.x & 31;
-    for (int i = lo; i < hi;) {
-        const int k = i + lane;
-        int l = 0, e = 0, u = 0;
-        if (k < hi) {
-            if constexpr (NATURAL) {
-                u = __ldg(&rows.len[k]);
-            } else {
-                const int a = __ldg(&rows.rp[k]), b = __ldg(&rows.lsplit[k]), c = __ldg(&rows.usplit[k]), d = __ldg(&rows.rp[k + 1]);
-                l = b - a; e = c - b; u = d - c;
-            }
-        }
-        const int longest = max(l, u);
-        int need = 0;
-        while (need < 5 && per_lane(longest, need) > most) need++;
-        const int shift = __shfl_sync(kAll, need, 0);
-        const unsigned fits = __ballot_sync(kAll, k < hi && lane < (32 >> shift) && need <= shift);
-        const int nrow = fits == kAll ? 32 : __ffs(~fits) - 1;
-        const bool in = lane < nrow;
-        const int pl = NATURAL ? 0 : __reduce_max_sync(kAll, in ? per_lane(l, shift) : 0);
-        const int pe = NATURAL ? 0 : __reduce_max_sync(kAll, in ? per_lane(e, shift) : 0);
-        const int pu = __reduce_max_sync(kAll, in ? per_lane(u, shift) : 0);
-        body(i, nrow, shift, pl, pe, pu);
-        i += nrow;
-    }
+template <bool NATURAL>
+__device__ __forceinline__ int3 row_parts(const CutRows& rows, int i) {
+    if constexpr (NATURAL) return make_int3(0, 0, __ldg(&rows.len[i]));
+    const int a = __ldg(&rows.rp[i]), b = __ldg(&rows.lsplit[i]), c = __ldg(&rows.usplit[i]), d = __ldg(&rows.rp[i + 1]);
+    return make_int3(b - a, c - b, d - c);
+}
+__device__ __forceinline__ int shift_of(int longest, int most) {
+    int s = 0;
+    while (s < 5 && per_lane(longest, s) > most) s++;
+    return s;
 }
 
+// A block per window (color, first row, end, end of the color) and a warp per choice: lane e cuts from
+// the window's row e. ends: how many rows the last slice reaches into the next window.
 template <bool NATURAL>
-__global__ void __launch_bounds__(128) cut_measure_kernel(int nwindows, const int4* __restrict__ windows, CutChoices choices,
-                                                          CutRows rows, CutStats* __restrict__ stats) {
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (gw >= nwindows * choices.count) return;
-    const int4 w = __ldg(&windows[gw / choices.count]);
+__global__ void __launch_bounds__(32 * kMaxChoices) cut_measure_kernel(const int4* __restrict__ windows, CutChoices choices,
+                                                                       CutRows rows, CutStats* __restrict__ stats,
+                                                                       unsigned char* __restrict__ ends) {
+    constexpr int kSpan = kWindow + 32;
+    __shared__ int3 part[kSpan];
+    __shared__ unsigned char need[kMaxChoices][kSpan];
+    const int lane = threadIdx.x & 31, o = threadIdx.x >> 5;
+    const int4 w = windows[blockIdx.x];
+    const int len = w.z - w.y, span = min(len + 31, w.w - w.y);
+    for (int k = threadIdx.x; k < span; k += blockDim.x) part[k] = row_parts<NATURAL>(rows, w.y + k);
+    __syncthreads();
+    for (int k = lane; k < span; k += 32) need[o][k] = (unsigned char)shift_of(max(part[k].x, part[k].z), choices.most[o]);
+    __syncwarp();
     CutStats s{};
-    cut_window<NATURAL>(rows, w.y, w.z, choices.most[gw % choices.count], [&](int, int, int shift, int l, int e, int u) {
-        const int part[2] = {NATURAL ? u : l, u};
+    int i = lane;
+    while (i < len) {
+        const int shift = need[o][i], cap = min(i + (32 >> shift), span);
+        int l = 0, e = 0, u = 0, k = i;
+        do {
+            const int3 p = part[k++];
+            l = max(l, p.x); e = max(e, p.y); u = max(u, p.z);
+        } while (k < cap && need[o][k] <= shift);
+        i = k;
+        l = per_lane(l, shift); e = per_lane(e, shift); u = per_lane(u, shift);
+        const int of[2] = {NATURAL ? u : l, u};
         #pragma unroll
-        for (int k = 0; k < (NATURAL ? 1 : 2); k++) {
-            const int chunks = (part[k] + kFlowChunk - 1) / kFlowChunk;
-            s.chain[k] = max(s.chain[k], 64 * (part[k] + 1) + (NATURAL ? 92 : 64) * shift + 500 * chunks);
-            s.ops[k] += part[k] + shift + (NATURAL ? kNaturalRowOps : kRowOps);
+        for (int d = 0; d < (NATURAL ? 1 : 2); d++) {
+            const int chunks = (of[d] + kFlowChunk - 1) / kFlowChunk;
+            s.chain[d] = max(s.chain[d], 64 * (of[d] + 1) + (NATURAL ? 92 : 64) * shift + 500 * chunks);
+            s.ops[d] += of[d] + shift + (NATURAL ? kNaturalRowOps : kRowOps);
         }
         s.slices++;
-        s.units += l + e + u;
         s.longest = max(s.longest, u);
-        s.bad |= l > 0xffff || u > 0xffff || e > 0xff;
-    });
-    if ((threadIdx.x & 31) == 0) stats[gw] = s;
+        // a slice's parts are 16 bits, its E part 8
+        if (l > 0xffff || u > 0xffff || e > 0xff) s.bad = 1;
+        else s.units += l + e + u;
+    }
+    const long long at = ((long long)blockIdx.x * choices.count + o) * 32 + lane;
+    stats[at] = s;
+    ends[at] = (unsigned char)max(i - len, 0);
 }
 
-// One block per color: the choice with the smallest modelled time, among those of at most max_slices
-// slices and max_longest entries per lane where there are any.
-__global__ void __launch_bounds__(256) cut_choose_kernel(const int* __restrict__ first, CutChoices choices, int sms,
-                                                         int max_slices, int max_longest, const CutStats* __restrict__ stats,
-                                                         int* __restrict__ best) {
-    __shared__ CutStats part[8];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double cost = -1.0;
-    bool within = false;
-    int pick = 0;
-    for (int o = 0; o < choices.count; o++) {
-        CutStats s{};
-        for (int w = first[blockIdx.x] + threadIdx.x; w < first[blockIdx.x + 1]; w += blockDim.x) {
-            const CutStats& t = stats[(long long)w * choices.count + o];
-            for (int k = 0; k < 2; k++) { s.chain[k] = max(s.chain[k], t.chain[k]); s.ops[k] += t.ops[k]; }
-            s.slices += t.slices;
-            s.longest = max(s.longest, t.longest);
-        }
-        for (int off = 16; off > 0; off >>= 1) {
-            for (int k = 0; k < 2; k++) s.ops[k] += __shfl_xor_sync(kAll, s.ops[k], off);
-            s.slices += __shfl_xor_sync(kAll, s.slices, off);
-        }
-        for (int k = 0; k < 2; k++) s.chain[k] = __reduce_max_sync(kAll, s.chain[k]);
-        s.longest = __reduce_max_sync(kAll, s.longest);
-        if (lane == 0) part[warp] = s;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int v = 1; v < 8; v++) {
-                for (int k = 0; k < 2; k++) { s.chain[k] = max(s.chain[k], part[v].chain[k]); s.ops[k] += part[v].ops[k]; }
-                s.slices += part[v].slices;
-                s.longest = max(s.longest, part[v].longest);
+// A block per color, a warp per choice: chains the color's windows (starts[w]: rows of window w that
+// belong to a slice before it) and takes the choice with the smallest modelled time, among those
+// of at most max_slices slices and max_longest entries per lane where there are any.
+__global__ void __launch_bounds__(32 * kMaxChoices) cut_choose_kernel(const int* __restrict__ first, CutChoices choices, int sms,
+                                                                      int max_slices, int max_longest,
+                                                                      const CutStats* __restrict__ stats,
+                                                                      const unsigned char* __restrict__ ends,
+                                                                      unsigned char* __restrict__ starts, int* __restrict__ best) {
+    __shared__ double cost[kMaxChoices];
+    __shared__ bool within[kMaxChoices];
+    const int lane = threadIdx.x & 31, o = threadIdx.x >> 5, last = first[blockIdx.x + 1];
+    int start = 0, chain[2] = {0, 0}, slices = 0, longest = 0;
+    long long ops[2] = {0, 0};
+    for (int w0 = first[blockIdx.x]; w0 < last; w0 += 32) {
+        int mine = 0;
+        for (int j = 0; j < 32; j += 8) {
+            int end[8];
+            #pragma unroll
+            for (int k = 0; k < 8; k++)
+                end[k] = w0 + j + k < last ? ends[((long long)(w0 + j + k) * choices.count + o) * 32 + lane] : 0;
+            #pragma unroll
+            for (int k = 0; k < 8; k++) {
+                if (lane == j + k) mine = start;
+                start = __shfl_sync(kAll, end[k], start);
             }
-            double c = 0.0;
-            for (int k = 0; k < 2; k++) c += fmax((double)s.chain[k], 19.0 * (double)s.ops[k] / sms);
-            const bool in = s.slices <= max_slices && s.longest <= max_longest;
-            if (cost < 0.0 || (in && !within) || (in == within && c < cost)) { cost = c; within = in; pick = o; }
         }
-        __syncthreads();
+        const int w = w0 + lane;
+        if (w < last) {
+            const long long at = (long long)w * choices.count + o;
+            starts[at] = (unsigned char)mine;
+            const CutStats s = stats[at * 32 + mine];
+            for (int d = 0; d < 2; d++) { chain[d] = max(chain[d], s.chain[d]); ops[d] += s.ops[d]; }
+            slices += s.slices;
+            longest = max(longest, s.longest);
+        }
     }
-    if (threadIdx.x == 0) best[blockIdx.x] = pick;
+    for (int off = 16; off > 0; off >>= 1)
+        for (int d = 0; d < 2; d++) ops[d] += __shfl_xor_sync(kAll, ops[d], off);
+    double c = 0.0;
+    for (int d = 0; d < 2; d++) c += fmax((double)__reduce_max_sync(kAll, chain[d]), 19.0 * (double)ops[d] / sms);
+    slices = __reduce_add_sync(kAll, slices);
+    longest = __reduce_max_sync(kAll, longest);
+    if (lane == 0) { cost[o] = c; within[o] = slices <= max_slices && longest <= max_longest; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int pick = 0;
+        for (int k = 1; k < choices.count; k++)
+            if ((within[k] && !within[pick]) || (within[k] == within[pick] && cost[k] < cost[pick])) pick = k;
+        best[blockIdx.x] = pick;
+    }
 }
 
 // First slice and unit of every window (one block), and the totals.
 __global__ void __launch_bounds__(1024) cut_scan_kernel(int nwindows, const int4* __restrict__ windows, CutChoices choices,
-                                                        const CutStats* __restrict__ stats, const int* __restrict__ best,
-                                                        int* __restrict__ slice0, long long* __restrict__ unit0, CutTotal* total) {
+                                                        const CutStats* __restrict__ stats, const unsigned char* __restrict__ starts,
+                                                        const int* __restrict__ best, int* __restrict__ slice0,
+                                                        long long* __restrict__ unit0, CutTotal* total) {
     __shared__ long long su[1024];
     __shared__ int ss[1024], sl[32], sb[32];
     const int t = threadIdx.x, each = (nwindows + 1023) / 1024;
     const int lo = min(t * each, nwindows), hi = min(lo + each, nwindows);
-    auto at = [&](int w) -> const CutStats& { return stats[(long long)w * choices.count + best[windows[w].x]]; };
+    auto at = [&](int w) -> const CutStats& {
+        const long long k = (long long)w * choices.count + best[windows[w].x];
+        return stats[k * 32 + starts[k]];
+    };
     long long units = 0;
     int slices = 0, longest = 0, bad = 0;
     for (int w = lo; w < hi; w++) {
@@ -194,21 +212,34 @@ __global__ void __launch_bounds__(1024) cut_scan_kernel(int nwindows, const int4
     }
 }
 
+// A warp per window: its slices' descriptors.
 template <bool NATURAL>
 __global__ void __launch_bounds__(128) cut_emit_kernel(int nwindows, const int4* __restrict__ windows, CutChoices choices,
-                                                       const int* __restrict__ best, CutRows rows, const int* __restrict__ slice0,
+                                                       const int* __restrict__ best, CutRows rows,
+                                                       const unsigned char* __restrict__ starts, const int* __restrict__ slice0,
                                                        const long long* __restrict__ unit0, int4* __restrict__ meta) {
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (gw >= nwindows) return;
     const int4 w = __ldg(&windows[gw]);
-    int k = slice0[gw];
-    long long at = unit0[gw];
-    cut_window<NATURAL>(rows, w.y, w.z, choices.most[best[w.x]], [&](int row0, int nrow, int shift, int l, int e, int u) {
-        if ((threadIdx.x & 31) == 0)
-            meta[k] = make_int4(row0, nrow | shift << 8 | e << 16, l | (int)((unsigned)u << 16), (int)(unsigned)at);
-        k++;
-        at += l + e + u;
-    });
+    const int o = best[w.x], most = choices.most[o];
+    int slice = slice0[gw];
+    long long unit = unit0[gw];
+    for (int i = w.y + starts[(long long)gw * choices.count + o]; i < w.z;) {
+        const int k = i + lane;
+        const int3 p = k < w.w ? row_parts<NATURAL>(rows, k) : make_int3(0, 0, 0);
+        const int need = shift_of(max(p.x, p.z), most);
+        const int shift = __shfl_sync(kAll, need, 0);
+        const unsigned fits = __ballot_sync(kAll, k < w.w && lane < (32 >> shift) && need <= shift);
+        const int nrow = fits == kAll ? 32 : __ffs(~fits) - 1;
+        const bool in = lane < nrow;
+        const int l = per_lane(__reduce_max_sync(kAll, in ? p.x : 0), shift);
+        const int e = per_lane(__reduce_max_sync(kAll, in ? p.y : 0), shift);
+        const int u = per_lane(__reduce_max_sync(kAll, in ? p.z : 0), shift);
+        if (lane == 0) meta[slice] = make_int4(i, nrow | shift << 8 | e << 16, l | (int)((unsigned)u << 16), (int)(unsigned)unit);
+        slice++;
+        unit += l + e + u;
+        i += nrow;
+    }
 }
 
 // Rows of each window of kSortWindow sorted by length, longest first, equal lengths in their order (one
@@ -246,7 +277,8 @@ int cut(FlowData& D, cudaStream_t st, int sms, const std::vector<int>& ranges, c
     std::vector<int> first(1, 0);
     const int colors = (int)ranges.size() - 1;
     for (int c = 0; c < colors; c++) {
-        for (int lo = ranges[c]; lo < ranges[c + 1]; lo += kWindow) windows.push_back(make_int4(c, lo, std::min(lo + kWindow, ranges[c + 1]), 0));
+        for (int lo = ranges[c]; lo < ranges[c + 1]; lo += kWindow)
+            windows.push_back(make_int4(c, lo, std::min(lo + kWindow, ranges[c + 1]), ranges[c + 1]));
         first.push_back((int)windows.size());
     }
     const int nw = (int)windows.size();
@@ -254,26 +286,29 @@ int cut(FlowData& D, cudaStream_t st, int sms, const std::vector<int>& ranges, c
     tmp.stream = st;
     struct Release { DevArena& m; ~Release() { m.release(); } } rel{tmp};
     int4* dw; int *dfirst, *best, *slice0; long long* unit0; CutStats* stats; CutTotal* dtot;
+    unsigned char *ends, *starts;
+    const size_t cuts = windows.size() * choices.count;
     FEEC_TRY(tmp.alloc(dw, windows.size())); FEEC_TRY(tmp.alloc(dfirst, first.size())); FEEC_TRY(tmp.alloc(best, (size_t)colors));
     FEEC_TRY(tmp.alloc(slice0, windows.size())); FEEC_TRY(tmp.alloc(unit0, windows.size()));
-    FEEC_TRY(tmp.alloc(stats, windows.size() * choices.count)); FEEC_TRY(tmp.alloc(dtot, 1));
+    FEEC_TRY(tmp.alloc(stats, 32 * cuts)); FEEC_TRY(tmp.alloc(ends, 32 * cuts)); FEEC_TRY(tmp.alloc(starts, cuts));
+    FEEC_TRY(tmp.alloc(dtot, 1));
     FEEC_TRY(cudaMemcpyAsync(dw, windows.data(), sizeof(int4) * windows.size(), cudaMemcpyHostToDevice, st));
     FEEC_TRY(cudaMemcpyAsync(dfirst, first.data(), sizeof(int) * first.size(), cudaMemcpyHostToDevice, st));
     for (int k = 0; k < 4; k++) note_launch();
-    cut_measure_kernel<NATURAL><<<(nw * choices.count + 3) / 4, 128, 0, st>>>(nw, dw, choices, rows, stats);
-    cut_choose_kernel<<<colors, 256, 0, st>>>(dfirst, choices, sms, max_slices, max_longest, stats, best);
-    cut_scan_kernel<<<1, 1024, 0, st>>>(nw, dw, choices, stats, best, slice0, unit0, dtot);
+    cut_measure_kernel<NATURAL><<<nw, 32 * choices.count, 0, st>>>(dw, choices, rows, stats, ends);
+    cut_choose_kernel<<<colors, 32 * choices.count, 0, st>>>(dfirst, choices, sms, max_slices, max_longest, stats, ends, starts, best);
+    cut_scan_kernel<<<1, 1024, 0, st>>>(nw, dw, choices, stats, starts, best, slice0, unit0, dtot);
     FEEC_TRY(cudaGetLastError());
     CutTotal total{};
     FEEC_TRY(cudaMemcpyAsync(&total, dtot, sizeof(total), cudaMemcpyDeviceToHost, st));
     FEEC_TRY(cudaStreamSynchronize(st));
-    // a slice's first unit is 32 bits, its parts 16 and its E part 8
+    // a slice's first unit is 32 bits
     if (total.bad || total.slices <= 0 || total.units > 0x7fffffffll) return FEEC_BADARG;
     D.nslices = total.slices;
     D.units = total.units;
     D.longest = total.longest;
     FEEC_TRY(D.mem.alloc(D.meta, (size_t)D.nslices));
-    cut_emit_kernel<NATURAL><<<(nw + 3) / 4, 128, 0, st>>>(nw, dw, choices, best, rows, slice0, unit0, D.meta);
+    cut_emit_kernel<NATURAL><<<(nw + 3) / 4, 128, 0, st>>>(nw, dw, choices, best, rows, starts, slice0, unit0, D.meta);
     FEEC_TRY(cudaGetLastError());
     return FEEC_OK;
 }
