@@ -137,8 +137,11 @@ int true_residual(feec_system* s, const double* bb, const double* xx, double* rr
     // At most four lanes per row: a warp's FP64 operation takes an SM 19 - 20 cycles whatever its
     // lanes add, so the tree over more lanes costs more than the shorter loads save (3D P2 refined
     // 5 times, 28 entries per row: 121 us at 16 lanes, 44 at 4, a solve of six such products 11.9 ms
-    // and 11.5; 3D P3, 50 and more entries per row: 11.86 ms at 32 lanes, 11.77 at 8, 4 and 2).
-    const int lanes = std::min(s->lanes, 4);
+    // and 11.5; 3D P3, 50 and more entries per row: 11.86 ms at 32 lanes, 11.77 at 8, 4 and 2). Rows of
+    // many hundred entries keep their lanes (a capped solve beside its iteration, three residuals,
+    // on 20,000 rows at 32 lanes and at 4: 180 entries per row 152 and 138 us, 362 entries 163 and 161,
+    // 726 entries 185 and 198; 200,000 rows of 198 entries 493 and 234).
+    const int lanes = s->nnz > 400ll * s->n ? s->lanes : std::min(s->lanes, 4);
     const int nb = residual_blocks(s->n, lanes);
     FEEC_TRY(launch_residual_f64(s->n, rp, ci, v, bb, xx, rr, s->partials, lanes, s->stream));
     FEEC_TRY(launch_sum_f64(nb, s->partials, s->scal, s->stream));

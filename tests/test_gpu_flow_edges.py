@@ -368,3 +368,25 @@ def test_slices_cost_no_more_than_a_few_iterations(method):
         extra.append(times[0] - min(times[1:]))
         s.close()
     assert min(extra[1:]) < 2e-3, extra
+
+
+@pytest.mark.parametrize("n,width", [(700, 399), (700, 401), (500, 500)])
+def test_residual_of_long_rows(n, width):
+    """The true residual of rows on either side of 400 entries on average, through the reported
+    quotient with the right-hand side's norm, against numpy: sums of `width` products and of n squares
+    are off by a few hundred units at most, 1e-12."""
+    import torch
+    from simplefem_gb300.system import System
+    rng = np.random.default_rng(width)
+    M = np.zeros((n, n))
+    for i in range(n):
+        M[i, (i + np.arange(width)) % n] = rng.uniform(-1.0, 1.0, width)
+    M += np.diag(np.full(n, 2.0 * width))
+    A, C, V = _csr(sp.csr_matrix(M))
+    s = System(A, C, V)
+    b, x0 = rng.uniform(-1.0, 1.0, n), rng.uniform(-1.0, 1.0, n)
+    x = torch.from_numpy(x0).cuda()
+    info = s.solve(torch.from_numpy(b).cuda(), x, method="cg", mode="fp64", precision=1e-3, max_iter=1)
+    rel = np.linalg.norm(b - M @ x.cpu().numpy()) / np.linalg.norm(b)
+    assert abs(info["true_relres"] - rel) <= 1e-12 * max(rel, 1.0), (info, rel)
+    s.close()
