@@ -490,6 +490,10 @@ const char* feec_status_string(int status);
  * time of the call. Returns FEEC_OK when the GPU answered normally afterwards. */
 int feec_selftest_wait_timeout(double limit_s, int* status, int* site, double* elapsed_ms);
 
+/* The same for the waits of the other solvers, with their own limit of 4 s: 1 a published value that
+ * the dataflow solvers gather, 2 a staged copy of the one-block solver. */
+int feec_selftest_solver_wait(int kind, int* status, int* site, double* elapsed_ms);
+
 #ifdef __cplusplus
 }
 #endif

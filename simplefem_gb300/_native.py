@@ -130,6 +130,8 @@ def gpu():
         L.feec_kernel_launches.restype = ctypes.c_ulonglong
         L.feec_selftest_wait_timeout.argtypes = [_dp, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int),
                                                  ctypes.POINTER(ctypes.c_double)]
+        L.feec_selftest_solver_wait.argtypes = [_ip, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int),
+                                                ctypes.POINTER(ctypes.c_double)]
         L.feec_status_string.restype = ctypes.c_char_p
         L.feec_status_string.argtypes = [_ip]
         _gpu = L

@@ -165,6 +165,7 @@ bool small_pcg_fits(const feec_system* s);
 int small_pcg_prepare(feec_system* s);
 int launch_small_pcg(feec_system* s, const PcgArgs<double>& a, LaunchShape& shape);
 void small_release(feec_system* s);
+cudaError_t launch_missing_copy(DeviceStatus* st, cudaStream_t s);   // self-test of the staging wait
 size_t small_bytes(const feec_system* s);
 // Natural-order slices of a matrix (kernels_flow_cg.cu), and the form that a solver over them runs
 // in: every vector in registers, vectors in memory with the gathered one published, or (neither) too

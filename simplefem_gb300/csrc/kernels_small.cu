@@ -440,6 +440,14 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_pcg(SmallArgs a) {
     finish(a.st, status, K, z_r, 0.0);
 }
 
+// A warp waits for a copy that nobody starts (feec_selftest_wait).
+__global__ void missing_copy_kernel(DeviceStatus* st) {
+    __shared__ unsigned long long bar;
+    if (threadIdx.x == 0) bar_init(&bar);
+    __syncwarp();
+    wait_slices(&bar, 0, st);
+}
+
 // Static shared memory of the kernel, left out of the vectors' share.
 constexpr int kSmallStatic = 8 * (kSmallThreads + 4) + 8 * kMaxSweepDepth + 256;
 
@@ -655,6 +663,12 @@ int small_pcg_prepare(feec_system* s) {
         small_release(s);
     }
     return e;
+}
+
+cudaError_t launch_missing_copy(DeviceStatus* st, cudaStream_t s) {
+    note_launch();
+    missing_copy_kernel<<<1, 32, 0, s>>>(st);
+    return cudaGetLastError();
 }
 
 int launch_small_pcg(feec_system* s, const PcgArgs<double>& p, LaunchShape& shape) {

@@ -390,3 +390,28 @@ def test_residual_of_long_rows(n, width):
     rel = np.linalg.norm(b - M @ x.cpu().numpy()) / np.linalg.norm(b)
     assert abs(info["true_relres"] - rel) <= 1e-12 * max(rel, 1.0), (info, rel)
     s.close()
+
+
+@pytest.mark.parametrize("kind,site", [(1, 78), (2, 0)], ids=["published_value", "staged_copy"])
+def test_waits_for_values_and_copies_give_up(cuda, kind, site):
+    """A wait that nothing satisfies ends after the solvers' limit (4 s) with FEEC_TIMEOUT and its site, and
+    the GPU goes on working: a solve right after gives the solution to 1e-9."""
+    import ctypes
+    import torch
+    from simplefem_gb300 import _native
+    from simplefem_gb300.system import System
+    lib = _native.gpu()
+    st, at, ms = ctypes.c_int(-1), ctypes.c_int(-1), ctypes.c_double(0.0)
+    assert lib.feec_selftest_solver_wait(kind, ctypes.byref(st), ctypes.byref(at), ctypes.byref(ms)) == _native.FEEC_OK
+    assert st.value == 4 and at.value == site
+    assert 4000.0 <= ms.value < 9000.0, ms.value
+    for bad in (-1, 0, 3):
+        assert lib.feec_selftest_solver_wait(bad, ctypes.byref(st), ctypes.byref(at), ctypes.byref(ms)) == 6
+    A, C, V = _csr(_tridiagonal(1000))
+    s = System(A, C, V)
+    x = torch.zeros(1000, dtype=torch.float64, device="cuda")
+    b = np.random.default_rng(0).uniform(-1.0, 1.0, 1000)
+    s.solve(torch.from_numpy(b).cuda(), x, method="cg", mode="fp64", precision=1e-11)
+    x_o = sp.linalg.spsolve(_tridiagonal(1000).tocsc(), b)
+    assert np.linalg.norm(x.cpu().numpy() - x_o) <= 1e-9 * np.linalg.norm(x_o)
+    s.close()
