@@ -314,6 +314,9 @@ int feec_system_set_ssor(feec_system* sys, const double* diagonal, double omega,
 
 /* Solves A x = b on the device. x (in/out, initial guess), b and residual are
  * device pointers of N doubles (residual may be NULL). max_iter <= 0 means N.
+ * A system serves one call at a time; solves of several systems on streams of their own (one
+ * thread each) share the GPU as far as they fit it: a solve takes one block for small SSOR and
+ * Rainbow systems, else a block per four row slices (about 32 to 128 rows) up to one per SM.
  * FEEC_MODE_MIXED (here and in the batched and serving entry points below): when an
  * FP32 inner solve gains less than half the digits it was asked for (condition
  * number times FP32 roundoff near 1e-2 or above), the solve continues in FP64 from
@@ -354,9 +357,11 @@ int feec_system_set_batch_config(feec_system* sys, int method, int mode, int rhs
 
 /* Batched solves of many systems, one right-hand side each (device pointers
  * x[i], b[i] of systems[i]->N doubles; host arrays of pointers). Systems are
- * processed largest first, one thread block per system. For
- * FEEC_METHOD_RAINBOW every system must have been prepared with
- * feec_system_set_rainbow. */
+ * processed largest first, one thread block per system, or a cluster of 2 to 16 blocks
+ * for a system that would alone outlast the rest of the batch spread over the GPU: the order
+ * in which its sums are formed, and with it the last bits of its solution (1e-14 of it),
+ * then depends on the other systems of the call. For FEEC_METHOD_RAINBOW every system must
+ * have been prepared with feec_system_set_rainbow. */
 int feec_solve_many(int nsys, feec_system* const* systems, int method, int mode,
                     double* const* x, const double* const* b, double precision, int max_iter,
                     feec_solve_info* infos, void* stream);
@@ -365,7 +370,10 @@ int feec_solve_many(int nsys, feec_system* const* systems, int method, int mode,
  * x[i], b[i] that stay valid for the batch's lifetime; x holds the initial guess
  * on every run). Everything is set up once and the launch sequence is captured in
  * a CUDA graph; feec_batch_run replays it and fills infos[i] (host, nsys entries,
- * may be NULL) and *device_ms. team_threads 0 = 256. In FEEC_MODE_MIXED the create
+ * may be NULL) and *device_ms. team_threads 0: teams by system size as in feec_solve_many;
+ * else one block of that many threads per system, with which a system's solution is the same
+ * bit for bit in any batch (but for columns that stagnate in FP32 and finish in FP64, whose
+ * teams depend on how many do). In FEEC_MODE_MIXED the create
  * call solves the batch once with FP32 and once with FP64 inner iterations (x is
  * restored afterwards) and keeps the faster; infos[i].inner_fp64 reports it. */
 typedef struct feec_batch feec_batch;
@@ -396,7 +404,9 @@ int feec_system_apply_f32(feec_system* sys, const float* x, float* y, float scal
  * 0 restores the automatic choice. Sizes beyond the co-resident limit are clamped. */
 int feec_system_set_launch(feec_system* sys, int blocks, int lanes);
 
-/* Bytes of device memory held by the system. */
+/* Bytes of device memory held by the system. The first solve of a method adds that method's own
+ * copy of the matrix (slices of the dataflow solvers, or the one-block solver's tables), which
+ * stays until the layout is set again or the system is destroyed. */
 int feec_system_memory(const feec_system* sys, size_t* bytes);
 
 int feec_system_destroy(feec_system* sys);

@@ -415,3 +415,26 @@ def test_waits_for_values_and_copies_give_up(cuda, kind, site):
     x_o = sp.linalg.spsolve(_tridiagonal(1000).tocsc(), b)
     assert np.linalg.norm(x.cpu().numpy() - x_o) <= 1e-9 * np.linalg.norm(x_o)
     s.close()
+
+
+@pytest.mark.parametrize("n", [1, 2])
+@pytest.mark.parametrize("method,mode", [("rainbow", "reference"), ("rainbow_eisenstat", "reference"), ("rainbow", "fp64"),
+                                         ("rainbow", "mixed"), ("cg", "reference"), ("cg", "mixed")])
+def test_one_and_two_rows_converge_beyond_the_cap(method, mode, n):
+    """The smallest systems, with room for the step after which they are exact: one slice, one block.
+    The solution within 1e-12 (cond < 3, residual below 1e-13 of b)."""
+    import torch
+    from oracle import oracle
+    from simplefem_gb300.system import System
+    M = _tridiagonal(n)
+    A, C, V = _csr(M)
+    s = System(A, C, V)
+    s.set_rainbow(oracle.csr_diagonal(A, C, V), 1.0, *oracle.rainbow(A, C))
+    for seed in range(8):
+        b = 1e3 * np.random.default_rng(seed).uniform(-1.0, 1.0, n)
+        x = torch.zeros(n, dtype=torch.float64, device="cuda")
+        info = s.solve(torch.from_numpy(b).cuda(), x, method=method, mode=mode, precision=1e-13, max_iter=20)
+        exact = np.linalg.solve(M.toarray(), b)
+        assert info["status"] == 0 and info["iterations"] <= 20, info
+        assert np.linalg.norm(x.cpu().numpy() - exact) <= 1e-12 * np.linalg.norm(exact), info
+    s.close()
