@@ -683,7 +683,9 @@ int launch_small_pcg(feec_system* s, const PcgArgs<double>& p, LaunchShape& shap
     shape.lanes = 1 << a.fwd.shift;
     note_launch();
     const auto kernel = a.fwd.warps > a.fwd.width || a.bwd.warps > a.bwd.width ? small_pcg<true> : small_pcg<false>;
-    FEEC_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    // the most that any system uses, not this one's: the attribute belongs to the kernel, and other
+    // threads launch it for other systems
+    FEEC_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin_bytes() - kSmallStatic));
     kernel<<<1, kSmallThreads, bytes, s->stream>>>(a);
     return cuda_status(cudaGetLastError());
 }

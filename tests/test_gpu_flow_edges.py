@@ -438,3 +438,39 @@ def test_one_and_two_rows_converge_beyond_the_cap(method, mode, n):
         assert info["status"] == 0 and info["iterations"] <= 20, info
         assert np.linalg.norm(x.cpu().numpy() - exact) <= 1e-12 * np.linalg.norm(exact), info
     s.close()
+
+
+def test_small_solves_of_different_sizes_on_threads():
+    """The one-block solver's shared memory differs by system, its kernel's limit does not: threads
+    that solve small and large systems at the same time, 3,000 capped solves each, all launch."""
+    import threading
+    import torch
+    from oracle import oracle
+    from simplefem_gb300.system import System
+    failed = []
+
+    def worker(n, gate):
+        A, C, V = _csr(_lattice(2, 1, 7, n))
+        s = System(A, C, V)
+        s.set_ssor(oracle.csr_diagonal(A, C, V), 1.0)
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            b = torch.ones(n, dtype=torch.float64, device="cuda")
+            x = torch.zeros_like(b)
+            gate.wait()
+            for _ in range(3000):
+                try:
+                    s.solve(b, x, method="ssor", mode="reference", precision=1e-12, max_iter=1)
+                except Exception as e:      # reported by the test's own thread
+                    failed.append((n, repr(e)))
+                    break
+        s.close()
+
+    sizes = (60, 100, 60, 13_000, 13_000, 13_000, 60, 13_500)
+    gate = threading.Barrier(len(sizes))
+    threads = [threading.Thread(target=worker, args=(n, gate)) for n in sizes]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
