@@ -134,9 +134,20 @@ struct TeamGroup {
 // 1.5 / 2 (at 2 the clusters alone outnumber the SMs); 128 systems 617 ms, then 118 / 104 / 66 /
 // 66; 48 systems 405 ms, then 42 / 46 / 45 / 45. Eight systems at kTeamRows 2048 / 4096 / 8192:
 // 13.2 / 15.5 / 21.8 ms.
+//
+// Two more conditions, from a model of an iteration fitted to batches of equal systems: its FP64
+// instructions divided by the team's blocks, and a step for each color (plain CG: three in all).
+// When the teams' blocks do not all fit the GPU at once, teams of systems up to kLargeRows whose share
+// of the instructions is below kSteps times the steps are halved until they do: a second wave costs
+// more than they gain. And a team is kept only if the system is faster with it, with a longer step
+// where teams share SMs. ms with one block each, with the teams of the rule above alone, and now, FP64
+// Rainbow to 1e-8: 2D P1, 4,225 rows, 100 systems 8.4 / 12.4 / 8.4, 200 systems 11.4 / 16.2 / 11.4; 3D P2,
+// 4,913 rows, 64 systems 6.6 / 8.3 / 6.6, 200 systems 7.8 / 16.4 / 7.8; 2D P2, 9,000 rows, 50 systems
+// 16.7 / 17.2 / 12.4; plain CG, 2D P1, 10,000 rows, 50 systems 32.5 / 17.5 / 12.9.
 std::vector<TeamGroup> plan_teams(const std::vector<feec_system*>& sys, int is_float, int rainbow, std::vector<int>& order) {
     constexpr double kRowOps = 14.0, kTeamShare = 1.5;
-    constexpr int kTeamRows = 2048;
+    constexpr int kTeamRows = 2048, kLargeRows = 8 * kTeamRows;
+    constexpr double kSteps = 1.9;
     const size_t nsys = sys.size();
     int dev = 0, sms = 1;
     cudaGetDevice(&dev);
@@ -150,9 +161,35 @@ std::vector<TeamGroup> plan_teams(const std::vector<feec_system*>& sys, int is_f
     double total = 0.0;
     for (size_t i = 0; i < nsys; i++) total += work[i] = std::sqrt((double)sys[i]->n) * (sys[i]->nnz + kRowOps * sys[i]->n);
     std::vector<int> team(nsys, 1);
-    for (size_t i = 0; i < nsys; i++)
+    long long blocks = 0;
+    for (size_t i = 0; i < nsys; i++) {
         while (team[i] < widest && work[i] * kTeamShare * sms > total * team[i] && sys[i]->n / kTeamRows >= team[i])
             team[i] *= 2;
+        if (team[i] > 1) blocks += team[i];
+    }
+    // an iteration's instructions and steps, in one unit
+    auto part = [&](size_t i) { return 1.19e-6 * (sys[i]->nnz + kRowOps * sys[i]->n); };
+    auto steps = [&](size_t i, bool shared) {
+        if (!rainbow) return 0.028;
+        const double step = shared ? (team[i] == 2 ? 0.0145 : 0.017) : 0.0095 + 0.0002 * sys[i]->nnz / sys[i]->n;
+        return step * sys[i]->nf;
+    };
+    const long long room = 2ll * cluster_batched_resident(is_float, 1, rainbow, 2);
+    for (bool halved = true; blocks > room && halved;) {
+        halved = false;
+        blocks = 0;
+        for (size_t i = 0; i < nsys; i++) {
+            if (team[i] > 1 && sys[i]->n <= kLargeRows && part(i) / team[i] < kSteps * steps(i, true)) {
+                team[i] /= 2;
+                halved = true;
+            }
+            if (team[i] > 1) blocks += team[i];
+        }
+    }
+    for (size_t i = 0; i < nsys; i++) {
+        const double alone = part(i) + (rainbow ? 0.0035 * sys[i]->nf : 0.01);
+        if (team[i] > 1 && part(i) / team[i] + steps(i, blocks > sms) > alone) team[i] = 1;
+    }
     order.resize(nsys);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) {

@@ -474,3 +474,37 @@ def test_small_solves_of_different_sizes_on_threads():
     for t in threads:
         t.join()
     assert not failed, failed
+
+
+@pytest.mark.parametrize("dim,r,L,count", [(2, 1, 6, 100), (2, 1, 6, 200), (3, 2, 3, 64), (3, 2, 3, 200), (3, 1, 4, 100)])
+def test_teams_of_a_batch_pay(dim, r, L, count):
+    """Equal systems that do not fit the GPU in teams of several blocks, or whose colors are too short
+    for them: the batch takes at most 1.15 times as long as with one block per system (up to twice as
+    long before teams were weighed against them), and the solutions agree to 1e-9."""
+    import torch
+    from oracle import oracle
+    from simplefem_gb300 import system
+    A, C, V = _csr(_lattice(dim, r, L, 0))
+    n = len(A) - 1
+    s = system.System(A, C, V)
+    s.set_rainbow(oracle.csr_diagonal(A, C, V), 1.0, *oracle.rainbow(A, C))
+    g = torch.Generator(device="cuda")
+    g.manual_seed(count)
+    bs = list((torch.rand(count, n, dtype=torch.float64, device="cuda", generator=g) * 2.0 - 1.0).unbind())
+    times, results = [], []
+    for threads in (256, 0):
+        xs = [torch.zeros(n, dtype=torch.float64, device="cuda") for _ in range(count)]
+        batch = system.Batch([s] * count, bs, xs, method="rainbow", mode="fp64", precision=1e-10, team_threads=threads)
+        ms = []
+        for _ in range(4):
+            for x in xs:
+                x.zero_()
+            infos, t = batch.run()
+            ms.append(t)
+        assert all(i["status"] == 0 for i in infos)
+        times.append(min(ms))
+        results.append(torch.stack(xs))
+        batch.close()
+    s.close()
+    assert times[1] <= 1.15 * times[0], times
+    assert torch.linalg.norm(results[0] - results[1]) <= 1e-9 * torch.linalg.norm(results[0])
