@@ -7,8 +7,8 @@
 //   chebyshev_persistent — ChebyshevIteration_DiagonalPreconditioner (:2428-2590)
 //
 // MINRES, and CR with at most kFlowCrRows rows, run kernels_flow_more.cu instead (one sum per
-// iteration, the gathered vector published); the kernels here serve larger CR systems and those
-// whose slices do not fit the device memory.
+// iteration, the gathered vector published); the kernels here serve larger CR systems, many long
+// rows, and systems whose slices do not fit the device memory.
 //
 // As in the CG kernels, every grid-wide sum is reduced deterministically (per-block
 // partials, then every block adds them in the same order), scalar recurrences run in
@@ -32,6 +32,7 @@ namespace feec {
 namespace {
 
 constexpr int kFlowCrRows = 200000;
+constexpr int kFlowLongRow = 128, kFlowLongEntries = 1400000;
 
 struct MoreArgs {
     int n;
@@ -443,16 +444,21 @@ int more_dropin(int kind, int N, double* x, const double* b, const int* A, const
     if (hbad) return FEEC_BADARG;
 
     // The dataflow kernels (kernels_flow_more.cu) for MINRES, and for CR up to kFlowCrRows rows; the
-    // barrier-phase kernels of this file for larger CR systems, Chebyshev (one sum per iteration as
-    // it is) and systems whose slices do not fit the device memory. Host calls, barrier-phase -> dataflow
-    // (which sorts rows and cuts slices first): MINRES 3D P1 100,000 rows 11.3 -> 7.4 ms, 274,625
-    // 24.3 -> 18.2, 2,146,689 272 -> 220; CR 3D P1 100,000 rows 8.0 -> 6.9 ms, 200,000 12.9 -> 12.1,
-    // 274,625 15.8 -> 17.1; 2D P1 200,000 rows 52.0 -> 38.6.
+    // barrier-phase kernels of this file for larger CR systems, for many long rows, for Chebyshev (one
+    // sum per iteration as it is) and for systems whose slices do not fit the device memory.
+    // Host calls to 1e-12, barrier-phase -> dataflow (which sorts rows and cuts slices first): MINRES 3D P1
+    // 100,000 rows 11.4 -> 6.5 ms, 274,625 24.8 -> 16.0, 2,146,689 269 -> 207; CR 3D P1 100,000 rows 8.0 ->
+    // 6.0, 200,000 12.9 -> 10.3, 274,625 15.8 -> 14.7, 2,146,689 164 -> 191; 2D P1 200,000 rows 51.8 -> 37.2;
+    // 3D P2 274,625 rows 49.6 -> 38.0. Rows of 201 entries, MINRES / CR of 35 iterations: 6,000 rows 1.00 -> 0.85
+    // / 0.86 -> 0.85, 20,000 rows 1.52 -> 1.57 / 1.48 -> 1.58, 60,000 rows 3.5 both / 3.3 -> 3.6; of 301
+    // entries: 3,000 rows 1.00 -> 0.85 / 0.88 -> 0.83, 6,000 rows 0.90 -> 0.98 / 0.85 -> 0.99 (most of a warp's
+    // time goes into adding 32 lanes per row there); of 101 entries the dataflow form wins up to 60,000 rows.
     int sms = 0;
     FEEC_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     FlowData flow;
     struct ReleaseFlow { FlowData& f; ~ReleaseFlow() { f.mem.release(); } } rel_flow{flow};
-    bool use_flow = kind == kKindMinres || (kind != kKindChebyshev && N <= kFlowCrRows);
+    const bool long_rows = nnz > kFlowLongRow * (long long)N && nnz > kFlowLongEntries;
+    bool use_flow = !long_rows && (kind == kKindMinres || (kind != kKindChebyshev && N <= kFlowCrRows));
     FlowForm form{};
     if (use_flow) {
         bool ok = flow_natural_build(flow, s, dev, N, dA, dC, dV, false) == FEEC_OK;

@@ -508,3 +508,22 @@ def test_teams_of_a_batch_pay(dim, r, L, count):
     s.close()
     assert times[1] <= 1.15 * times[0], times
     assert torch.linalg.norm(results[0] - results[1]) <= 1e-9 * torch.linalg.norm(results[0])
+
+
+@pytest.mark.parametrize("solver", ["minres", "cr"])
+@pytest.mark.parametrize("n,half", [(5600, 124), (5600, 126), (11_300, 62), (11_300, 65)])
+def test_minres_and_cr_of_long_rows(cuda, n, half, solver):
+    """Banded rows on either side of the line between the two forms (128 entries a row, 1.4 M entries): K
+    within 2% (at least 1) of the oracle, the solution within 1e-9 of it."""
+    import simplefem_gb300 as S
+    from oracle import oracle
+    off = np.arange(1, half + 1)
+    R = sp.diags([-np.ones(n - o) for o in off], off, shape=(n, n))
+    R = (R + R.T).tocsr()
+    A, C, V = _csr(R + sp.diags(np.asarray(abs(R).sum(axis=1)).ravel() * 1.01 + 1.0))
+    b = 1e3 * np.random.default_rng(n).uniform(-1.0, 1.0, n)
+    x, res = np.zeros(n), np.zeros(n)
+    K = (S.MINRESCSR if solver == "minres" else S.ConjugateResidualSolverCSR)(n, x, b, A, C, V, res, 1e-11, -3)
+    K_o, x_o, _ = (oracle.minres if solver == "minres" else oracle.cr)(A, C, V, b, precision=1e-11)
+    assert abs(K - K_o) <= max(1, int(np.ceil(0.02 * K_o))), (K, K_o)
+    assert np.linalg.norm(x - x_o) <= 1e-9 * np.linalg.norm(x_o)
