@@ -170,7 +170,7 @@ size_t small_bytes(const feec_system* s);
 // Natural-order slices of a matrix (kernels_flow_cg.cu), and the form that a solver over them runs
 // in: every vector in registers, vectors in memory with the gathered one published, or (neither) too
 // large for publishing to pay.
-constexpr int kFlowPublishedRows = 80000;   // measured in kernels_flow_cg.cu
+constexpr int kFlowPublishedRows = 80000, kFlowPublishedEntries = 8000000;   // measured in kernels_flow_cg.cu
 struct FlowForm {
     int blocks, threads;
     bool registers, published;

@@ -69,10 +69,12 @@ __device__ __forceinline__ void cg_control(const double (&tot)[4], int K, int n,
     }
 }
 
-// kCgRegisters as above. Otherwise the vectors are in memory: up to kFlowPublishedRows rows d is
-// published (kCgPublished; 9.2 us per iteration against 10.8 on 60,000 rows of 3D P1, equal at
-// 100,000); above, publishing costs a sentinel store per row and gathers that skip L1, and a
-// second grid barrier before the product costs less (kCgBarrier). There the product is bound by
+// kCgRegisters as above. Otherwise the vectors are in memory: up to kFlowPublishedRows rows
+// and kFlowPublishedEntries entries d is published (kCgPublished; 9.2 us per iteration against 10.8 on
+// 60,000 rows of 3D P1, equal at 100,000; a solve of 44 iterations, 201 entries per row, 20,000 rows 1.19
+// ms here, 40,000 rows 1.87 against 1.71, 80,000 rows 3.53 against 2.67); above, publishing costs a
+// sentinel store per row and gathers that skip L1, and a second grid barrier before the product costs
+// less (kCgBarrier; compiled for 64 registers, it spills 128 bytes a thread). There the product is bound by
 // the FP64 rate (a warp's FP64 instruction takes an SM 19 - 20 cycles: 78 us of the 102 on 3D P1
 // refined 7 times) and wants 32 warps with 4 entries in flight each: 102 us against 111 for 16
 // warps with 8, 107 for 24 with 4, 125 for 32 with 2, and 130 for cg_persistent.
@@ -360,7 +362,7 @@ FlowForm flow_natural_form(const FlowData& D, int n, int sms) {
     const int warps = (D.nslices + f.blocks - 1) / f.blocks;
     f.threads = 32 * std::min(warps, kFlowWarps);
     f.registers = warps <= kFlowWarps && D.longest <= kFlowChunk;
-    f.published = n <= kFlowPublishedRows;
+    f.published = n <= kFlowPublishedRows && 32 * D.units <= kFlowPublishedEntries;
     return f;
 }
 

@@ -527,3 +527,28 @@ def test_minres_and_cr_of_long_rows(cuda, n, half, solver):
     K_o, x_o, _ = (oracle.minres if solver == "minres" else oracle.cr)(A, C, V, b, precision=1e-11)
     assert abs(K - K_o) <= max(1, int(np.ceil(0.02 * K_o))), (K, K_o)
     assert np.linalg.norm(x - x_o) <= 1e-9 * np.linalg.norm(x_o)
+
+
+@pytest.mark.parametrize("mode", ["reference", "mixed"])
+@pytest.mark.parametrize("half", [196, 204])
+def test_cg_of_many_long_rows(half, mode):
+    """Plain CG on 20,000 banded rows on either side of 8 M stored entries, beyond which d is not
+    published. K within 2% (at least 1) of the oracle, the solution within 1e-9 of it."""
+    import torch
+    from oracle import oracle
+    from simplefem_gb300.system import System
+    n = 20_000
+    off = np.arange(1, half + 1)
+    R = sp.diags([-np.ones(n - o) for o in off], off, shape=(n, n))
+    R = (R + R.T).tocsr()
+    A, C, V = _csr(R + sp.diags(np.asarray(abs(R).sum(axis=1)).ravel() * 1.01 + 1.0))
+    b = 1e3 * np.random.default_rng(n).uniform(-1.0, 1.0, n)
+    K_o, x_o, _ = oracle.cg(A, C, V, b, precision=1e-12)
+    s = System(A, C, V)
+    x = torch.zeros(n, dtype=torch.float64, device="cuda")
+    info = s.solve(torch.from_numpy(b).cuda(), x, method="cg", mode=mode, precision=1e-12)
+    assert info["status"] == 0, info
+    assert np.linalg.norm(x.cpu().numpy() - x_o) <= 1e-9 * np.linalg.norm(x_o), info
+    if mode == "reference":
+        assert abs(info["iterations"] - K_o) <= max(1, int(np.ceil(0.02 * K_o))), (info, K_o)
+    s.close()
