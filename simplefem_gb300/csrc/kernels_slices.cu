@@ -7,8 +7,8 @@
 // refined 5 times) and, for colors, by the fill of the slices (190 us).
 //
 // The rows of a color (or of a matrix) are cut greedily from the first: a slice takes the following
-// rows as long as they need no more lanes than its first and fit 32 lanes. So that windows of kWindow
-// rows can be cut at the same time, each is cut from all the rows where the slice before it may end,
+// rows as long as they need no more lanes than its first and fit 32 lanes. So that windows of rows
+// can be cut at the same time, each is cut from all the rows where the slice before it may end,
 // one per lane: its first to its 32nd. The windows' ends are then chained (cut_choose_kernel), which
 // gives the one cut that starts at the color's first row.
 //
@@ -32,7 +32,8 @@
 namespace feec {
 namespace {
 
-constexpr int kWindow = 512;
+// Rows per window: short ones walk faster, many take longer to chain (one warp chains a matrix's).
+constexpr int window_rows(bool natural) { return natural ? 512 : 256; }
 constexpr int kRowOps = 12, kNaturalRowOps = 7;   // FP64 operations of a row besides its entries
 constexpr int kMaxChoices = 8;
 constexpr unsigned kAll = 0xffffffffu;
@@ -76,7 +77,7 @@ template <bool NATURAL>
 __global__ void __launch_bounds__(32 * kMaxChoices) cut_measure_kernel(const int4* __restrict__ windows, CutChoices choices,
                                                                        CutRows rows, CutStats* __restrict__ stats,
                                                                        unsigned char* __restrict__ ends) {
-    constexpr int kSpan = kWindow + 32;
+    constexpr int kSpan = window_rows(NATURAL) + 32;
     __shared__ int3 part[kSpan];
     __shared__ unsigned char need[kMaxChoices][kSpan];
     const int lane = threadIdx.x & 31, o = threadIdx.x >> 5;
@@ -129,17 +130,14 @@ __global__ void __launch_bounds__(32 * kMaxChoices) cut_choose_kernel(const int*
     int start = 0, chain[2] = {0, 0}, slices = 0, longest = 0;
     long long ops[2] = {0, 0};
     for (int w0 = first[blockIdx.x]; w0 < last; w0 += 32) {
-        int mine = 0;
-        for (int j = 0; j < 32; j += 8) {
-            int end[8];
-            #pragma unroll
-            for (int k = 0; k < 8; k++)
-                end[k] = w0 + j + k < last ? ends[((long long)(w0 + j + k) * choices.count + o) * 32 + lane] : 0;
-            #pragma unroll
-            for (int k = 0; k < 8; k++) {
-                if (lane == j + k) mine = start;
-                start = __shfl_sync(kAll, end[k], start);
-            }
+        int mine = 0, end[32];
+        #pragma unroll
+        for (int k = 0; k < 32; k++)
+            end[k] = w0 + k < last ? ends[((long long)(w0 + k) * choices.count + o) * 32 + lane] : 0;
+        #pragma unroll
+        for (int k = 0; k < 32; k++) {
+            if (lane == k) mine = start;
+            start = __shfl_sync(kAll, end[k], start);
         }
         const int w = w0 + lane;
         if (w < last) {
@@ -212,33 +210,40 @@ __global__ void __launch_bounds__(1024) cut_scan_kernel(int nwindows, const int4
     }
 }
 
-// A warp per window: its slices' descriptors.
+// A warp per window, which one lane walks: its slices' descriptors.
 template <bool NATURAL>
-__global__ void __launch_bounds__(128) cut_emit_kernel(int nwindows, const int4* __restrict__ windows, CutChoices choices,
-                                                       const int* __restrict__ best, CutRows rows,
-                                                       const unsigned char* __restrict__ starts, const int* __restrict__ slice0,
-                                                       const long long* __restrict__ unit0, int4* __restrict__ meta) {
+__global__ void __launch_bounds__(64) cut_emit_kernel(int nwindows, const int4* __restrict__ windows, CutChoices choices,
+                                                      const int* __restrict__ best, CutRows rows,
+                                                      const unsigned char* __restrict__ starts, const int* __restrict__ slice0,
+                                                      const long long* __restrict__ unit0, int4* __restrict__ meta) {
+    constexpr int kSpan = window_rows(NATURAL) + 32;
+    __shared__ int3 parts[2][kSpan];
+    __shared__ unsigned char needs[2][kSpan];
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (gw >= nwindows) return;
-    const int4 w = __ldg(&windows[gw]);
-    const int o = best[w.x], most = choices.most[o];
+    int3* const part = parts[threadIdx.x >> 5];
+    unsigned char* const need = needs[threadIdx.x >> 5];
+    const int4 w = windows[gw];
+    const int o = best[w.x], most = choices.most[o], len = w.z - w.y, span = min(len + 31, w.w - w.y);
+    for (int k = lane; k < span; k += 32) {
+        const int3 p = row_parts<NATURAL>(rows, w.y + k);
+        part[k] = p;
+        need[k] = (unsigned char)shift_of(max(p.x, p.z), most);
+    }
+    __syncwarp();
+    if (lane != 0) return;
     int slice = slice0[gw];
     long long unit = unit0[gw];
-    for (int i = w.y + starts[(long long)gw * choices.count + o]; i < w.z;) {
-        const int k = i + lane;
-        const int3 p = k < w.w ? row_parts<NATURAL>(rows, k) : make_int3(0, 0, 0);
-        const int need = shift_of(max(p.x, p.z), most);
-        const int shift = __shfl_sync(kAll, need, 0);
-        const unsigned fits = __ballot_sync(kAll, k < w.w && lane < (32 >> shift) && need <= shift);
-        const int nrow = fits == kAll ? 32 : __ffs(~fits) - 1;
-        const bool in = lane < nrow;
-        const int l = per_lane(__reduce_max_sync(kAll, in ? p.x : 0), shift);
-        const int e = per_lane(__reduce_max_sync(kAll, in ? p.y : 0), shift);
-        const int u = per_lane(__reduce_max_sync(kAll, in ? p.z : 0), shift);
-        if (lane == 0) meta[slice] = make_int4(i, nrow | shift << 8 | e << 16, l | (int)((unsigned)u << 16), (int)(unsigned)unit);
-        slice++;
+    for (int i = starts[(long long)gw * choices.count + o]; i < len;) {
+        const int first = i, shift = need[i], cap = min(i + (32 >> shift), span);
+        int l = 0, e = 0, u = 0;
+        do {
+            const int3 p = part[i++];
+            l = max(l, p.x); e = max(e, p.y); u = max(u, p.z);
+        } while (i < cap && need[i] <= shift);
+        l = per_lane(l, shift); e = per_lane(e, shift); u = per_lane(u, shift);
+        meta[slice++] = make_int4(w.y + first, (i - first) | shift << 8 | e << 16, l | (int)((unsigned)u << 16), (int)(unsigned)unit);
         unit += l + e + u;
-        i += nrow;
     }
 }
 
@@ -275,10 +280,11 @@ int cut(FlowData& D, cudaStream_t st, int sms, const std::vector<int>& ranges, c
         int max_slices, int max_longest, const CutRows& rows) {
     std::vector<int4> windows;
     std::vector<int> first(1, 0);
+    constexpr int kRows = window_rows(NATURAL);
     const int colors = (int)ranges.size() - 1;
     for (int c = 0; c < colors; c++) {
-        for (int lo = ranges[c]; lo < ranges[c + 1]; lo += kWindow)
-            windows.push_back(make_int4(c, lo, std::min(lo + kWindow, ranges[c + 1]), ranges[c + 1]));
+        for (int lo = ranges[c]; lo < ranges[c + 1]; lo += kRows)
+            windows.push_back(make_int4(c, lo, std::min(lo + kRows, ranges[c + 1]), ranges[c + 1]));
         first.push_back((int)windows.size());
     }
     const int nw = (int)windows.size();
@@ -308,7 +314,7 @@ int cut(FlowData& D, cudaStream_t st, int sms, const std::vector<int>& ranges, c
     D.units = total.units;
     D.longest = total.longest;
     FEEC_TRY(D.mem.alloc(D.meta, (size_t)D.nslices));
-    cut_emit_kernel<NATURAL><<<(nw + 3) / 4, 128, 0, st>>>(nw, dw, choices, best, rows, starts, slice0, unit0, D.meta);
+    cut_emit_kernel<NATURAL><<<(nw + 1) / 2, 64, 0, st>>>(nw, dw, choices, best, rows, starts, slice0, unit0, D.meta);
     FEEC_TRY(cudaGetLastError());
     return FEEC_OK;
 }

@@ -303,11 +303,11 @@ def test_product_reads_no_entry_that_a_row_does_not_have(cuda, length):
     s.close()
 
 
-@pytest.mark.parametrize("n", [1, 31, 1023, 1025, 2047, 2049, 4096, 6145])
+@pytest.mark.parametrize("n", [1, 31, 255, 257, 511, 513, 1023, 1025, 2047, 2049, 4096, 6145])
 @pytest.mark.parametrize("method", ["cg", "rainbow_eisenstat"])
 def test_slices_at_the_edges_of_their_windows(n, method):
-    """Rows are cut within windows of 1,024 rows of a color and 2,048 of a matrix: counts around
-    them, rows without entries beside the diagonal, and one row far longer than the rest in the
+    """Rows are cut in windows of 256 rows of a color and 512 of a matrix, which is sorted in windows of
+    2,048: counts around them, rows without entries beside the diagonal, and one row far longer than the rest in the
     last window. K within 2% (at least 1) of the oracle, the solution within 1e-9 of it."""
     import torch
     from oracle import oracle
