@@ -533,7 +533,6 @@ __global__ void coo_product_big_rows_kernel(int rows, const int* __restrict__ LA
     if (lane == 0) cnt[i] = d;
 }
 
-// Host-side checks of a CSR given by host pointers.
 // Entries of the product of a checked (A1, C1) with a matrix of row pointers A2.
 long long product_entries(int rows, const int* A1, const int* C1, const int* A2) {
     long long total = 0;

@@ -16,9 +16,9 @@
 // Rows, slices and the two forms (vectors in registers or in memory) are those of plain CG
 // (kernels_flow_cg.cu). What is left of an iteration is one publication's way through L2, the
 // product and one reduction. Host calls against the barrier-phase kernels, to 1e-12: 3D P1 refined
-// 5 times (35,937 rows) MINRES 6.85 -> 3.68 ms (358 iterations, 18.3 -> 8.6 us each), CR 4.50 ->
-// 3.25; 3D P2 refined 4 times (35,937 rows, 27 entries each) 14.7 -> 6.9 and 11.5 -> 6.5; 2D P1
-// refined 5 times (1,089 rows) 3.53 -> 1.42 and 2.43 -> 1.37.
+// 5 times (35,937 rows) MINRES 6.85 -> 3.50 ms (358 iterations, 18.3 -> 8.6 us each), CR 4.50 ->
+// 3.08; 3D P2 refined 4 times (35,937 rows, 27 entries each) 14.7 -> 6.6 and 11.5 -> 5.8; 2D P1
+// refined 5 times (1,089 rows) 3.53 -> 1.53 and 2.43 -> 1.49.
 #include <cmath>
 #include <cstdio>
 

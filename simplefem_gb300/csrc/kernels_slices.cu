@@ -3,7 +3,7 @@
 // more than that. First solves less later ones, with the rows walked on the host once for each choice of
 // lanes per row -> here: colors of 3D P1 refined 7 times (2,146,689 rows) 50 -> 1.0 ms, 6 times 6.7 -> 0.3,
 // 3D P2 refined 5 times (274,625 rows) 7.4 -> 0.5; natural order 13.3 -> 0.7, 2.6 -> 0.3, 3.3 -> 0.3; 2D P1
-// refined 6 times (4,225 rows) 0.15 -> 0.20. Bound by the chains of a window's walk (90 to 113 us on 3D P2
+// refined 6 times (4,225 rows) 0.15 -> 0.20. Bound by the chains of a window's walk (80 to 90 us on 3D P2
 // refined 5 times) and, for colors, by the fill of the slices (190 us).
 //
 // The rows of a color (or of a matrix) are cut greedily from the first: a slice takes the following
