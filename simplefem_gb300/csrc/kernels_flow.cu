@@ -459,7 +459,7 @@ int flow_build(feec_system* s, bool f32) {
         const int e = cut_colors(D, st, sms, s->color_ranges, s->rp, s->lsplit, s->usplit);
         if (e != FEEC_OK) return e;
         FEEC_TRY(D.mem.alloc(D.ci, (size_t)D.units * 32));
-        for (int k = 0; k < 4; k++) FEEC_TRY(D.mem.alloc(D.pub[k], (size_t)n));
+        FEEC_TRY(alloc_published(D, 4, n));
     }
     if (f32) FEEC_TRY(D.mem.alloc(D.val32, (size_t)D.units * 32));
     else FEEC_TRY(D.mem.alloc(D.val64, (size_t)D.units * 32));

@@ -379,7 +379,7 @@ int flow_natural_build(FlowData& D, cudaStream_t st, int dev, int n, const int* 
         const int e = cut_natural(D, st, sms, n, A);
         if (e != FEEC_OK) return e;
         FEEC_TRY(D.mem.alloc(D.ci, (size_t)D.units * 32));
-        for (int k = 0; k < 2; k++) FEEC_TRY(D.mem.alloc(D.pub[k], (size_t)n));
+        FEEC_TRY(alloc_published(D, 2, n));
         for (int k = 0; k < 5; k++) FEEC_TRY(D.mem.alloc(D.own[k], (size_t)n));
     }
     if (f32) FEEC_TRY(D.mem.alloc(D.val32, (size_t)D.units * 32));
