@@ -265,18 +265,20 @@ def test_small_solves_on_several_streams_share_the_gpu(method, mode):
             solve(i)
         gate.wait()
 
-    threads = [threading.Thread(target=worker, args=(i,)) for i in range(T)]
-    for th in threads:
-        th.start()
-    gate.wait()
-    t = time.perf_counter()
-    gate.wait()
-    together = time.perf_counter() - t
-    for th in threads:
-        th.join()
-    torch.cuda.synchronize()
-    assert [x.cpu().numpy().tobytes() for x in xs] == alone
-    assert together < 0.5 * serial, (together, serial)
+    together = []
+    for _ in range(3):          # the best counts: the host may be interrupted
+        threads = [threading.Thread(target=worker, args=(i,)) for i in range(T)]
+        for th in threads:
+            th.start()
+        gate.wait()
+        t = time.perf_counter()
+        gate.wait()
+        together.append(time.perf_counter() - t)
+        for th in threads:
+            th.join()
+        torch.cuda.synchronize()
+        assert [x.cpu().numpy().tobytes() for x in xs] == alone
+    assert min(together) < 0.5 * serial, (together, serial)
     for s in systems:
         s.close()
 
